@@ -1804,11 +1804,13 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     const size_t nCounters = std::max<size_t>(allChunks.size() + kNumShapes, 2 * kNumShapes);
     CK(ctx->dCounter.ensure(nCounters), "alloc counters");
 
-    // Null-model jobs: up to 32 pairs of reads of one length per warp (the
-    // lanes run in lock step over the columns), the pairs of one read
-    // side by side, the longest reads first: the kernel's warps take the jobs
-    // round-robin, so that each warp ends on short jobs and the kernel has no
-    // tail of long reads started last.
+    // Null-model jobs: up to 32 pairs per job (one lane each, in lock step over
+    // the columns of the longest), the pairs of one read side by side, the
+    // longest reads first: the kernel's warps take the jobs round-robin, so
+    // that each warp ends on short jobs and the kernel has no tail of long
+    // reads started last.  A job's reads are at least 7/8 of its longest one's
+    // length: reads of many lengths against one profile (prefilter windows)
+    // would otherwise run one pair per warp.
     std::vector<int> jobPairs(n);
     {
         // A counting sort of the (profile-major) pair slots by read, with the
@@ -1835,7 +1837,8 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     long long nullTmpEntries = 0;
     for (size_t k = 0; k < n;) {
         size_t e = k;
-        while (e < n && e - k < 32 && dp[jobPairs[e]].L == dp[jobPairs[k]].L) ++e;
+        const int longest = dp[jobPairs[k]].L;
+        while (e < n && e - k < 32 && dp[jobPairs[e]].L >= longest - longest / 8) ++e;
         nullJobs.push_back(NullJob{(int)k, (int)(e - k)});
         nullTmpOff.push_back(nullTmpEntries);
         nullTmpEntries += dmst::nullTmpEntries(dp[jobPairs[k]].L);
@@ -1969,7 +1972,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         ctx->nullBlocksPerSm = std::max(1, perSm);
     }
     const int nullBlocks =
-        std::max(1, std::min((nj + kNullWarps - 1) / kNullWarps, ctx->smCount * ctx->nullBlocksPerSm));
+        std::max(1, std::min((nj + kNullJobs - 1) / kNullJobs, ctx->smCount * ctx->nullBlocksPerSm));
     DpArgs g;
     g.pairs = S.dPairs.p;
     g.profiles = ctx->dProfiles.p;

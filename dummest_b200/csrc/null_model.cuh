@@ -48,41 +48,6 @@ __device__ __forceinline__ XS scaleScore(XS a, double f) {
     return splitNorm(__dmul_rn((double)a.m, f), a.e);
 }
 
-// scaleScore by a positive finite factor below 1 (the frameshift emission
-// rates): the product of a float mantissa in [0.5, 1] and f is 0 or a normal
-// double, so splitNorm's infinity and subnormal cases cannot occur; the
-// result is scaleScore's.
-__device__ __forceinline__ XS scaleByRate(XS a, double f) {
-    if (a.m == 0.0f) return xsZero();
-    const double x = __dmul_rn((double)a.m, f);
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    const int ef = (int)((u >> 52) & 0x7FFULL);
-    const double m = __longlong_as_double((long long)((u & 0xFFFFFFFFFFFFFULL) | (1022ULL << 52)));
-    return XS{__double2float_rn(m), a.e + ef - 1022};
-}
-
-// batchAddScores (dummest-batch.hh:78-108).
-__device__ __forceinline__ XS batchAdd(XS a, XS b) {
-    if (a.m == 0.0f) return b;
-    if (b.m == 0.0f) return a;
-    const bool agebe = a.e >= b.e;
-    const float mh = agebe ? a.m : b.m, ml = agebe ? b.m : a.m;
-    const int eh = agebe ? a.e : b.e, el = agebe ? b.e : a.e;
-    int d = eh - el;
-    d = d > 60 ? 60 : d;
-    // 1 / 2^d is the exact power 2^-d (0 <= d <= 60), built from its exponent
-    // bits instead of a double division; ml * 2^-d is exact, so the sum
-    // rounds once, as the reference's does.
-    const double inv = __longlong_as_double((long long)(1023 - d) << 52);
-    double s = __dadd_rn((double)mh, __dmul_rn((double)ml, inv));
-    int e = eh;
-    if (s >= 1.0) {
-        s *= 0.5;
-        e += 1;
-    }
-    return XS{__double2float_rn(s), e};
-}
-
 // addScores, the scalar form (dummest-score.hh:169-181).  ldexp(m, -d) for
 // 0 <= d <= 60 is the product of m and the power 2^-d built from its exponent
 // bits: both exact, so the same bits.
@@ -127,62 +92,234 @@ __device__ __forceinline__ float packScore(XS a) {
     return ldexpf(a.m, e);
 }
 
+// ---------------------------------------------------------------------------
+// The recurrences' score algebra without double arithmetic, bit for bit the
+// double forms of dummest-batch.hh: each of those rounds the exact result of
+// one operation on two float mantissas to a float, so one correctly rounded
+// float operation gives the same mantissa, and the same operation rounded
+// toward zero tells on which side of a power of two the exact result lies
+// (the reference tests the double before it rounds to float, so a mantissa
+// that rounds up to a power of two keeps the smaller exponent).  A dependent
+// step then costs about 12 cycles (multiply) or 25 (add), where the double
+// forms with their conversions took several hundred for a column.
+//
+// A zero carries the exponent kZeroExp, so that it is never the larger
+// operand of a sum.
+// ---------------------------------------------------------------------------
+constexpr int kZeroExp = -(1 << 28);
+
+__device__ __forceinline__ void storeXS(XS *p, XS v) {  // 8-byte aligned
+    *reinterpret_cast<float2 *>(p) = make_float2(v.m, __int_as_float(v.e));
+}
+__device__ __forceinline__ XS tagZero(XS a) { return XS{a.m, a.m == 0.0f ? kZeroExp : a.e}; }
+
+// batchMulScores with eFold = 0 (dummest-batch.hh:58-72), and scaleScore by a
+// float factor given as mantissa in [0.5, 1) and exponent
+// (dummest-batch.hh:114-130): the product of two mantissas in [0.5, 1] is in
+// [0.25, 1], doubled when the exact product is below 0.5.
+__device__ __forceinline__ XS mulF(XS a, XS b) {
+    const float p = __fmul_rn(a.m, b.m);
+    const bool lt = __fmul_rz(a.m, b.m) < 0.5f;
+    return XS{lt ? p + p : p, a.e + b.e - (lt ? 1 : 0)};
+}
+
+// batchAddScores (dummest-batch.hh:78-108).  The smaller mantissa times 2^-d
+// (d <= 60) is an exact float; the double sum is exact for d <= 29, and for
+// larger d the smaller term is below 2^-29, where both roundings return the
+// larger mantissa.
+__device__ __forceinline__ XS addF(XS a, XS b) {
+    const bool ag = a.e >= b.e;
+    const float mh = ag ? a.m : b.m, ml = ag ? b.m : a.m;
+    const int eh = max(a.e, b.e), d = min(eh - min(a.e, b.e), 60);
+    const float inv = __int_as_float((127 - d) << 23);
+    const float s = __fmaf_rn(ml, inv, mh);
+    const bool ge = __fmaf_rz(ml, inv, mh) >= 1.0f && ml != 0.0f;
+    return XS{ge ? s * 0.5f : s, eh + (ge ? 1 : 0)};
+}
+
+// scaleScore (dummest-batch.hh:114-130) by a double factor f, 0 < f < 1 (0:
+// the result is zero): the one product whose 53-bit rounding can differ from
+// a direct rounding to float, so it stays in double.  The mantissa goes to
+// double by moving its bits.
+__device__ __forceinline__ XS scaleD(XS a, double f) {
+    const unsigned b = __float_as_uint(a.m);
+    const double am = __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+    const double x = __dmul_rn(am, f);
+    const int hi = __double2hiint(x);
+    const float m = __double2float_rn(__hiloint2double((hi & 0xFFFFF) | 0x3FE00000, __double2loint(x)));
+    const bool nz = a.m != 0.0f && f != 0.0;
+    return XS{nz ? m : 0.0f, nz ? a.e + (hi >> 20) - 1022 : kZeroExp};
+}
+
 struct NullRates {
     double single;      // BACKGROUND_FRAMESHIFT_RATE (a float value)
     double dbl;         // BACKGROUND_FRAMESHIFT_RATE_2 (a float value)
 };
 
-__device__ __forceinline__ float bgAt(const float *bg, const uint8_t *codes, int L, int j) {
-    return (j >= 0 && j < L) ? bg[codes[j]] : 0.0f;  // beyond the sequence: zero_idx, bg 0
+// A frameshift emission rate as the recurrences use it.  The rates are float
+// values, so the mantissa is exact.  A rate of 0 gives 2^-1023 of its operand
+// (mantissa 0.5), as splitting a zero product's bits does.
+struct RateF {
+    XS f;
+    bool zero;
+};
+__device__ __forceinline__ RateF rateF(double v) {
+    RateF r;
+    r.zero = v == 0.0;
+    r.f = r.zero ? XS{0.5f, -1021} : splitNorm(v, 0);
+    return r;
+}
+template <bool ZERO>
+__device__ __forceinline__ XS scaleByRate(XS a, const RateF &r) {
+    const XS v = mulF(a, r.f);
+    if (ZERO && r.zero) return XS{a.m == 0.0f ? 0.0f : 0.5f, a.e - 1022};
+    return v;
 }
 
-// Prefix recurrence (dummest-dp-backward.hh:66-99) step i, given the three
-// previous prefix values.
-__device__ __forceinline__ XS prefixStep(int i, const float *bg, const uint8_t *codes, int L, XS p1, XS p2, XS p3,
-                                         double keep, double sNE, double dNE) {
-    const float bgc = bgAt(bg, codes, L, i - 2);
-    const double codonScale = __dmul_rn((double)bgc, keep);
-    const double frame = 1.0 / 3.0;
-    XS codon;
-    if (i >= 3)
-        codon = scaleScore(p3, codonScale);
-    else if (i == 2)
-        codon = scaleScore(splitNorm((double)bgc, 0), frame);
-    else if (i == 1)
-        codon = scaleScore(pow2Score(-4), frame);
-    else
-        codon = scaleScore(pow2Score(-2), frame);
-    XS single = scaleByRate(i > 0 ? p1 : xsZero(), sNE);
-    XS dbl = scaleByRate(i >= 2 ? p2 : xsZero(), dNE);
-    return batchAdd(codon, batchAdd(single, dbl));
-}
-
-// Pairs whose reads have one length are scored by one warp, one lane per
-// pair (the pairs of one read side by side, so that their codon loads are
-// broadcasts): the lanes run in lock step over the L columns, keep the
-// suffix recurrence in registers, store the temporary prefix and suffix
-// probabilities interleaved (one coalesced 256-byte store per column), and
-// write their seed vectors through a shared-memory transpose, so that each
-// store instruction writes 32 consecutive seeds of one pair.
-// Temporary ExpScores of one null-model job: the prefix [L][32] and the
-// suffix [L+1][32] probabilities of its (up to) 32 pairs, interleaved.
+// Pairs of one job are scored by two warps, one lane per pair (the pairs of
+// one read side by side, so that their codon loads are broadcasts): one warp
+// runs the prefix recurrence and then the prefix seeds, the other the suffix
+// recurrence and the suffix seeds.  The lanes run in lock step over the
+// columns of the longest read, store the recurrences' values interleaved (one
+// coalesced 256-byte store per column) and write their seeds through a
+// shared-memory transpose, so that each store writes 32 consecutive seeds of
+// one pair.
+//
+// Bound: the serial chain of a column (prefix or suffix: a rate product and
+// two sums) in small calls, issue in large ones.  With both chains and the
+// seeds' power chains one after another on one warp, in double (540
+// instructions and 2700 cycles a column), this took 4.40 ms for 200 reads of
+// 3.1 kb, 13.3 ms for 16 of 10 kb and 5.3 ms for 128,000 pairs of 150-3000 nt;
+// now 0.78, 2.35 and 2.2 ms.
+//
+// Temporary ExpScores of one job: prefix and suffix values [L+1][32] each.
 __host__ __device__ constexpr long long nullTmpEntries(long long L) { return 2 * 32 * (L + 1); }
 
 struct NullJob {
-    int first;  // index of the job's first pair in the pair-index array
-    int count;  // pairs in the job (<= 32), all with the same read
+    int first;  // index of the job's first (longest) pair in the pair-index array
+    int count;  // pairs in the job (<= 32)
 };
 
 constexpr int kNullWarps = 4;
+constexpr int kNullJobs = kNullWarps / 2;  // jobs of a CTA at a time
+constexpr int kNullAhead = 8;   // codes loaded ahead of the recurrences
+constexpr int kNullChunk = 16;  // stored values loaded ahead of the seed chains
 
-__device__ __forceinline__ void flushSeeds(float (*stage)[33], float *const *dst, int count, int j0, int ncol,
+// Columns j0 .. j0+31 of the job's seeds: stage[c][p] holds column j0 + c of
+// pair p; write pair p's columns with lanes over columns.
+__device__ __forceinline__ void flushSeeds(float (*stage)[33], float *const *dst, const int *len, int count, int j0,
                                            int lane) {
-    // stage[c][p] holds column j0 + c of pair p; write pair p's columns with
-    // lanes over columns.
     __syncwarp();
     for (int p = 0; p < count; ++p)
-        if (lane < ncol) dst[p][j0 + lane] = stage[lane][p];
+        if (j0 + lane < len[p]) dst[p][j0 + lane] = stage[lane][p];
     __syncwarp();
+}
+
+// Prefix recurrence (dummest-dp-backward.hh:58-100), i = 0 .. Lmax-1; a lane
+// past its read's end computes values that nothing reads.
+template <bool ZERO>
+__device__ __forceinline__ void prefixPass(const uint8_t *cd, int L, int Lmax, const double *tab, float bg0, XS *pfx,
+                                           int lane, const RateF &sNE, const RateF &dNE) {
+    const double frame = 1.0 / 3.0;
+    XS p1{0.0f, kZeroExp}, p2 = p1, p3 = p1;
+    for (int i = 0; i < 3 && i < Lmax; ++i) {
+        const XS codon = tagZero(i == 2 ? scaleScore(splitNorm((double)bg0, 0), frame)
+                                        : scaleScore(pow2Score(i == 1 ? -4 : -2), frame));
+        const XS zero{0.0f, kZeroExp};
+        const XS q = addF(codon, addF(i > 0 ? scaleByRate<ZERO>(p1, sNE) : zero, i > 1 ? scaleByRate<ZERO>(p2, dNE) : zero));
+        storeXS(pfx + i * 32 + lane, q);
+        p3 = p2;
+        p2 = p1;
+        p1 = q;
+    }
+    // the code of column i is that of position i - 2
+    const int last = L - 1;
+    int c[kNullAhead];
+#pragma unroll
+    for (int u = 0; u < kNullAhead; ++u) c[u] = cd[min(1 + u, last)];
+    for (int i0 = 3; i0 < Lmax; i0 += kNullAhead) {
+#pragma unroll
+        for (int u = 0; u < kNullAhead; ++u) {
+            const int i = i0 + u;
+            if (i >= Lmax) break;
+            const double f = tab[min(c[u], 25) * 32];
+            c[u] = cd[min(i + kNullAhead - 2, last)];
+            const XS codon = scaleD(p3, f);
+            const XS q = addF(codon, addF(scaleByRate<ZERO>(p1, sNE), scaleByRate<ZERO>(p2, dNE)));
+            storeXS(pfx + (size_t)i * 32 + lane, q);
+            p3 = p2;
+            p2 = p1;
+            p1 = q;
+        }
+    }
+}
+
+// Suffix recurrence (:6-55) from suffix[L] = 1 and suffix[L+1..L+3] = 0; step
+// k is column i = L-1-k, stored at k.
+template <bool ZERO>
+__device__ __forceinline__ void suffixPass(const uint8_t *cd, int L, int Lmax, const double *tab, double keep, XS *sfx,
+                                           int lane, const RateF &sNE, const RateF &dNE) {
+    const XS trailing = tagZero(splitNorm(0.5 * keep, 0));
+    XS s1 = pow2Score(0), s2{0.0f, kZeroExp}, s3 = s2;  // suffix[i+1], [i+2], [i+3]
+    for (int k = 0; k < 2 && k < Lmax; ++k) {
+        const XS codon{trailing.m, trailing.e - 2 * (k + 1) + 1};
+        const XS v = addF(codon, addF(scaleByRate<ZERO>(s1, sNE), scaleByRate<ZERO>(k > 0 ? s2 : pow2Score(2), dNE)));
+        storeXS(sfx + k * 32 + lane, v);
+        s3 = s2;
+        s2 = s1;
+        s1 = v;
+    }
+    const int last = L - 1;
+    int c[kNullAhead];
+#pragma unroll
+    for (int u = 0; u < kNullAhead; ++u) c[u] = cd[max(last - 2 - u, 0)];
+    for (int k0 = 2; k0 < Lmax; k0 += kNullAhead) {
+#pragma unroll
+        for (int u = 0; u < kNullAhead; ++u) {
+            const int k = k0 + u;
+            if (k >= Lmax) break;
+            const double f = tab[min(c[u], 25) * 32];
+            c[u] = cd[max(last - k - kNullAhead, 0)];
+            const XS codon = scaleD(s3, f);
+            const XS v = addF(codon, addF(scaleByRate<ZERO>(s1, sNE), scaleByRate<ZERO>(s2, dNE)));
+            storeXS(sfx + (size_t)k * 32 + lane, v);
+            s3 = s2;
+            s2 = s1;
+            s1 = v;
+        }
+    }
+}
+
+// The seeds of columns 0 .. Lmax-1 (dummest-dp-backward.hh:137-164): stored
+// value times a running power, the values of kNullChunk columns loaded while
+// the ones before are used.  SUFFIX: column j's value is suffix[j+1], stored
+// at L-2-j (1 at the last column).
+template <bool SUFFIX>
+__device__ __forceinline__ void seedPass(const XS *val, int L, int Lmax, XS run, XS step, float (*stage)[33],
+                                         float *const *dst, const int *len, int count, int lane) {
+    auto load = [&](int j) -> XS {
+        const int q = SUFFIX ? L - 2 - j : j;
+        if (SUFFIX ? j >= L - 1 : j >= L) return pow2Score(0);
+        const float2 t = *reinterpret_cast<const float2 *>(val + (size_t)q * 32 + lane);
+        return XS{t.x, __float_as_int(t.y)};
+    };
+    XS next[kNullChunk];
+#pragma unroll
+    for (int u = 0; u < kNullChunk; ++u) next[u] = load(u);
+    for (int j0 = 0; j0 < Lmax; j0 += kNullChunk) {
+        XS v[kNullChunk];
+#pragma unroll
+        for (int u = 0; u < kNullChunk; ++u) {
+            v[u] = next[u];
+            next[u] = load(j0 + kNullChunk + u);
+        }
+#pragma unroll
+        for (int u = 0; u < kNullChunk; ++u) {
+            stage[(j0 & 16) + u][lane] = packScore(mulF(v[u], run));
+            run = mulF(run, step);
+        }
+        if ((j0 & 16) || j0 + kNullChunk >= Lmax) flushSeeds(stage, dst, len, count, j0 & ~31, lane);
+    }
 }
 
 __global__ void __launch_bounds__(kNullWarps * 32) nullModelKernel(const NullJob *jobs, int nJobs, const int *jobPairs,
@@ -191,120 +328,93 @@ __global__ void __launch_bounds__(kNullWarps * 32) nullModelKernel(const NullJob
                                                                    const long long *tmpOff, PairScales *scales,
                                                                    NullRates r) {
     __shared__ float stageAll[kNullWarps][32][33];
-    __shared__ float *dstAll[kNullWarps][2][32];
+    __shared__ double tabAll[kNullJobs][26][32];  // a lane's codon factor by code: background x keep, 0 past code 24
+    __shared__ float *dstAll[kNullWarps][32];
+    __shared__ int lenAll[kNullWarps][32];
+    __shared__ XS baseAll[kNullJobs][2][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int jw = warp >> 1;                    // the job of this warp pair
+    const bool suffixWarp = (warp & 1) != 0;
+    auto pairSync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + jw) : "memory"); };
     float (*stage)[33] = stageAll[warp];
-    const double keep = 1.0 - r.single - r.dbl;  // codonKeepProbability
-    const double sNE = r.single * 0.25;          // singleNucleotideEmission
-    const double dNE = r.dbl * 0.0625;           // doubleNucleotideEmission
-    for (int ji = blockIdx.x * kNullWarps + warp; ji < nJobs; ji += gridDim.x * kNullWarps) {
+    const double keep = 1.0 - r.single - r.dbl;      // codonKeepProbability
+    const RateF sNE = rateF(r.single * 0.25);        // singleNucleotideEmission
+    const RateF dNE = rateF(r.dbl * 0.0625);         // doubleNucleotideEmission
+    const bool anyZero = sNE.zero || dNE.zero;
+    for (int ji = blockIdx.x * kNullJobs + jw; ji < nJobs; ji += gridDim.x * kNullJobs) {
         const NullJob job = jobs[ji];
         const bool on = lane < job.count;
         const int pi = jobPairs[job.first + (on ? lane : 0)];
         const DevPair p = pairs[pi];
         const int L = p.L;
+        const int Lmax = __shfl_sync(kFull, L, 0);
         const uint8_t *cd = codes + p.codeOff;
         const float *bg = profiles[p.prof].bg;
         float *pre = seeds + p.seedOff;
-        dstAll[warp][0][lane] = on ? pre : nullptr;
-        dstAll[warp][1][lane] = on ? pre + L : nullptr;
-        XS *pfx = tmp + tmpOff[ji];           // [L x 32] interleaved prefix probabilities
-        XS *sfx = pfx + 32 * ((size_t)L + 1);  // [(L+1) x 32] interleaved suffix probabilities
-
-        // Pass 1: the prefix recurrence (dummest-dp-backward.hh:58-100, i = 0..L-1)
-        // and the suffix recurrence (:6-55, i = L-1..0, from suffix[L] = 1 and
-        // suffix[L+1..L+3] = 0), two independent chains run side by side; both
-        // sequences are kept for the seed passes.
-        XS p1 = xsZero(), p2 = xsZero(), p3 = xsZero();
-        const XS trailing = splitNorm(0.5 * keep, 0);
-        XS s1 = pow2Score(0), s2 = xsZero(), s3 = xsZero();  // suffix[i+1], [i+2], [i+3]
-        for (int k = 0; k < L; ++k) {
-            const XS q = prefixStep(k, bg, cd, L, p1, p2, p3, keep, sNE, dNE);
-            pfx[(size_t)k * 32 + lane] = q;
-            p3 = p2;
-            p2 = p1;
-            p1 = q;
-            const int i = L - 1 - k;
-            const double codonScale = __dmul_rn((double)bgAt(bg, cd, L, i), keep);
-            const XS single = scaleByRate(s1, sNE);
-            const XS dIn = (i + 1 < L) ? s2 : pow2Score(2);
-            const XS dbl = scaleByRate(dIn, dNE);
-            const XS codon = (i + 2 < L) ? scaleScore(s3, codonScale) : XS{trailing.m, trailing.e - 2 * (L - i) + 1};
-            const XS v = batchAdd(codon, batchAdd(single, dbl));
-            sfx[(size_t)i * 32 + lane] = v;
-            s3 = s2;
-            s2 = s1;
-            s1 = v;
-        }
-        // Total and scales (dummest-dp-backward.hh:103-129).
-        const double keepSingle = 1.0 - r.single;
-        const double keepBoth = keepSingle - r.dbl;
-        const XS trailingSingle = scaleScore(p2, keepSingle * 0.25);
-        const XS trailingDouble = scaleScore(p3, keepBoth * 0.0625);
-        const XS total = scalarAdd(scalarAdd(p1, trailingSingle), trailingDouble);
-        const float nullLog = (total.m == 0.0f) ? -INFINITY : (float)(log2((double)total.m) + (double)total.e);
-        double perBaseLog = -(double)nullLog / (double)L;
-        if (!(perBaseLog < 120.0)) perBaseLog = 120.0;
-        const double perBaseRaw = exp2(perBaseLog);
-        const XS perBase = splitNorm(perBaseRaw, 0);
-        const XS perBaseInv = splitNorm(1.0 / perBaseRaw, 0);
-        const XS quarter = splitNorm(0.25, 0), sixteenth = splitNorm(0.0625, 0);
-        if (on) {
-            PairScales sc;
-            sc.s1 = packScore(scalarMul(perBase, quarter));
-            sc.s2 = packScore(scalarMul(scalarMul(perBase, perBase), sixteenth));
-            sc.sC = packScore(scalarMul(scalarMul(perBase, perBase), perBase));
-            sc.pad = 0.0f;
-            scales[pi] = sc;
-        }
-
-        // Pass 2: prefix seeds (dummest-dp-backward.hh:155-164) from the kept
-        // prefix, beside the L-1 multiplications that start the suffix seeds'
-        // running scale (:137-145).
-        XS running = pow2Score(0);
-        XS runPre = perBase;
-        for (int j0 = 0; j0 < L; j0 += 32) {
-            const int ncol = L - j0 < 32 ? L - j0 : 32;
-            for (int c0 = 0; c0 < ncol; c0 += 8) {
-                // the kept prefix values of 8 columns, loaded before the chain uses them
-                XS v[8];
+        dstAll[warp][lane] = suffixWarp ? pre + L : pre;
+        lenAll[warp][lane] = on ? L : 0;
+        XS *val = tmp + tmpOff[ji] + (suffixWarp ? 32 * ((size_t)Lmax + 1) : 0);
+        pairSync();  // the previous job's table and bases are no longer read
+        // each warp of the pair fills half of the table (scaleScore gives zero
+        // for a factor that is not positive and finite)
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    v[u] = (c0 + u < ncol) ? pfx[(size_t)(j0 + c0 + u) * 32 + lane] : xsZero();
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int c = c0 + u;
-                    if (c >= ncol) break;
-                    const int j = j0 + c;
-                    stage[c][lane] = packScore(batchMul(v[u], runPre));
-                    runPre = batchMul(runPre, perBase);
-                    if (j < L - 1) running = batchMul(running, perBase);
-                }
+        for (int c = 0; c < 13; ++c) {
+            const int code = 2 * c + (suffixWarp ? 1 : 0);
+            const double f = __dmul_rn(code < kNumCodes ? (double)bg[code] : 0.0, keep);
+            tabAll[jw][code][lane] = f > 0.0 && isfinite(f) ? f : 0.0;
+        }
+        pairSync();
+        const double *tab = &tabAll[jw][0][lane];
+        if (suffixWarp) {
+            if (anyZero)
+                suffixPass<true>(cd, L, Lmax, tab, keep, val, lane, sNE, dNE);
+            else
+                suffixPass<false>(cd, L, Lmax, tab, keep, val, lane, sNE, dNE);
+        } else {
+            const float bg0 = bg[cd[0]];
+            if (anyZero)
+                prefixPass<true>(cd, L, Lmax, tab, bg0, val, lane, sNE, dNE);
+            else
+                prefixPass<false>(cd, L, Lmax, tab, bg0, val, lane, sNE, dNE);
+            // Total and scales (dummest-dp-backward.hh:103-129).
+            const XS p1 = val[(size_t)(L - 1) * 32 + lane];
+            const XS p2 = L > 1 ? val[(size_t)(L - 2) * 32 + lane] : xsZero();
+            const XS p3 = L > 2 ? val[(size_t)(L - 3) * 32 + lane] : xsZero();
+            const double keepSingle = 1.0 - r.single;
+            const double keepBoth = keepSingle - r.dbl;
+            const XS trailingSingle = scaleScore(p2, keepSingle * 0.25);
+            const XS trailingDouble = scaleScore(p3, keepBoth * 0.0625);
+            const XS total = scalarAdd(scalarAdd(p1, trailingSingle), trailingDouble);
+            const float nullLog = (total.m == 0.0f) ? -INFINITY : (float)(log2((double)total.m) + (double)total.e);
+            double perBaseLog = -(double)nullLog / (double)L;
+            if (!(perBaseLog < 120.0)) perBaseLog = 120.0;
+            const double perBaseRaw = exp2(perBaseLog);
+            const XS perBase = splitNorm(perBaseRaw, 0);
+            baseAll[jw][0][lane] = perBase;
+            baseAll[jw][1][lane] = splitNorm(1.0 / perBaseRaw, 0);
+            if (on) {
+                const XS quarter = splitNorm(0.25, 0), sixteenth = splitNorm(0.0625, 0);
+                PairScales sc;
+                sc.s1 = packScore(scalarMul(perBase, quarter));
+                sc.s2 = packScore(scalarMul(scalarMul(perBase, perBase), sixteenth));
+                sc.sC = packScore(scalarMul(scalarMul(perBase, perBase), perBase));
+                sc.pad = 0.0f;
+                scales[pi] = sc;
             }
-            flushSeeds(stage, dstAll[warp][0], job.count, j0, ncol, lane);
         }
-
-        // Pass 3: suffix seeds (dummest-dp-backward.hh:146-154).
-        for (int j0 = 0; j0 < L; j0 += 32) {
-            const int ncol = L - j0 < 32 ? L - j0 : 32;
-            for (int c0 = 0; c0 < ncol; c0 += 8) {
-                XS v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int j = j0 + c0 + u;
-                    v[u] = (c0 + u < ncol && j + 1 < L) ? sfx[(size_t)(j + 1) * 32 + lane] : pow2Score(0);
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int c = c0 + u;
-                    if (c >= ncol) break;
-                    stage[c][lane] = packScore(batchMul(v[u], running));
-                    running = batchMul(running, perBaseInv);
-                }
+        pairSync();
+        const XS perBase = baseAll[jw][0][lane], perBaseInv = baseAll[jw][1][lane];
+        if (suffixWarp) {
+            // the suffix seeds' power starts at perBase^(L-1), one rounded product at a time
+            XS running = pow2Score(0);
+            for (int k = 1; k < Lmax; ++k) {
+                const XS t = mulF(running, perBase);
+                if (k < L) running = t;
             }
-            flushSeeds(stage, dstAll[warp][1], job.count, j0, ncol, lane);
+            seedPass<true>(val, L, Lmax, running, perBaseInv, stage, dstAll[warp], lenAll[warp], job.count, lane);
+        } else {
+            seedPass<false>(val, L, Lmax, perBase, perBase, stage, dstAll[warp], lenAll[warp], job.count, lane);
         }
-        __syncwarp();
     }
 }
 
