@@ -6,6 +6,7 @@
 #include "dp_exact.cuh"
 #include "dp_adjoint.cuh"
 #include "dp_posterior.cuh"
+#include "dp_pipe.cuh"
 #include "dp_plain.cuh"
 #include "dp_exact_wave.cuh"
 #include "dp_search.cuh"
@@ -415,6 +416,38 @@ DpKern dpKernelFor(int R, bool mid, int warps, bool gt) {
     return gt ? dpKernelShape<true>(R, mid, warps) : dpKernelShape<false>(R, mid, warps);
 }
 
+// The stripe pipeline's schedule of a call: rows per lane, warps per CTA, CTAs
+// per cluster and clusters (clusters = 0: one warp per pair instead).
+using PipeKern = void (*)(PipeArgs);
+template <bool MID>
+PipeKern pipeKernelByR(int R) {
+    return R == 4 ? pipeKernel<4, MID> : (R == 2 ? pipeKernel<2, MID> : pipeKernel<1, MID>);
+}
+PipeKern pipeKernelFor(int R, bool mid) { return mid ? pipeKernelByR<true>(R) : pipeKernelByR<false>(R); }
+inline size_t pipeWindowBytes(int R) {
+    return R == 4 ? sizeof(WindowP<4>) : (R == 2 ? sizeof(WindowP<2>) : sizeof(WindowP<1>));
+}
+struct PipePlan {
+    int R = 1, W = 1, C = 1, clusters = 0;
+    PipeKern kern = nullptr;
+    size_t smem = 0;
+    long long w1Slot = 0, ringSlot = 0;  // floats, entries
+};
+// Launch configuration of a grid of plan.C-CTA clusters.
+cudaLaunchConfig_t pipeLaunch(const PipePlan &plan, int ctas, cudaLaunchAttribute *at, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg{};
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = plan.C;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(plan.W * kLanes);
+    cfg.dynamicSmemBytes = plan.smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 using PlainKern = void (*)(const DevPair *, int, const DevProfile *, const float *, const float *, const uint8_t *,
                           const float *, const PairScales *, float *, PairOut *, int);
 template <bool MID>
@@ -516,6 +549,7 @@ struct CallSlot {
     PinnedBuf<int> hAnchorE, hAnchorRow;
     PinnedBuf<DevPair> hPairs;
     PinnedBuf<Chunk> hChunks;
+    PinnedBuf<int> hPipeList;
     PinnedBuf<NullJob> hNullJobs;
     PinnedBuf<int> hJobPairs;
     PinnedBuf<long long> hNullTmpOff;
@@ -530,7 +564,7 @@ struct CallSlot {
     bool pending = false;
     size_t n = 0;
     int mode = 0;
-    bool mid = false, nullOnly = false, sequentialExact = false, exactOnDevice = false, search = false;
+    bool mid = false, nullOnly = false, sequentialExact = false, exactOnDevice = false, search = false, pipe = false;
     dmst_score *anchorBest = nullptr;  // anchors: the caller's outputs (columns in the caller's pair order)
     int *anchorRowOut = nullptr;
     long long anchorCols = 0;
@@ -602,6 +636,9 @@ struct dmst_ctx {
     DevBuf<Chunk> dChunks;
     DevBuf<int> dCounter;
     DevBuf<float> dW1, dRing;
+    DevBuf<unsigned long long> dPipeRing;    // stripe pipeline: boundary rows, kRingEmpty between kernels
+    DevBuf<int> dPipeList, dPipeAbort;       // ... pair positions; an abort flag per cluster
+    bool pipeClean = false;                  // the ring and the flags are as a kernel expects them
     DevBuf<ExactJob> dJobs;
     DevBuf<AdjointJob> dAdjJobs;             // dmst_loglik_grad, dmst_posteriors
     int adjCheckpoint = DMST_ADJ_CKPT_AUTO;   // dmst_adjoint_checkpoint
@@ -759,6 +796,7 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
         sl.dQueueCount.release();
         sl.hPairs.release();
         sl.hChunks.release();
+        sl.hPipeList.release();
         sl.hNullJobs.release();
         sl.hJobPairs.release();
         sl.hNullTmpOff.release();
@@ -818,6 +856,9 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
     ctx->dCounter.release();
     ctx->dW1.release();
     ctx->dRing.release();
+    ctx->dPipeRing.release();
+    ctx->dPipeList.release();
+    ctx->dPipeAbort.release();
     ctx->dJobs.release();
     ctx->dAdjJobs.release();
     ctx->dAdjF.release();
@@ -1510,6 +1551,75 @@ static float elapsedMs(dmst_ctx *ctx, cudaEvent_t a, cudaEvent_t b) {
     return ms;
 }
 
+// The stripe pipeline's shape for n pairs whose rows average `rows` (weighted
+// by cells).
+//
+// Two rows per lane (one when a single 32-row stripe holds the profile) were
+// the fastest or within 5% of it over M = 20-2000, L = 200-10000 and 2-1200
+// pairs: one row doubles the boundary values and steps, four rows double the
+// time of a step and the fill.  The warps of a pair (g) share the GPU's 12
+// warps per SM among the pairs, in equal rounds over the stripes, and few
+// pairs are spread over a cluster of CTAs, so that every SM has work.
+static int pipeShape(dmst_ctx *ctx, size_t n, double rows, PipePlan &plan) {
+    const int stripes = std::max(1, (int)std::ceil(rows / (kLanes * plan.R)));
+    const size_t sm = (size_t)ctx->smCount;
+    const int share = (int)std::max<size_t>(1, 12 * sm / n);
+    const int rounds = (stripes + std::min(share, stripes) - 1) / std::min(share, stripes);
+    const int g = (stripes + rounds - 1) / rounds;
+    plan.C = 1;
+    while (plan.C < kPipeMaxCluster && 2 * plan.C <= g && 2 * plan.C * n <= sm) plan.C *= 2;
+    const int maxW = (int)std::min<size_t>(pipeMaxWarps(plan.R), ((size_t)ctx->maxSmemOptin - 1024) / pipeWindowBytes(plan.R));
+    const int perCta = (g + plan.C - 1) / plan.C;
+    plan.W = (perCta + (perCta + maxW - 1) / maxW - 1) / ((perCta + maxW - 1) / maxW);
+    plan.smem = (size_t)plan.W * pipeWindowBytes(plan.R);
+    CK(cudaFuncSetAttribute(plan.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem), "smem attribute");
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = pipeLaunch(plan, plan.C * ctx->smCount, &at, nullptr);
+    int resident = 0;
+    CK(cudaOccupancyMaxActiveClusters(&resident, plan.kern, &cfg), "cluster occupancy");
+    if (resident < 1) return ctx->fail(DMST_ERANGE, "kernel does not fit on an SM");
+    plan.clusters = (int)std::min<size_t>(resident, n);
+    return DMST_OK;
+}
+
+// The stripe pipeline runs calls of at most six pairs per SM: half of what the
+// batched kernel holds at one warp per pair.  Measured DP times, batched with
+// tuned shapes against the pipeline (M, L, pairs): (2000, 10000, 16) 36.5 / 2.85
+// ms, (300, 3100, 200) 1.88 / 0.91, (300, 3100, 600) 2.60 / 2.05, (800, 3000,
+// 400) 4.34 / 3.04; beyond the line (300, 3100, 1500) 3.84 / 4.42, (800, 3000,
+// 1200) 8.42 / 8.72, (100, 1000, 3000) 1.08 / 1.30.
+static int pipePlan(dmst_ctx *ctx, const std::vector<DevPair> &dp, bool mid, PipePlan &plan) {
+    const size_t n = dp.size();
+    if (n > 6 * (size_t)ctx->smCount) return DMST_OK;
+    double cells = 0, weighted = 0;
+    int maxM = 0;
+    for (const DevPair &d : dp) {
+        const double c = (double)(d.M + 1) * d.L;
+        cells += c;
+        weighted += c * (d.M + 1);
+        maxM = std::max(maxM, d.M);
+    }
+    plan.R = maxM < kLanes ? 1 : 2;
+    plan.kern = pipeKernelFor(plan.R, mid);
+    for (const DevPair &d : dp) {
+        if (mid) plan.w1Slot = std::max(plan.w1Slot, pipeW1Floats(d.M, d.L, plan.R));
+        plan.ringSlot = std::max(plan.ringSlot, pipeRingEntries(d.M, d.L, plan.R));
+    }
+    plan.w1Slot = (plan.w1Slot + 63) / 64 * 64;
+    if (const int st = pipeShape(ctx, n, weighted / cells, plan)) return st;
+    // the slots within the device budget
+    const size_t slotBytes = (size_t)plan.w1Slot * sizeof(float) + (size_t)plan.ringSlot * sizeof(unsigned long long);
+    size_t budget = ctx->opts.device_budget_bytes;
+    const size_t held = ctx->dW1.cap * sizeof(float) + ctx->dPipeRing.cap * sizeof(unsigned long long);
+    if (!budget && plan.clusters * slotBytes > held) {
+        size_t freeB = 0, totalB = 0;
+        CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
+        budget = (size_t)(0.6 * (double)(freeB + held));
+    }
+    if (budget) plan.clusters = (int)std::max<size_t>(1, std::min<size_t>(plan.clusters, budget / slotBytes));
+    return DMST_OK;
+}
+
 // Internal mode bit: set up the pairs and run the null model only (the
 // device pair descriptors, seeds and scales of the call stay in the context).
 constexpr int kModeNullOnly = 0x10000;
@@ -1636,6 +1746,10 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         if (mid) w1Max = std::max(w1Max, (size_t)stagSlotFloats(d.M, d.L, d.R));
         ringMax = std::max(ringMax, 2 * (size_t)stagPeriod(d.L, d.R));
     }
+    PipePlan pipe;
+    if (!plain && !nullOnly && !forceExact && !search && !ctx->tune.forceR && ctx->opts.rows_per_lane == 0 &&
+        (st = pipePlan(ctx, dp, mid, pipe)))
+        return st;
     // Kernel groups by shape.  Chunks: runs of pairs of one profile and shape,
     // costliest first within each group.
     struct Group {
@@ -1689,7 +1803,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     // and the like keep them for the next such call) are given up when the
     // slots of a full GPU (every SM at the widest CTA) would not fit without them.
     size_t maxSlots = SIZE_MAX;
-    if (mid && !nullOnly) {
+    if (mid && !nullOnly && !pipe.clusters) {
         size_t freeB = 0, totalB = 0;
         CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
         const size_t held = (ctx->dW1.cap + ctx->dRing.cap) * sizeof(float);
@@ -1730,7 +1844,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         chunkPairsOf[q] =
             plain ? 1 : (int)std::max<long long>(1, std::min<long long>(4LL * G.warps, std::max(floorPairs, perCta)));
     }
-    for (size_t k = 0; k < n && !nullOnly;) {
+    for (size_t k = 0; k < n && !nullOnly && !pipe.clusters;) {
         Group &G = groups[groupOf(k)];
         size_t e = k;
         double cost = 0;
@@ -1798,7 +1912,27 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     // 25% headroom: the slot size follows the call's longest pairs and their
     // kernel shapes, so calls of one workload vary, and a grown W1 buffer
     // (tens of GB) costs the host a long allocation
-    CK(ctx->dW1.ensure(std::max<size_t>(std::max(slotsMax * w1Slot, plainScratch), 1), 0.25), "alloc W1 slots");
+    CK(ctx->dW1.ensure(std::max<size_t>({slotsMax * w1Slot, plainScratch, (size_t)(pipe.clusters * pipe.w1Slot), 1}), 0.25),
+       "alloc W1 slots");
+    if (pipe.clusters) {
+        const size_t entries = (size_t)(pipe.clusters * pipe.ringSlot);
+        if (entries > ctx->dPipeRing.cap || (size_t)pipe.clusters > ctx->dPipeAbort.cap) ctx->pipeClean = false;
+        CK(ctx->dPipeRing.ensure(entries, 0.25), "alloc stripe rings");
+        CK(ctx->dPipeAbort.ensure(pipe.clusters), "alloc stripe rings");
+        if (!ctx->pipeClean) {
+            CK(cudaMemsetAsync(ctx->dPipeRing.p, 0xff, ctx->dPipeRing.cap * sizeof(unsigned long long), ctx->stream),
+               "empty stripe rings");
+            CK(cudaMemsetAsync(ctx->dPipeAbort.p, 0, ctx->dPipeAbort.cap * sizeof(int), ctx->stream), "zero abort flags");
+            ctx->pipeClean = true;
+        }
+        std::vector<int> list(n);
+        std::iota(list.begin(), list.end(), 0);
+        std::stable_sort(list.begin(), list.end(), [&](int x, int y) {
+            return (long long)(dp[x].M + 1) * dp[x].L > (long long)(dp[y].M + 1) * dp[y].L;
+        });
+        CK(ctx->dPipeList.ensure(n), "alloc pair list");
+        if ((st = upload(S.hPipeList, ctx->dPipeList.p, list.data(), n, "upload pair list"))) return st;
+    }
     CK(ctx->dRing.ensure(std::max<size_t>(slotsMax * ringSlot, 1), 0.25), "alloc ring slots");
     // one counter per group (search: the second wave's after them; the one-warp plain schedule: one per chunk)
     const size_t nCounters = std::max<size_t>(allChunks.size() + kNumShapes, 2 * kNumShapes);
@@ -2030,7 +2164,16 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
             CK(cudaGetLastError(), "survivor kernel");
             ++launches;
         }
-        if (!forceExact && !nullOnly) {
+        if (pipe.clusters) {
+            CK(cudaMemsetAsync(S.dOut.p, 0, n * sizeof(PairOut), ctx->stream), "zero results");
+            PipeArgs pa{ctx->dPipeList.p, nullptr, (int)n, g.pairs, g.profiles, g.emit, g.params, g.codes, g.seeds,
+                        g.scales, ctx->dW1.p, pipe.w1Slot, ctx->dPipeRing.p, pipe.ringSlot, ctx->dPipeAbort.p,
+                        S.dOut.p};
+            cudaLaunchAttribute at;
+            const cudaLaunchConfig_t cfg = pipeLaunch(pipe, pipe.clusters * pipe.C, &at, ctx->stream);
+            CK(cudaLaunchKernelEx(&cfg, pipe.kern, pa), "stripe pipeline kernel");
+            ++launches;
+        } else if (!forceExact && !nullOnly) {
             for (int gi = 0; gi < kNumShapes; ++gi) {
                 Group &G = groups[gi];
                 if (G.chunks.empty()) continue;
@@ -2095,6 +2238,10 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                                       (uintptr_t)exactGroups,
                                       (uintptr_t)S.dExOut.p, (uintptr_t)S.dQueue.p, (uintptr_t)S.dQueueCount.p,
                                       (uintptr_t)S.hOut.p, (uintptr_t)S.hExOut.p};
+        for (uintptr_t v : {(uintptr_t)pipe.kern, (uintptr_t)pipe.clusters, (uintptr_t)pipe.C, (uintptr_t)pipe.W,
+                            (uintptr_t)pipe.w1Slot, (uintptr_t)pipe.ringSlot, (uintptr_t)ctx->dPipeRing.p,
+                            (uintptr_t)ctx->dPipeList.p, (uintptr_t)ctx->dPipeAbort.p})
+            key.push_back(v);
         for (const Group &G : groups) {
             const uintptr_t v[8] = {(uintptr_t)G.kern, (uintptr_t)G.grid,         (uintptr_t)G.warps,
                                     (uintptr_t)G.smem, (uintptr_t)G.chunks.size(), (uintptr_t)G.chunkBase,
@@ -2192,6 +2339,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     S.sequentialExact = sequentialExact;
     S.exactOnDevice = exactOnDevice;
     S.search = search;
+    S.pipe = pipe.clusters > 0;
     S.anchorBest = anchorBest;
     S.anchorRowOut = anchorRow;
     S.anchorCols = anchorCols;
@@ -2236,6 +2384,12 @@ static int completeCall(dmst_ctx *ctx) {
     const bool search = S.search;
     const uint8_t *survived = search ? S.hMask.p : nullptr;
     const PairOut *pf = search ? S.hOutF.p : nullptr;
+    if (S.pipe)
+        for (size_t k = 0; k < n; ++k)
+            if (std::isnan(po[k].filt)) {  // a wait of the stripe pipeline ran out: its rings are not empty
+                ctx->pipeClean = false;
+                if (!mid) return ctx->fail(DMST_ETIMEOUT, "the stripe pipeline of pair %d gave up a wait", order[k]);
+            }
     // Pairs outside the fast path's exact range go to the row-rescaled kernel.
     std::vector<int> flagged;
     for (size_t k = 0; k < n; ++k) {

@@ -146,8 +146,16 @@ __device__ __forceinline__ void storeW1S(float *p, const float (&w)[R]) {
         storeW1<R>(p, w);
 }
 
-__device__ __forceinline__ void ringStoreS(float *ring, int col, float w, float y) {
-    __stcg(reinterpret_cast<float2 *>(ring) + col, make_float2(w, y));
+// A ring entry.  SHARED: read by another warp (dp_pipe.cuh), so one 64-bit
+// store, of which a reader sees both values or neither.
+template <bool SHARED>
+__device__ __forceinline__ void ringStoreS(float2 *p, float w, float y) {
+    if constexpr (SHARED) {
+        const unsigned long long v = ((unsigned long long)__float_as_uint(y) << 32) | __float_as_uint(w);
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    } else {
+        __stcg(p, make_float2(w, y));
+    }
 }
 
 // The window's first entries: local times [-S, kSBlock) now (the leading rows
@@ -214,14 +222,17 @@ struct BwdS {
     const float *eG;  // or the global address (tall profiles)
 };
 
-template <int R, bool MID, int PH, bool GEN, bool SH>
+// PIPE: the sweep is one stripe, whose coefficients the caller has loaded, and
+// its ring is read by another warp (dp_pipe.cuh); otherwise a lane loads its
+// coefficients when its leading row starts a stripe.
+template <int R, bool MID, int PH, bool GEN, bool SH, bool PIPE = false>
 __device__ __forceinline__ void bwdStepS(BwdS<R> &b, const SweepArgs &a, WindowS<R> &win, int lane,
                                          bool ringWriter, const RunPtrs &ip) {
     constexpr int S = kLanes * R;
     constexpr int SW = kLanes * stagLaneStride(R);  // floats per W1 group
     float inW = __shfl_down_sync(kFull, b.sendW, 1);
     float inY = __shfl_down_sync(kFull, b.sendY, 1);
-    if (GEN && b.u >= 0 && b.jj == 0 && b.sp < a.nS) {
+    if (GEN && !PIPE && b.u >= 0 && b.jj == 0 && b.sp < a.nS) {
         // the leading row starts a stripe; the lane's other rows are idle
         const int rowBase = (a.nS - 1 - b.sp) * S + lane * R;
         loadBackwardCoef<R>(b.c, a, rowBase);
@@ -318,7 +329,7 @@ __device__ __forceinline__ void bwdStepS(BwdS<R> &b, const SweepArgs &a, WindowS
         if (MID) storeW1S<R>(b.wp, nW);
         b.wp += SW;
         if (lane == 0 && b.u >= 0 && b.sp < a.nS - 1 && b.jj >= R - 1 && b.jj < a.L + R - 1)
-            ringStoreS(a.ring, b.jj - (R - 1), nW[0], nY[0]);
+            ringStoreS<PIPE>(reinterpret_cast<float2 *>(a.ring) + (b.jj - (R - 1)), nW[0], nY[0]);
         if (b.u >= 0 && ++b.jj == a.P) {
             b.jj = 0;
             ++b.sp;
@@ -326,7 +337,7 @@ __device__ __forceinline__ void bwdStepS(BwdS<R> &b, const SweepArgs &a, WindowS
         ++b.u;
     } else {  // the run advances u, jj and the W1 pointer
         if (MID) storeW1S<R>(ip.w1 + PH * SW, nW);
-        if (ringWriter) __stcg(ip.ringOut + PH, make_float2(nW[0], nY[0]));
+        if (ringWriter) ringStoreS<PIPE>(ip.ringOut + PH, nW[0], nY[0]);
     }
 }
 
@@ -438,7 +449,7 @@ __device__ __forceinline__ void cpAsyncStage(float *dst, const float *src) {
     }
 }
 
-template <int R, int PH, bool GEN, bool SH>
+template <int R, int PH, bool GEN, bool SH, bool PIPE = false>
 __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS<R> &win, int lane,
                                          bool ringWriter, const RunPtrs &ip) {
     constexpr int S = kLanes * R;
@@ -467,7 +478,7 @@ __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS
     }
     float inW = __shfl_up_sync(kFull, f.sendIn, 1);
     float inY = __shfl_up_sync(kFull, f.sendY, 1);
-    if (GEN && f.u >= 0 && f.jj == 0 && f.sp < a.nS) {
+    if (GEN && !PIPE && f.u >= 0 && f.jj == 0 && f.sp < a.nS) {
         const int rowBase = f.sp * S + lane * R;
         loadForwardCoef<R>(f.c, a, rowBase);
         if (SH)
@@ -542,7 +553,7 @@ __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS
     // the stage for the step kSW1Ahead later goes into the slot read one step ago
     if (GEN) {
         if (lane == kLanes - 1 && f.u >= 0 && f.sp < a.nS - 1 && f.jj >= R - 1 && f.jj < a.L + R - 1)
-            ringStoreS(a.ring, f.jj - (R - 1), nN[R - 1], nY[R - 1]);
+            ringStoreS<PIPE>(reinterpret_cast<float2 *>(a.ring) + (f.jj - (R - 1)), nN[R - 1], nY[R - 1]);
         if (f.gAhead >= 0) cpAsyncStage<R>(&win.w1[(PH + kSW1Ahead) % kSW1Slots][lane * stagLaneStride(R)], f.w1src);
         cpAsyncCommit();
         f.w1src -= SW;
@@ -553,7 +564,7 @@ __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS
         }
         ++f.u;
     } else {  // the run advances u, jj and the staging cursor
-        if (ringWriter) __stcg(ip.ringOut + PH, make_float2(nN[R - 1], nY[R - 1]));
+        if (ringWriter) ringStoreS<PIPE>(ip.ringOut + PH, nN[R - 1], nY[R - 1]);
         cpAsyncStage<R>(&win.w1[(PH + kSW1Ahead) % kSW1Slots][lane * stagLaneStride(R)], ip.w1 - PH * SW);
         cpAsyncCommit();
     }
