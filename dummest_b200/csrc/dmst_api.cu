@@ -489,11 +489,35 @@ inline int lengthClass(int L) { return L < kShortRead ? 1 : 0; }
 // cells per millisecond.
 struct Tuning {
     bool tuned = false;
-    int warps[2][kNumR] = {{kCtaWarps, kCtaWarps, kCtaWarps, kCtaWarps}, {kCtaWarps, kCtaWarps, kCtaWarps, kCtaWarps}};
+    int warps[2][kNumR] = {{kCtaWarpsMid, kCtaWarpsMid, kCtaWarpsMid, kCtaWarpsMid},
+                           {kCtaWarpsMid, kCtaWarpsMid, kCtaWarpsMid, kCtaWarpsMid}};
     double rate[2][kNumR] = {};
     double rates[2][kNumR][3] = {};  // per class, R, kShapeWarps: the measured rates (cells per ms)
     int forceR = 0, forceWarps = 0;  // set while the autotuner measures one shape
 };
+
+// Rows per lane of an untuned pair: the least expected time, steps of a sweep
+// times the cost of a step.  The costs (relative, of a step of 128, 96, 64 and
+// 32 cells) are 32 R over the rates of 12-warp CTAs on the batched
+// configuration: 300, 292, 229 and 146 GCUPS of computed cells; counting
+// steps instead of rows puts a sweep's fill and the shortest stripe period
+// (stagPeriod) in, which is what decides for short reads.  Over M = 40-2000
+// and L = 75-3000 12-warp CTAs lead for almost every size, R = 2 up to about
+// 300 nt and where a 128-row stripe pads, R = 4 elsewhere; four rows on 16
+// warps (128 registers), the default before, took 1.2-2.4 times as long.
+constexpr double kStepCost[kNumR] = {128 / 300.0, 96 / 292.0, 64 / 229.0, 32 / 146.0};
+int untunedR(int M, int L) {
+    int R = 4;
+    double least = 1e300;
+    for (int q = 0; q < kNumR; ++q) {
+        const double t = (double)stagSteps(M, L, kShapeR[q]) * kStepCost[q];
+        if (t < least) {
+            least = t;
+            R = kShapeR[q];
+        }
+    }
+    return R;
+}
 
 // The kernel shape of a pair of a profile of length M and a read of length L.
 void shapeOf(int M, int L, int forced, const Tuning &t, int &R, int &W) {
@@ -503,8 +527,7 @@ void shapeOf(int M, int L, int forced, const Tuning &t, int &R, int &W) {
     } else if (t.forceR) {
         R = t.forceR;
     } else if (!t.tuned) {
-        // Untuned default: four rows per lane.
-        R = 4;
+        R = untunedR(M, L);
     } else {
         // Tuned: the R with the least expected time (computed rows / rate).
         R = 4;
@@ -1694,12 +1717,12 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         }
     }
     // The kernel shape of every pair (rows per lane and warps per CTA, from
-    // the profile's length and the read's length class).  With tuned shapes,
-    // a shape group too small to give every CTA two chunks would run as its
+    // the profile's length and the read's length or its class).  A shape group too small to give every CTA two chunks would run as its
     // own underfilled launch; its pairs join the largest group instead.
     std::vector<int> pairShape(n);
     {
-        // the shape depends on the profile and the read's length class only
+        // tuned (or forced), the shape depends on the profile and the read's length class only
+        const bool byLength = !ctx->tune.tuned && !ctx->tune.forceR && ctx->opts.rows_per_lane == 0;
         const size_t nProf = ctx->profiles.size();
         std::vector<int> shapeTab(2 * nProf);
         for (size_t q = 0; q < nProf; ++q)
@@ -1711,10 +1734,18 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
             }
         long long groupPairs[kNumShapes] = {};
         for (size_t i = 0; i < n; ++i) {
-            pairShape[i] = shapeTab[2 * (size_t)pairs[i].profile + lengthClass(ctx->seqLen[pairs[i].seq])];
+            const int L = ctx->seqLen[pairs[i].seq];
+            if (byLength) {
+                int R, W;
+                shapeOf(ctx->profiles[pairs[i].profile].M, L, 0, ctx->tune, R, W);
+                if (plainStriped && R == 3) R = 4;
+                pairShape[i] = rIndex(R) * 3 + wIndex(W);
+            } else {
+                pairShape[i] = shapeTab[2 * (size_t)pairs[i].profile + lengthClass(L)];
+            }
             ++groupPairs[pairShape[i]];
         }
-        if (ctx->tune.tuned && !ctx->tune.forceR && ctx->opts.rows_per_lane == 0 && !plain) {
+        if (!ctx->tune.forceR && ctx->opts.rows_per_lane == 0 && !plain) {
             int big = 0;
             for (int q = 1; q < kNumShapes; ++q)
                 if (groupPairs[q] > groupPairs[big]) big = q;
