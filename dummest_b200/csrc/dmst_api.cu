@@ -5,6 +5,7 @@
 #include "dp_common.cuh"
 #include "dp_exact.cuh"
 #include "dp_adjoint.cuh"
+#include "dp_adjoint_pipe.cuh"
 #include "dp_posterior.cuh"
 #include "dp_pipe.cuh"
 #include "dp_plain.cuh"
@@ -433,15 +434,15 @@ struct PipePlan {
     size_t smem = 0;
     long long w1Slot = 0, ringSlot = 0;  // floats, entries
 };
-// Launch configuration of a grid of plan.C-CTA clusters.
-cudaLaunchConfig_t pipeLaunch(const PipePlan &plan, int ctas, cudaLaunchAttribute *at, cudaStream_t stream) {
+// Launch configuration of `ctas` CTAs of W warps in clusters of C.
+cudaLaunchConfig_t clusterLaunch(int C, int W, size_t smem, int ctas, cudaLaunchAttribute *at, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     at->id = cudaLaunchAttributeClusterDimension;
-    at->val.clusterDim.x = plan.C;
+    at->val.clusterDim.x = C;
     at->val.clusterDim.y = at->val.clusterDim.z = 1;
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(plan.W * kLanes);
-    cfg.dynamicSmemBytes = plan.smem;
+    cfg.blockDim = dim3(W * kLanes);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
@@ -664,6 +665,7 @@ struct dmst_ctx {
     bool pipeClean = false;                  // the ring and the flags are as a kernel expects them
     DevBuf<ExactJob> dJobs;
     DevBuf<AdjointJob> dAdjJobs;             // dmst_loglik_grad, dmst_posteriors
+    DevBuf<int> dAdjStatus;                  // ... per job, then the launch's abort flag
     int adjCheckpoint = DMST_ADJ_CKPT_AUTO;   // dmst_adjoint_checkpoint
     bool lastAdjCheckpointed = false;
     DevBuf<double> dPost;                    // dmst_posteriors: the batch's posterior tables
@@ -884,6 +886,7 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
     ctx->dPipeAbort.release();
     ctx->dJobs.release();
     ctx->dAdjJobs.release();
+    ctx->dAdjStatus.release();
     ctx->dAdjF.release();
     ctx->dAdjB.release();
     ctx->dGrad.release();
@@ -1574,30 +1577,38 @@ static float elapsedMs(dmst_ctx *ctx, cudaEvent_t a, cudaEvent_t b) {
     return ms;
 }
 
+// Warps of a CTA and CTAs of a cluster for n pairs of `stripes` stripes each,
+// at most maxW warps per CTA and warpsPerSm on an SM: the warps of a pair share
+// the GPU's warps with the other pairs, in equal rounds over the stripes, and
+// few pairs are spread over a cluster of CTAs, so that every SM has work.  A
+// pair gets at least `least` warps (as far as it has stripes).
+static void pipeSpread(const dmst_ctx *ctx, size_t n, int stripes, int maxW, int warpsPerSm, int least, int &W, int &C) {
+    const size_t sm = (size_t)ctx->smCount;
+    const int share = std::min(stripes, (int)std::max<size_t>(least, warpsPerSm * sm / n));
+    const int rounds = (stripes + share - 1) / share;
+    const int g = (stripes + rounds - 1) / rounds;
+    C = 1;
+    while (C < kPipeMaxCluster && 2 * C <= g && 2 * C * n <= sm) C *= 2;
+    const int perCta = (g + C - 1) / C;
+    const int ctaRounds = (perCta + maxW - 1) / maxW;
+    W = (perCta + ctaRounds - 1) / ctaRounds;
+}
+
 // The stripe pipeline's shape for n pairs whose rows average `rows` (weighted
 // by cells).
 //
 // Two rows per lane (one when a single 32-row stripe holds the profile) were
 // the fastest or within 5% of it over M = 20-2000, L = 200-10000 and 2-1200
 // pairs: one row doubles the boundary values and steps, four rows double the
-// time of a step and the fill.  The warps of a pair (g) share the GPU's 12
-// warps per SM among the pairs, in equal rounds over the stripes, and few
-// pairs are spread over a cluster of CTAs, so that every SM has work.
+// time of a step and the fill.  Twelve warps per SM.
 static int pipeShape(dmst_ctx *ctx, size_t n, double rows, PipePlan &plan) {
     const int stripes = std::max(1, (int)std::ceil(rows / (kLanes * plan.R)));
-    const size_t sm = (size_t)ctx->smCount;
-    const int share = (int)std::max<size_t>(1, 12 * sm / n);
-    const int rounds = (stripes + std::min(share, stripes) - 1) / std::min(share, stripes);
-    const int g = (stripes + rounds - 1) / rounds;
-    plan.C = 1;
-    while (plan.C < kPipeMaxCluster && 2 * plan.C <= g && 2 * plan.C * n <= sm) plan.C *= 2;
     const int maxW = (int)std::min<size_t>(pipeMaxWarps(plan.R), ((size_t)ctx->maxSmemOptin - 1024) / pipeWindowBytes(plan.R));
-    const int perCta = (g + plan.C - 1) / plan.C;
-    plan.W = (perCta + (perCta + maxW - 1) / maxW - 1) / ((perCta + maxW - 1) / maxW);
+    pipeSpread(ctx, n, stripes, maxW, 12, 1, plan.W, plan.C);
     plan.smem = (size_t)plan.W * pipeWindowBytes(plan.R);
     CK(cudaFuncSetAttribute(plan.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem), "smem attribute");
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = pipeLaunch(plan, plan.C * ctx->smCount, &at, nullptr);
+    const cudaLaunchConfig_t cfg = clusterLaunch(plan.C, plan.W, plan.smem, plan.C * ctx->smCount, &at, nullptr);
     int resident = 0;
     CK(cudaOccupancyMaxActiveClusters(&resident, plan.kern, &cfg), "cluster occupancy");
     if (resident < 1) return ctx->fail(DMST_ERANGE, "kernel does not fit on an SM");
@@ -2201,7 +2212,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                         g.scales, ctx->dW1.p, pipe.w1Slot, ctx->dPipeRing.p, pipe.ringSlot, ctx->dPipeAbort.p,
                         S.dOut.p};
             cudaLaunchAttribute at;
-            const cudaLaunchConfig_t cfg = pipeLaunch(pipe, pipe.clusters * pipe.C, &at, ctx->stream);
+            const cudaLaunchConfig_t cfg = clusterLaunch(pipe.C, pipe.W, pipe.smem, pipe.clusters * pipe.C, &at, ctx->stream);
             CK(cudaLaunchKernelEx(&cfg, pipe.kern, pa), "stripe pipeline kernel");
             ++launches;
         } else if (!forceExact && !nullOnly) {
@@ -3159,17 +3170,17 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
             o += 2LL * (M + 1) * ctx->seqLen[pairs[i].seq];
         }
     }
-    std::vector<AdjointJob> jobs(n);
-    std::vector<long long> needF(n), needB(n), needP(n);
     // Batches of pairs under the device budget.  The full forward store is
-    // 24 bytes per cell; the checkpointed one keeps the stripes' top rows and
-    // a checkpoint every kAdjCk columns (about 1/12 of it) and recomputes.
-    // Auto: the full store when every pair's fits the budget at once.
-    size_t freeB = 0, totalB = 0;
+    // 24 bytes per cell; the checkpointed one keeps a checkpoint every kAdjCk
+    // columns (about 1/12 of it) and recomputes.  Auto: the full store when
+    // every pair's fits the budget at once.
     CK(cudaSetDevice(ctx->device), "set device");
-    CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
-    const size_t held = (ctx->dAdjF.cap + ctx->dAdjB.cap + ctx->dPost.cap) * sizeof(double);
-    const size_t budget = ctx->opts.device_budget_bytes ? ctx->opts.device_budget_bytes : (freeB + held) / 2;
+    size_t budget = ctx->opts.device_budget_bytes;
+    if (!budget) {
+        size_t freeB = 0, totalB = 0;
+        CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
+        budget = (freeB + (ctx->dAdjF.cap + ctx->dAdjB.cap + ctx->dPost.cap) * sizeof(double)) / 2;
+    }
     long long fullAll = 0;
     for (size_t k = 0; k < n; ++k) {
         const int L = ctx->seqLen[pairs[order[k]].seq];
@@ -3178,19 +3189,11 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
     const bool ckpt = ctx->adjCheckpoint == DMST_ADJ_CKPT_ON ||
                       (ctx->adjCheckpoint == DMST_ADJ_CKPT_AUTO && (size_t)fullAll * 8 > budget);
     ctx->lastAdjCheckpointed = ckpt;
-    for (size_t k = 0; k < n; ++k) {
-        const int L = ctx->seqLen[pairs[order[k]].seq];
-        jobs[k] = AdjointJob{(int)k, 0, 0, 0, tables ? 0 : -1};
-        // 256-byte aligned stores (cp.async)
-        needF[k] = ((ckpt ? adjCkptDoubles(M, L) : adjStoreDoubles(M, L)) + 31) & ~31LL;
-        needB[k] = adjBoundDoubles(L);
-        needP[k] = tables ? 2LL * (M + 1) * L : 0;
-    }
     const size_t gN = (size_t)(M + 2) * kParamFloats + (size_t)(M + 1) * kNumCodes;
     CK(ctx->dGrad.ensure(gN), "alloc gradient");
     CK(ctx->dLogT.ensure(n), "alloc log T");
     CK(ctx->dAdjJobs.ensure(n), "alloc adjoint jobs");
-    CK(cudaMemsetAsync(ctx->dGrad.p, 0, gN * sizeof(double), ctx->stream), "zero gradient");
+    CK(ctx->dAdjStatus.ensure(n + 1), "alloc adjoint status");
     // Summary outputs in the caller's order: pair i's columns at the sum of
     // the earlier pairs' lengths, its rows at i (M+1).
     std::vector<long long> colOff(n + 1, 0);
@@ -3203,71 +3206,149 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
         CK(ctx->dRowMatch.ensure(n * (size_t)(M + 1)), "alloc row sums");
         sumJobs.resize(n);
     }
-    for (size_t k0 = 0; k0 < n;) {
-        size_t k1 = k0;
-        long long f = 0, b = 0, pp = 0;
-        while (k1 < n && (k1 == k0 || (size_t)(f + needF[k1] + b + needB[k1] + pp + needP[k1]) * 8 <= budget)) {
-            jobs[k1].fOff = f;
-            jobs[k1].bOff = b;
-            if (tables) jobs[k1].pOff = pp;
-            f += needF[k1];
-            b += needB[k1];
-            pp += needP[k1];
-            ++k1;
-        }
-        const int nj = (int)(k1 - k0);
-        CK(ctx->dAdjF.ensure((size_t)f), "alloc adjoint store");
-        CK(ctx->dAdjB.ensure((size_t)b), "alloc adjoint rows");
-        if (tables) CK(ctx->dPost.ensure((size_t)std::max<long long>(pp, 1)), "alloc posterior tables");
-        CK(cudaMemcpyAsync(ctx->dAdjJobs.p, jobs.data() + k0, nj * sizeof(AdjointJob), cudaMemcpyHostToDevice,
-                           ctx->stream),
-           "upload adjoint jobs");
-        const int blocks = (nj + kAdjWarps - 1) / kAdjWarps;
-        auto kern = ckpt ? (tables ? adjointKernel<true, true> : adjointKernel<false, true>)
-                         : (tables ? adjointKernel<true> : adjointKernel<false>);
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjSmem), "smem attribute");
-        CK(cudaEventRecord(ctx->ev[3], ctx->stream), "event");
-        kern<<<blocks, kAdjWarps * 32, kAdjSmem, ctx->stream>>>(
-            ctx->dAdjJobs.p, nj, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p, ctx->dCodes.p,
-            S.dSeeds.p, S.dScales.p, ctx->dAdjF.p, ctx->dAdjB.p, ctx->dGrad.p, ctx->dLogT.p + k0,
-            tables ? ctx->dPost.p : nullptr);
-        CK(cudaGetLastError(), "adjoint kernel");
-        ++launches;
-        if (summary) {
-            int maxL = 0;
-            for (size_t k = k0; k < k1; ++k) {
-                const int ci = order[k];
-                const int L = ctx->seqLen[pairs[ci].seq];
-                sumJobs[k] = PostSumJob{jobs[k].pOff, colOff[ci], (long long)ci * (M + 1), M, L};
-                maxL = std::max(maxL, L);
-            }
-            CK(cudaMemcpyAsync(ctx->dPostJobs.p, sumJobs.data() + k0, nj * sizeof(PostSumJob),
-                               cudaMemcpyHostToDevice, ctx->stream),
-               "upload summary jobs");
-            if (colPost || colRow) {
-                postColumnKernel<<<dim3((maxL + kPostThreads - 1) / kPostThreads, nj), kPostThreads, 0, ctx->stream>>>(
-                    ctx->dPostJobs.p, ctx->dPost.p, ctx->dColPost.p, ctx->dColRow.p);
-                CK(cudaGetLastError(), "posterior column kernel");
-                ++launches;
-            }
-            if (rowMatch) {
-                const int rowsPer = kPostThreads / kLanes;
-                postRowKernel<<<dim3((M + 1 + rowsPer - 1) / rowsPer, nj), kPostThreads, 0, ctx->stream>>>(
-                    ctx->dPostJobs.p, ctx->dPost.p, ctx->dRowMatch.p);
-                CK(cudaGetLastError(), "posterior row kernel");
-                ++launches;
-            }
-        }
-        CK(cudaEventRecord(ctx->ev[4], ctx->stream), "event");
-        if (post)
-            for (size_t k = k0; k < k1; ++k)
-                CK(cudaMemcpyAsync(post + postOff[order[k]], ctx->dPost.p + jobs[k].pOff,
-                                   (size_t)needP[k] * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
-                   "download posterior tables");
-        CK(cudaStreamSynchronize(ctx->stream), "adjoint kernel");
-        adjMs += elapsedMs(ctx, ctx->ev[3], ctx->ev[4]);
-        k0 = k1;
+    std::vector<double> lt(n);
+    // The pipelined kernel's shape (stripes of 32 rows), and its grid.  Five
+    // warps per pair also when pairs alone would fill the GPU: with one, the
+    // last pairs run alone (1,024 reads of 600-2400 nt, M = 400: 17.9 ms
+    // checkpointed and 9.2 ms with the full store, against 25.2 and 13.8).
+    int pW = 1, pC = 1, pClusters = 1;
+    auto pipeKern = ckpt ? (tables ? adjointPipeKernel<true, true> : adjointPipeKernel<false, true>)
+                         : (tables ? adjointPipeKernel<true, false> : adjointPipeKernel<false, false>);
+    pipeSpread(ctx, n, adjStripes(M), kAdjPipeWarps, kAdjPipeWarps, 5, pW, pC);
+    {
+        const size_t smem = pW * sizeof(AdjWin);
+        CK(cudaFuncSetAttribute(pipeKern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = clusterLaunch(pC, pW, smem, pC * ctx->smCount, &at, nullptr);
+        CK(cudaOccupancyMaxActiveClusters(&pClusters, pipeKern, &cfg), "cluster occupancy");
+        if (pClusters < 1) return ctx->fail(DMST_ERANGE, "adjoint kernel does not fit on an SM");
     }
+    // Runs the adjoint over the positions `which` (longest read first) in
+    // batches under the budget; pipe: the pipelined kernel, whose per-job
+    // status goes to `status`.
+    auto runBatches = [&](const std::vector<int> &which, bool pipe, std::vector<int> &status) -> int {
+        const size_t m = which.size();
+        std::vector<AdjointJob> jobs(m);
+        std::vector<long long> needF(m), needB(m), needP(m);
+        for (size_t q = 0; q < m; ++q) {
+            const int L = ctx->seqLen[pairs[order[which[q]]].seq];
+            jobs[q] = AdjointJob{which[q], 0, 0, 0, tables ? 0 : -1};
+            // 256-byte aligned stores (cp.async)
+            needF[q] = ((pipe ? (ckpt ? adjPipeCkpt(M, L, pW * pC) : adjPipeFull(M, L))
+                              : (ckpt ? adjCkptDoubles(M, L) : adjStoreDoubles(M, L))) +
+                        31) & ~31LL;
+            needB[q] = pipe ? adjPipeBound(M, L) : adjBoundDoubles(L);
+            needP[q] = tables ? 2LL * (M + 1) * L : 0;
+        }
+        status.assign(m + 1, 0);
+        for (size_t k0 = 0; k0 < m;) {
+            size_t k1 = k0;
+            long long f = 0, b = 0, pp = 0;
+            while (k1 < m && (k1 == k0 || (size_t)(f + needF[k1] + b + needB[k1] + pp + needP[k1]) * 8 <= budget)) {
+                jobs[k1].fOff = f;
+                jobs[k1].bOff = b;
+                if (tables) jobs[k1].pOff = pp;
+                f += needF[k1];
+                b += needB[k1];
+                pp += needP[k1];
+                ++k1;
+            }
+            const int nj = (int)(k1 - k0);
+            CK(ctx->dAdjF.ensure((size_t)f), "alloc adjoint store");
+            CK(ctx->dAdjB.ensure((size_t)b), "alloc adjoint rows");
+            if (tables) CK(ctx->dPost.ensure((size_t)std::max<long long>(pp, 1)), "alloc posterior tables");
+            CK(cudaMemcpyAsync(ctx->dAdjJobs.p, jobs.data() + k0, nj * sizeof(AdjointJob), cudaMemcpyHostToDevice,
+                               ctx->stream),
+               "upload adjoint jobs");
+            CK(cudaEventRecord(ctx->ev[3], ctx->stream), "event");
+            if (pipe) {
+                CK(cudaMemsetAsync(ctx->dAdjB.p, 0xff, (size_t)b * sizeof(double), ctx->stream), "empty adjoint rows");
+                CK(cudaMemsetAsync(ctx->dAdjStatus.p, 0, ((size_t)nj + 1) * sizeof(int), ctx->stream), "zero adjoint status");
+                AdjPipeArgs a{ctx->dAdjJobs.p, nj, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p,
+                              ctx->dCodes.p, S.dSeeds.p, S.dScales.p, ctx->dAdjF.p,
+                              reinterpret_cast<unsigned long long *>(ctx->dAdjB.p), ctx->dGrad.p, ctx->dLogT.p,
+                              tables ? ctx->dPost.p : nullptr, ctx->dAdjStatus.p, ctx->dAdjStatus.p + nj};
+                cudaLaunchAttribute at;
+                const cudaLaunchConfig_t cfg = clusterLaunch(pC, pW, pW * sizeof(AdjWin), pC * std::min(pClusters, nj),
+                                                             &at, ctx->stream);
+                CK(cudaLaunchKernelEx(&cfg, pipeKern, a), "adjoint kernel");
+            } else {
+                const int blocks = (nj + kAdjWarps - 1) / kAdjWarps;
+                auto kern = ckpt ? (tables ? adjointKernel<true, true> : adjointKernel<false, true>)
+                                 : (tables ? adjointKernel<true> : adjointKernel<false>);
+                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjSmem), "smem attribute");
+                kern<<<blocks, kAdjWarps * 32, kAdjSmem, ctx->stream>>>(
+                    ctx->dAdjJobs.p, nj, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p, ctx->dCodes.p,
+                    S.dSeeds.p, S.dScales.p, ctx->dAdjF.p, ctx->dAdjB.p, ctx->dGrad.p, ctx->dLogT.p,
+                    tables ? ctx->dPost.p : nullptr);
+            }
+            CK(cudaGetLastError(), "adjoint kernel");
+            ++launches;
+            if (summary) {
+                int maxL = 0;
+                for (size_t k = k0; k < k1; ++k) {
+                    const int ci = order[which[k]];
+                    const int L = ctx->seqLen[pairs[ci].seq];
+                    sumJobs[k] = PostSumJob{jobs[k].pOff, colOff[ci], (long long)ci * (M + 1), M, L};
+                    maxL = std::max(maxL, L);
+                }
+                CK(cudaMemcpyAsync(ctx->dPostJobs.p, sumJobs.data() + k0, nj * sizeof(PostSumJob),
+                                   cudaMemcpyHostToDevice, ctx->stream),
+                   "upload summary jobs");
+                if (colPost || colRow) {
+                    postColumnKernel<<<dim3((maxL + kPostThreads - 1) / kPostThreads, nj), kPostThreads, 0, ctx->stream>>>(
+                        ctx->dPostJobs.p, ctx->dPost.p, ctx->dColPost.p, ctx->dColRow.p);
+                    CK(cudaGetLastError(), "posterior column kernel");
+                    ++launches;
+                }
+                if (rowMatch) {
+                    const int rowsPer = kPostThreads / kLanes;
+                    postRowKernel<<<dim3((M + 1 + rowsPer - 1) / rowsPer, nj), kPostThreads, 0, ctx->stream>>>(
+                        ctx->dPostJobs.p, ctx->dPost.p, ctx->dRowMatch.p);
+                    CK(cudaGetLastError(), "posterior row kernel");
+                    ++launches;
+                }
+            }
+            CK(cudaEventRecord(ctx->ev[4], ctx->stream), "event");
+            if (post)
+                for (size_t k = k0; k < k1; ++k)
+                    CK(cudaMemcpyAsync(post + postOff[order[which[k]]], ctx->dPost.p + jobs[k].pOff,
+                                       (size_t)needP[k] * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
+                       "download posterior tables");
+            std::vector<double> blt(nj);
+            CK(cudaMemcpyAsync(blt.data(), ctx->dLogT.p, nj * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
+               "download log T");
+            int aborted = 0;
+            if (pipe) {
+                CK(cudaMemcpyAsync(status.data() + k0, ctx->dAdjStatus.p, nj * sizeof(int), cudaMemcpyDeviceToHost,
+                                   ctx->stream),
+                   "download adjoint status");
+                CK(cudaMemcpyAsync(&aborted, ctx->dAdjStatus.p + nj, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
+                   "download adjoint status");
+            }
+            CK(cudaStreamSynchronize(ctx->stream), "adjoint kernel");
+            for (int q = 0; q < nj; ++q) lt[which[k0 + q]] = blt[q];
+            if (aborted) status[m] = kAdjRedo;
+            adjMs += elapsedMs(ctx, ctx->ev[3], ctx->ev[4]);
+            k0 = k1;
+        }
+        return DMST_OK;
+    };
+    CK(cudaMemsetAsync(ctx->dGrad.p, 0, gN * sizeof(double), ctx->stream), "zero gradient");
+    std::vector<int> all(n), beyond, status;
+    std::iota(all.begin(), all.end(), 0);
+    if ((st = runBatches(all, true, status))) return st;
+    bool redo = false;
+    for (size_t k = 0; k <= n; ++k) {
+        redo |= status[k] == kAdjRedo;
+        if (k < n && status[k] == kAdjRange) beyond.push_back((int)k);
+    }
+    if (redo) {  // part of a gradient is in the sums: every pair again
+        CK(cudaMemsetAsync(ctx->dGrad.p, 0, gN * sizeof(double), ctx->stream), "zero gradient");
+        beyond = all;
+    }
+    // pairs whose values need the stripe offsets
+    if (!beyond.empty() && (st = runBatches(beyond, false, status))) return st;
     // Timing of the call: [1] null model, [2] adjoint kernels, [0] both.
     ctx->lastNullMs = nullMs;
     ctx->lastDpMs = adjMs;
@@ -3275,9 +3356,8 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
     ctx->lastTotalMs = nullMs + adjMs;
     ctx->lastLaunches = launches;
     ctx->lastWallMs = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - wallT0).count();
-    std::vector<double> g(gN), lt(n);
+    std::vector<double> g(gN);
     CK(cudaMemcpy(g.data(), ctx->dGrad.p, gN * sizeof(double), cudaMemcpyDeviceToHost), "download gradient");
-    CK(cudaMemcpy(lt.data(), ctx->dLogT.p, n * sizeof(double), cudaMemcpyDeviceToHost), "download log T");
     if (log_t)
         for (size_t k = 0; k < n; ++k) log_t[order[k]] = lt[k];
     if (grad_params) std::memcpy(grad_params, g.data(), (size_t)(M + 2) * kParamFloats * sizeof(double));
