@@ -9,7 +9,7 @@
 #include "dp_posterior.cuh"
 #include "dp_pipe.cuh"
 #include "dp_plain.cuh"
-#include "dp_exact_wave.cuh"
+#include "dp_exact_pipe.cuh"
 #include "dp_search.cuh"
 #include "dp_stagger.cuh"
 #include "dp_traceback.cuh"
@@ -559,7 +559,7 @@ struct CallSlot {
     DevBuf<PairOut> dOut;
     DevBuf<ExactOut> dExOut;  // exact-path results, by pair position
     DevBuf<int> dQueue;       // exact-path queue, by queue position
-    DevBuf<int> dQueueCount;  // [0] queued pairs, [1] next queue position
+    DevBuf<int> dQueueCount;  // queued pairs
     DevBuf<PairOut> dOutF;    // search: the filter wave's results
     DevBuf<uint8_t> dMask;    // search: survivors
     PinnedBuf<PairOut> hOutF;
@@ -619,6 +619,7 @@ struct dmst_ctx {
     cudaEvent_t evSeqStage[2] = {};  // ... each block's copy done
     int seqStageNext = 0;
     cudaEvent_t ev[6] = {};
+    cudaEvent_t evExact = nullptr;  // the last exact-path kernel done
     std::string err;
 
     std::vector<HostProfile> profiles;
@@ -678,7 +679,10 @@ struct dmst_ctx {
     int nextSlot = 0;                        // the slot the next submit uses
     int oldest = 0;                          // the oldest pending call's slot
     int lastSlot = 0;                        // the slot of the last completed call
-    DevBuf<float> dExactPool;                // exact-path scratch: one slot per CTA
+    DevBuf<float> dExactPool;                // exact-path scratch: one slot per cluster
+    DevBuf<unsigned long long> dExactRing;   // exact path: boundary rows, kRingEmpty between kernels
+    DevBuf<int> dExactAbort;                 // ... an abort flag per cluster
+    bool exactClean = false;                 // the rings and the flags are as a kernel expects them
     DevBuf<Chunk> dMidChunks;                // search: the survivors' chunks
     DevBuf<int> dSurvivors;                  // search: survivor pair indices by chunk
     DevBuf<float> dMinBest;                  // search: per-profile filter gate
@@ -700,7 +704,7 @@ struct dmst_ctx {
     double lastPostMs = 0, lastWallMs = 0;
     int lastExactPairs = 0;
     int lastLaunches = 0;
-    int lastFlagged = 0;  // pairs the last completed mid-score call sent to the exact path
+    int lastFlagged = -1;  // pairs the last completed mid-score call sent to the exact path (-1: none yet)
     int waitLimit = 0;    // exact path: iterations of a stripe wait before it gives up (0: the default)
 
     int fail(int status, const char *fmt, ...) {
@@ -788,6 +792,7 @@ int dmst_ctx_create(const dmst_opts *opts, dmst_ctx **out) {
         return DMST_EDEVICE;
     }
     for (auto &e : ctx->ev) cudaEventCreate(&e);
+    cudaEventCreateWithFlags(&ctx->evExact, cudaEventDisableTiming);
     for (auto &e : ctx->evSeqStage) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     for (auto &sl : ctx->slot) {
         for (auto &e : sl.ev) cudaEventCreate(&e);
@@ -845,6 +850,8 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
         if (sl.evFork) cudaEventDestroy(sl.evFork);
     }
     ctx->dExactPool.release();
+    ctx->dExactRing.release();
+    ctx->dExactAbort.release();
     for (auto &hb : ctx->hSeqStage) hb.release();
     for (auto &e : ctx->evSeqStage)
         if (e) cudaEventDestroy(e);
@@ -905,6 +912,7 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
         if (e) cudaEventDestroy(e);
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
+    if (ctx->evExact) cudaEventDestroy(ctx->evExact);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->stream2) cudaStreamDestroy(ctx->stream2);
     delete ctx;
@@ -2030,59 +2038,57 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         return st;
 
     // The exact path on the device: flagged pairs go to a queue that
-    // persistent CTAs of the exact kernel drain, each CTA (or, when no pair of
-    // the call has more than kPipeWarps / 2 stripes and more pairs than SMs are
-    // expected, each half of a CTA) with a scratch slot sized for the largest
-    // pair of the call.
+    // persistent clusters of the exact kernel drain, each with scratch and
+    // rings sized for the largest pair of the call.  How many pairs to expect:
+    // all of a forced call, else the last call's count (none yet: one in 64).
     const bool exactOnDevice = mid && !nullOnly && !sequentialExact;
-    long long poolSlot = 0;
-    int exactGrid = 0, exactGroups = 1;
+    long long poolSlot = 0, exactRing = 0;
+    int exactW = 1, exactC = 1, exactClusters = 0;
     if (exactOnDevice) {
-        int maxWarps = 1;
-        for (size_t k = 0; k < n; ++k) maxWarps = std::max(maxWarps, exactWarps(dp[k].M));
-        // two groups pay only with more exact-path pairs than SMs (the
-        // grouped kernel holds more per thread; with fewer pairs, one pair per
-        // SM is faster): a forced call sends every pair, otherwise the last
-        // call's count stands in
-        const long long exactPairsExpected = forceExact ? (long long)n : (long long)ctx->lastFlagged;
-        exactGroups = maxWarps <= kPipeWarps / 2 && exactPairsExpected > ctx->smCount ? 2 : 1;
-        for (size_t k = 0; k < n; ++k)
-            poolSlot = std::max(poolSlot, exactWaveScratch(dp[k].M, dp[k].L,
-                                                           std::min(exactWarps(dp[k].M), kPipeWarps / exactGroups),
-                                                           anchors));
-        poolSlot = (poolSlot + 63) / 64 * 64;
-        size_t freeB = 0, totalB = 0;
-        CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
-        const size_t poolBudget = std::max<size_t>((freeB + ctx->dExactPool.cap * sizeof(float)) / 4, (size_t)256 << 20);
-        exactGrid = (int)std::max<size_t>(
-            1, std::min<size_t>((size_t)ctx->smCount,
-                                poolBudget / ((size_t)poolSlot * exactGroups * sizeof(float))));
-        CK(ctx->dExactPool.ensure((size_t)exactGrid * exactGroups * poolSlot), "alloc exact scratch");
-        CK(S.dExOut.ensure(n), "alloc exact out");
-        CK(S.dQueue.ensure(n), "alloc exact queue");
-        CK(S.dQueueCount.ensure(2), "alloc exact queue");
-        CK(S.hExOut.ensure(n), "alloc exact out");
+        int maxM = 0;
+        for (size_t k = 0; k < n; ++k) {
+            maxM = std::max(maxM, dp[k].M);
+            poolSlot = std::max(poolSlot, exactPipeScratch(dp[k].M, dp[k].L, anchors));
+            exactRing = std::max(exactRing, exactRingWords(dp[k].M, dp[k].L));
+        }
+        const size_t expected =
+            forceExact ? n : std::min<size_t>(n, std::max<size_t>(1, ctx->lastFlagged < 0 ? n / 64 : (size_t)ctx->lastFlagged));
+        pipeSpread(ctx, expected, exactStripes(maxM), kExactMaxWarps, kExactMaxWarps, 1, exactW, exactC);
         if (!ctx->exactAttrSet) {
-            CK(cudaFuncSetAttribute(exactWaveKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kPipeWarps * sizeof(Window))),
-               "smem attribute");
-            CK(cudaFuncSetAttribute(exactWaveKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kPipeWarps * sizeof(Window))),
-               "smem attribute");
-            CK(cudaFuncSetAttribute(exactWaveKernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kPipeWarps * sizeof(Window))),
-               "smem attribute");
-            CK(cudaFuncSetAttribute(exactWaveKernel<false, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kPipeWarps * sizeof(Window))),
-               "smem attribute");
-            CK(cudaFuncSetAttribute(exactWaveKernel<true, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kPipeWarps * sizeof(Window))),
-               "smem attribute");
-            CK(cudaFuncSetAttribute(exactWaveKernel<true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kPipeWarps * sizeof(Window))),
-               "smem attribute");
+            for (auto k : {exactPipeKernel<false>, exactPipeKernel<true>, exactPipeKernel<true, true>})
+                CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)(kExactMaxWarps * sizeof(WindowX))),
+                   "smem attribute");
             ctx->exactAttrSet = true;
         }
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = clusterLaunch(exactC, exactW, exactW * sizeof(WindowX), exactC * ctx->smCount, &at, nullptr);
+        CK(cudaOccupancyMaxActiveClusters(&exactClusters, exactPipeKernel<true, true>, &cfg), "cluster occupancy");
+        exactClusters = (int)std::min<size_t>(std::max(1, exactClusters), n);
+        const size_t slotBytes = (size_t)poolSlot * sizeof(float) + (size_t)exactRing * sizeof(unsigned long long);
+        const size_t held = ctx->dExactPool.cap * sizeof(float) + ctx->dExactRing.cap * sizeof(unsigned long long);
+        if (exactClusters * slotBytes > held) {
+            size_t freeB = 0, totalB = 0;
+            CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
+            const size_t poolBudget = std::max<size_t>((freeB + held) / 4, (size_t)256 << 20);
+            exactClusters = (int)std::max<size_t>(1, std::min<size_t>(exactClusters, poolBudget / slotBytes));
+        }
+        CK(ctx->dExactPool.ensure((size_t)exactClusters * poolSlot), "alloc exact scratch");
+        if ((size_t)(exactClusters * exactRing) > ctx->dExactRing.cap || (size_t)exactClusters > ctx->dExactAbort.cap)
+            ctx->exactClean = false;
+        CK(ctx->dExactRing.ensure((size_t)exactClusters * exactRing), "alloc exact rings");
+        CK(ctx->dExactAbort.ensure(exactClusters), "alloc exact rings");
+        if (!ctx->exactClean) {
+            CK(cudaStreamWaitEvent(ctx->stream, ctx->evExact, 0), "stream dependency");
+            CK(cudaMemsetAsync(ctx->dExactRing.p, 0xff, ctx->dExactRing.cap * sizeof(unsigned long long), ctx->stream),
+               "empty exact rings");
+            CK(cudaMemsetAsync(ctx->dExactAbort.p, 0, ctx->dExactAbort.cap * sizeof(int), ctx->stream), "zero abort flags");
+            ctx->exactClean = true;
+        }
+        CK(S.dExOut.ensure(n), "alloc exact out");
+        CK(S.dQueue.ensure(n), "alloc exact queue");
+        CK(S.dQueueCount.ensure(1), "alloc exact queue");
+        CK(S.hExOut.ensure(n), "alloc exact out");
     }
     CK(S.hOut.ensure(n), "alloc results");
     long long anchorCols = 0;
@@ -2177,7 +2183,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     auto enqueue = [&]() -> int {
         launches = 0;
         CK(cudaMemsetAsync(ctx->dCounter.p, 0, nCounters * sizeof(int), ctx->stream), "zero counters");
-        if (exactOnDevice) CK(cudaMemsetAsync(S.dQueueCount.p, 0, 2 * sizeof(int), ctx->stream), "zero queue");
+        if (exactOnDevice) CK(cudaMemsetAsync(S.dQueueCount.p, 0, sizeof(int), ctx->stream), "zero queue");
         CK(record(S.ev[0]), "event");
         nullModelKernel<<<nullBlocks, kNullWarps * 32, 0, ctx->stream>>>(
             ctx->dNullJobs.p, nj, ctx->dNullJobPairs.p, S.dPairs.p, ctx->dProfiles.p, ctx->dCodes.p,
@@ -2276,8 +2282,6 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                                       (uintptr_t)ctx->dW1.p, (uintptr_t)ctx->dRing.p, (uintptr_t)S.dOut.p,
                                       (uintptr_t)ctx->dChunks.p, (uintptr_t)w1Slot, (uintptr_t)ringSlot,
                                       (uintptr_t)n, (uintptr_t)exactOnDevice, (uintptr_t)forceExact,
-                                      (uintptr_t)exactGrid, (uintptr_t)poolSlot, (uintptr_t)ctx->dExactPool.p,
-                                      (uintptr_t)exactGroups,
                                       (uintptr_t)S.dExOut.p, (uintptr_t)S.dQueue.p, (uintptr_t)S.dQueueCount.p,
                                       (uintptr_t)S.hOut.p, (uintptr_t)S.hExOut.p};
         for (uintptr_t v : {(uintptr_t)pipe.kern, (uintptr_t)pipe.clusters, (uintptr_t)pipe.C, (uintptr_t)pipe.W,
@@ -2326,8 +2330,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     }
     // The exact path and the result copies go on the second stream, after the
     // flag kernel, when the exact path is expected to leave SMs idle (the
-    // previous call flagged fewer pairs than three quarters of the SMs, each
-    // pair taking one CTA): the next call's null model and DP kernels (first
+    // previous call flagged fewer pairs than three quarters of the SMs): the next call's null model and DP kernels (first
     // stream) then fill them.  A larger exact path keeps the stream order.
     const bool overlapExact = exactOnDevice && !align && ctx->lastFlagged * 4 < ctx->smCount * 3;
     cudaStream_t tail = overlapExact ? ctx->stream2 : ctx->stream;
@@ -2336,16 +2339,19 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
             CK(cudaEventRecord(S.evFork, ctx->stream), "event");
             CK(cudaStreamWaitEvent(ctx->stream2, S.evFork, 0), "stream dependency");
         }
-        auto ek = exactGroups == 2
-                      ? (align ? exactWaveKernel<true, true, 2>
-                               : (anchors ? exactWaveKernel<true, false, 2> : exactWaveKernel<false, false, 2>))
-                      : (align ? exactWaveKernel<true, true> : (anchors ? exactWaveKernel<true> : exactWaveKernel<false>));
-        ek<<<exactGrid, kPipeWarps * kLanes, kPipeWarps * sizeof(Window), tail>>>(
-            S.dQueue.p, S.dQueueCount.p, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p,
-            ctx->dCodes.p, S.dSeeds.p, S.dScales.p, ctx->dExactPool.p, poolSlot, S.dExOut.p,
-            anchors ? S.dAnchorOff.p : nullptr, S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p,
-            align ? ctx->dAlignJobOf.p : nullptr, align ? ctx->dAlignJobs.p : nullptr,
-            align ? ctx->dAlignCells.p : nullptr, align ? ctx->dAlignRows.p : nullptr, ctx->waitLimit);
+        // the scratch and the rings are the previous call's until its kernel ends, on whichever stream
+        CK(cudaStreamWaitEvent(tail, ctx->evExact, 0), "stream dependency");
+        auto ek = align ? exactPipeKernel<true, true> : (anchors ? exactPipeKernel<true> : exactPipeKernel<false>);
+        const ExactPipeArgs ea{S.dQueue.p, S.dQueueCount.p, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p,
+                               ctx->dCodes.p, S.dSeeds.p, S.dScales.p, ctx->dExactPool.p, poolSlot, ctx->dExactRing.p,
+                               exactRing, ctx->dExactAbort.p, S.dExOut.p, anchors ? S.dAnchorOff.p : nullptr,
+                               S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p, align ? ctx->dAlignJobOf.p : nullptr,
+                               align ? ctx->dAlignJobs.p : nullptr, align ? ctx->dAlignCells.p : nullptr,
+                               align ? ctx->dAlignRows.p : nullptr, ctx->waitLimit > 0 ? ctx->waitLimit : kRingSpin};
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = clusterLaunch(exactC, exactW, exactW * sizeof(WindowX), exactC * exactClusters, &at, tail);
+        CK(cudaLaunchKernelEx(&cfg, ek, ea), "exact kernel");
+        CK(cudaEventRecord(ctx->evExact, tail), "event");
         CK(cudaGetLastError(), "exact kernel");
         ++launches;
     }
@@ -2491,9 +2497,11 @@ static int completeCall(dmst_ctx *ctx) {
         exactMs = elapsedMs(ctx, ctx->ev[3], ctx->ev[4]);
     }
     for (size_t f = 0; f < eo.size(); ++f)
-        if (eo[f].failed)
+        if (eo[f].failed) {
+            ctx->exactClean = false;  // its rings are not empty
             return ctx->fail(DMST_ETIMEOUT, "exact path: the stripe pipeline of pair %d gave up a wait",
                              order[flagged[f]]);
+        }
     ctx->lastExactMs = exactMs;
     ctx->lastExactPairs = (int)flagged.size();
     if (mid) ctx->lastFlagged = (int)flagged.size();

@@ -1,5 +1,5 @@
 // The row-contiguous stripe wavefront: the step functions of the exact
-// row-rescaled path (dp_exact_wave.cuh, dp_exact.cuh) and of the plain
+// row-rescaled path (dp_exact_pipe.cuh, dp_exact.cuh) and of the plain
 // one-pair-per-launch schedule (dp_plain.cuh).  The batched kernel of the
 // fast path is dp_stagger.cuh.
 //
@@ -37,7 +37,7 @@
 // never exceed RESCALE_THRESH.  They report the largest backward Y (Y >= W1
 // at every cell) and the largest forward W0/Y0, so the host can tell whether
 // the reference would have rescaled; such pairs are re-scored by the exact
-// row-rescaled path (dp_exact_wave.cuh), whose modes apply the reference's
+// row-rescaled path (dp_exact_pipe.cuh), whose modes apply the reference's
 // rescale counts.
 //
 // Mid score.  The reference forms promote(W0)*promote(W1) in double and
@@ -270,11 +270,16 @@ struct Window {
 __device__ __forceinline__ float4 ringLoad(const float *ring, int col) {
     return __ldcg(reinterpret_cast<const float4 *>(ring) + col);
 }
-__device__ __forceinline__ void ringStore(float *ring, int col, float w, float y, int cnt) {
-    __stcg(reinterpret_cast<float4 *>(ring) + col, make_float4(w, y, __int_as_float(cnt), 0.0f));
-}
+// Each half in one 64-bit store: the exact path's readers (dp_exact_pipe.cuh)
+// see a half whole or not at all.
 __device__ __forceinline__ void ringStore(float *ring, int col, float w, float y) {
-    __stcg(reinterpret_cast<float2 *>(ring) + 2 * col, make_float2(w, y));
+    const unsigned long long v = ((unsigned long long)__float_as_uint(y) << 32) | __float_as_uint(w);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(ring + 4 * (size_t)col), "l"(v) : "memory");
+}
+__device__ __forceinline__ void ringStore(float *ring, int col, float w, float y, int cnt) {
+    ringStore(ring, col, w, y);
+    const unsigned long long v = (unsigned)cnt;
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(ring + 4 * (size_t)col + 2), "l"(v) : "memory");
 }
 
 // max(a, b, c) in one instruction (the three-input max.f32 of sm_100).
@@ -434,9 +439,43 @@ struct BwdState {
     double rowBest[R];       // replay: per-row max of W1 * prefixSeed
 };
 
+// A lane takes up its rows of profile stripe s: coefficients, empty histories.
+template <int R, int MODE>
+__device__ __forceinline__ void backwardStart(BwdState<R, MODE> &b, const SweepArgs &a, int lane, int s,
+                                              const ExactRows *x) {
+    const int rowBase = s * kLanes * R + lane * R, lag = kLanes - 1 - lane;
+    loadBackwardCoef<R>(b.c, a, rowBase);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) b.h[q][k] = b.z[q][k] = 0.0f;
+        b.rb[q] = 0.0f;
+    }
+    b.wp = a.w1 + (((size_t)s * a.D + lag) * kLanes + lane) * R;
+    if (MODE == kDiscover) {
+        b.cnt = 0;
+#pragma unroll
+        for (int k = 0; k < R; ++k) b.rmax[k] = 0.0f;
+    }
+    if (MODE == kReplay) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int i = rowBase + k;
+            const int ci = i <= a.M() ? i : a.M() + 1;
+            const int cIn = __ldcg(x->cntB + (ci + 1 <= a.M() + 1 ? ci + 1 : a.M() + 1));
+            b.cOut[k] = __ldcg(x->cntB + ci);
+            b.fOut[k] = stepsDown(b.cOut[k] - cIn);
+            b.c.rs[k] = seedCoef(i <= a.M(), cIn);
+            b.rowBest[k] = 0.0;
+        }
+    }
+}
+
 // PIPE: the sweep runs one of several warps' stripes of a pair (a stripe
 // pipeline: stripes sFirst, sFirst + sStep, ...; ring slot per stripe).
-template <int R, int MODE, int PH, bool PIPE = (MODE == kDiscover || MODE == kReplay), bool SH = false>
+// START: the lane takes up a stripe at its first column (false: the caller has
+// done so for the sweep's only stripe).
+template <int R, int MODE, int PH, bool PIPE = (MODE == kDiscover || MODE == kReplay), bool SH = false, bool START = true>
 __device__ __forceinline__ void backwardStep(BwdState<R, MODE> &b, const SweepArgs &a, Window &win, int lane,
                                              int total, const ExactRows *x, ExactBest *exact) {
     constexpr int S = kLanes * R;
@@ -447,37 +486,10 @@ __device__ __forceinline__ void backwardStep(BwdState<R, MODE> &b, const SweepAr
     float inY = __shfl_down_sync(kFull, b.sendY, 1);
     int inC = 0;
     if (MODE == kDiscover) inC = __shfl_down_sync(kFull, b.sendC, 1);
-    const int lag = kLanes - 1 - lane;
     if (b.u >= 0 && b.u < total && b.jj < a.L) {
         const int s = a.nS - 1 - b.sp;
         const int rowBase = s * S + lane * R;
-        if (b.jj == 0) {
-            loadBackwardCoef<R>(b.c, a, rowBase);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-#pragma unroll
-                for (int k = 0; k < R; ++k) b.h[q][k] = b.z[q][k] = 0.0f;
-                b.rb[q] = 0.0f;
-            }
-            b.wp = a.w1 + (((size_t)s * a.D + lag) * kLanes + lane) * R;
-            if (MODE == kDiscover) {
-                b.cnt = 0;
-#pragma unroll
-                for (int k = 0; k < R; ++k) b.rmax[k] = 0.0f;
-            }
-            if (MODE == kReplay) {
-#pragma unroll
-                for (int k = 0; k < R; ++k) {
-                    const int i = rowBase + k;
-                    const int ci = i <= a.M() ? i : a.M() + 1;
-                    const int cIn = x->cntB[ci + 1 <= a.M() + 1 ? ci + 1 : a.M() + 1];
-                    b.cOut[k] = x->cntB[ci];
-                    b.fOut[k] = stepsDown(b.cOut[k] - cIn);
-                    b.c.rs[k] = seedCoef(i <= a.M(), cIn);
-                    b.rowBest[k] = 0.0;
-                }
-            }
-        }
+        if (START && b.jj == 0) backwardStart<R, MODE>(b, a, lane, s, x);
         const int slot = b.u & (kWin - 1);
         const float4 col = win.col[slot];
         if (lane == kLanes - 1) {
@@ -703,6 +715,34 @@ struct FwdState {
     double rowBest[R];
 };
 
+template <int R, int MODE>
+__device__ __forceinline__ void forwardStart(FwdState<R, MODE> &f, const SweepArgs &a, int lane, int s,
+                                             const ExactRows *x) {
+    const int rowBase = s * kLanes * R + lane * R;
+    loadForwardCoef<R>(f.c, a, rowBase);
+#pragma unroll
+    for (int h = 0; h < 3; ++h)
+#pragma unroll
+        for (int k = 0; k < R; ++k) f.w[h][k] = f.z[h][k] = 0.0f;
+    if (MODE == kDiscover) {
+        f.cnt = 0;
+#pragma unroll
+        for (int k = 0; k < R; ++k) f.rmax[k] = 0.0f;
+    }
+    if (MODE == kReplay) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int i = rowBase + k;
+            const int ci = i <= a.M() ? i : a.M();
+            f.cIn[k] = __ldcg(x->cntF + ci);
+            f.fOut[k] = stepsDown(__ldcg(x->cntF + ci + 1) - f.cIn[k]);
+            f.cB[k] = __ldcg(x->cntB + ci);
+            f.c.rs[k] = seedCoef(i <= a.M(), f.cIn[k]);
+            f.rowBest[k] = 0.0;
+        }
+    }
+}
+
 // One forward step of a lane (dummest-dp-forward.hh:112-223) at phase PH;
 // q holds the W1 values of this step.  Slot (3-PH)%3 holds column j-1,
 // (4-PH)%3 column j-2, (5-PH)%3 column j-3, which the new column j replaces.
@@ -713,7 +753,7 @@ struct FwdState {
 // lane writes the stripe's partial, and the stripes are folded in order after
 // the sweep.
 template <int R, int MODE, int PH, bool ANCH = false, bool PIPE = (MODE == kDiscover || MODE == kReplay),
-          bool SH = false>
+          bool SH = false, bool START = true>
 __device__ __forceinline__ void forwardStep(FwdState<R, MODE> &f, const SweepArgs &a, Window &win, int lane,
                                             int total, const float (&q)[R], const ExactRows *x, ExactBest *exact) {
     constexpr int S = kLanes * R;
@@ -736,30 +776,7 @@ __device__ __forceinline__ void forwardStep(FwdState<R, MODE> &f, const SweepArg
     if (MODE == kDiscover) inC = __shfl_up_sync(kFull, f.sendC, 1);
     if (f.u >= 0 && f.u < total && f.j < a.L) {
         const int rowBase = f.s * S + lane * R;
-        if (f.j == 0) {
-            loadForwardCoef<R>(f.c, a, rowBase);
-#pragma unroll
-            for (int h = 0; h < 3; ++h)
-#pragma unroll
-                for (int k = 0; k < R; ++k) f.w[h][k] = f.z[h][k] = 0.0f;
-            if (MODE == kDiscover) {
-                f.cnt = 0;
-#pragma unroll
-                for (int k = 0; k < R; ++k) f.rmax[k] = 0.0f;
-            }
-            if (MODE == kReplay) {
-#pragma unroll
-                for (int k = 0; k < R; ++k) {
-                    const int i = rowBase + k;
-                    const int ci = i <= a.M() ? i : a.M();
-                    f.cIn[k] = x->cntF[ci];
-                    f.fOut[k] = stepsDown(x->cntF[ci + 1] - f.cIn[k]);
-                    f.cB[k] = x->cntB[ci];
-                    f.c.rs[k] = seedCoef(i <= a.M(), f.cIn[k]);
-                    f.rowBest[k] = 0.0;
-                }
-            }
-        }
+        if (START && f.j == 0) forwardStart<R, MODE>(f, a, lane, f.s, x);
         const int slot = f.u & (kWin - 1);
         const float4 col = win.col[slot];
         if (lane == 0) {
@@ -927,7 +944,7 @@ __device__ __forceinline__ void forwardStep(FwdState<R, MODE> &f, const SweepArg
 // W1 copy, read it from the staging ring, run the step, and stage the W1 of
 // the step kW1Ahead later into the slot this lane read one step ago.
 template <int R, int MODE, int P6, bool ANCH = false, bool PIPE = (MODE == kDiscover || MODE == kReplay),
-          bool SH = false>
+          bool SH = false, bool START = true>
 __device__ __forceinline__ void forwardStaged(FwdState<R, MODE> &f, const SweepArgs &a, Window &win, int lane,
                                               int total, W1Stage<R, PIPE> &st,
                                               const ExactRows *x, ExactBest *exact) {
@@ -946,7 +963,7 @@ __device__ __forceinline__ void forwardStaged(FwdState<R, MODE> &f, const SweepA
 #pragma unroll
         for (int k = 0; k < R; ++k) q[k] = 0.0f;
     }
-    forwardStep<R, MODE, P6 % 3, ANCH, PIPE, SH>(f, a, win, lane, total, q, x, exact);
+    forwardStep<R, MODE, P6 % 3, ANCH, PIPE, SH, START>(f, a, win, lane, total, q, x, exact);
     if (kReadW1) st.issue(a, win, (P6 + kW1Ahead) % kW1Slots, lane, total);
 }
 
