@@ -429,8 +429,9 @@ inline size_t pipeWindowBytes(int R) {
     return R == 4 ? sizeof(WindowP<4>) : (R == 2 ? sizeof(WindowP<2>) : sizeof(WindowP<1>));
 }
 struct PipePlan {
+    bool whole = false;  // the whole call runs on the pipeline (otherwise, a search's survivors)
     int R = 1, W = 1, C = 1, clusters = 0;
-    PipeKern kern = nullptr;
+    PipeKern kern = nullptr, kernF = nullptr;  // kernF: the filter wave of a search
     size_t smem = 0;
     long long w1Slot = 0, ringSlot = 0;  // floats, entries
 };
@@ -685,6 +686,7 @@ struct dmst_ctx {
     bool exactClean = false;                 // the rings and the flags are as a kernel expects them
     DevBuf<Chunk> dMidChunks;                // search: the survivors' chunks
     DevBuf<int> dSurvivors;                  // search: survivor pair indices by chunk
+    DevBuf<int> dSurvivorList, dSurvivorCount;  // ... all of them; their number, and how many run from the list
     DevBuf<float> dMinBest;                  // search: per-profile filter gate
     DevBuf<float> dExactScratch;
     DevBuf<ExactOut> dExactOut;
@@ -872,6 +874,8 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
     ctx->dAlignSegOut.release();
     ctx->dMidChunks.release();
     ctx->dSurvivors.release();
+    ctx->dSurvivorList.release();
+    ctx->dSurvivorCount.release();
     ctx->dMinBest.release();
     ctx->dEmit.release();
     ctx->dParams.release();
@@ -1603,18 +1607,20 @@ static void pipeSpread(const dmst_ctx *ctx, size_t n, int stripes, int maxW, int
 }
 
 // The stripe pipeline's shape for n pairs whose rows average `rows` (weighted
-// by cells).
+// by cells), at least `least` warps a pair.
 //
 // Two rows per lane (one when a single 32-row stripe holds the profile) were
 // the fastest or within 5% of it over M = 20-2000, L = 200-10000 and 2-1200
 // pairs: one row doubles the boundary values and steps, four rows double the
 // time of a step and the fill.  Twelve warps per SM.
-static int pipeShape(dmst_ctx *ctx, size_t n, double rows, PipePlan &plan) {
+static int pipeShape(dmst_ctx *ctx, size_t n, double rows, int least, PipePlan &plan) {
     const int stripes = std::max(1, (int)std::ceil(rows / (kLanes * plan.R)));
     const int maxW = (int)std::min<size_t>(pipeMaxWarps(plan.R), ((size_t)ctx->maxSmemOptin - 1024) / pipeWindowBytes(plan.R));
-    pipeSpread(ctx, n, stripes, maxW, 12, 1, plan.W, plan.C);
+    pipeSpread(ctx, n, stripes, maxW, 12, least, plan.W, plan.C);
     plan.smem = (size_t)plan.W * pipeWindowBytes(plan.R);
     CK(cudaFuncSetAttribute(plan.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem), "smem attribute");
+    if (plan.kernF)
+        CK(cudaFuncSetAttribute(plan.kernF, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem), "smem attribute");
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = clusterLaunch(plan.C, plan.W, plan.smem, plan.C * ctx->smCount, &at, nullptr);
     int resident = 0;
@@ -1630,9 +1636,14 @@ static int pipeShape(dmst_ctx *ctx, size_t n, double rows, PipePlan &plan) {
 // ms, (300, 3100, 200) 1.88 / 0.91, (300, 3100, 600) 2.60 / 2.05, (800, 3000,
 // 400) 4.34 / 3.04; beyond the line (300, 3100, 1500) 3.84 / 4.42, (800, 3000,
 // 1200) 8.42 / 8.72, (100, 1000, 3000) 1.08 / 1.30.
-static int pipePlan(dmst_ctx *ctx, const std::vector<DevPair> &dp, bool mid, PipePlan &plan) {
-    const size_t n = dp.size();
-    if (n > 6 * (size_t)ctx->smCount) return DMST_OK;
+//
+// A search of more pairs has a plan for the survivors of its filter wave
+// (dp_search.cuh), of which 12 per SM are expected.
+static int pipePlan(dmst_ctx *ctx, const std::vector<DevPair> &dp, bool mid, bool search, PipePlan &plan) {
+    size_t n = dp.size();
+    plan.whole = n <= 6 * (size_t)ctx->smCount;
+    if (!plan.whole && !search) return DMST_OK;
+    if (!plan.whole) n = std::min<size_t>(n, 12 * (size_t)ctx->smCount);
     double cells = 0, weighted = 0;
     int maxM = 0;
     for (const DevPair &d : dp) {
@@ -1643,12 +1654,13 @@ static int pipePlan(dmst_ctx *ctx, const std::vector<DevPair> &dp, bool mid, Pip
     }
     plan.R = maxM < kLanes ? 1 : 2;
     plan.kern = pipeKernelFor(plan.R, mid);
+    if (search && plan.whole) plan.kernF = pipeKernelFor(plan.R, false);
     for (const DevPair &d : dp) {
         if (mid) plan.w1Slot = std::max(plan.w1Slot, pipeW1Floats(d.M, d.L, plan.R));
         plan.ringSlot = std::max(plan.ringSlot, pipeRingEntries(d.M, d.L, plan.R));
     }
     plan.w1Slot = (plan.w1Slot + 63) / 64 * 64;
-    if (const int st = pipeShape(ctx, n, weighted / cells, plan)) return st;
+    if (const int st = pipeShape(ctx, n, weighted / cells, plan.whole ? 1 : 4, plan)) return st;
     // the slots within the device budget
     const size_t slotBytes = (size_t)plan.w1Slot * sizeof(float) + (size_t)plan.ringSlot * sizeof(unsigned long long);
     size_t budget = ctx->opts.device_budget_bytes;
@@ -1797,9 +1809,10 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         ringMax = std::max(ringMax, 2 * (size_t)stagPeriod(d.L, d.R));
     }
     PipePlan pipe;
-    if (!plain && !nullOnly && !forceExact && !search && !ctx->tune.forceR && ctx->opts.rows_per_lane == 0 &&
-        (st = pipePlan(ctx, dp, mid, pipe)))
+    if (!plain && !nullOnly && !forceExact && !ctx->tune.forceR && ctx->opts.rows_per_lane == 0 &&
+        (st = pipePlan(ctx, dp, mid, search, pipe)))
         return st;
+    const bool pipeWhole = pipe.whole && pipe.clusters > 0;
     // Kernel groups by shape.  Chunks: runs of pairs of one profile and shape,
     // costliest first within each group.
     struct Group {
@@ -1853,7 +1866,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     // and the like keep them for the next such call) are given up when the
     // slots of a full GPU (every SM at the widest CTA) would not fit without them.
     size_t maxSlots = SIZE_MAX;
-    if (mid && !nullOnly && !pipe.clusters) {
+    if (mid && !nullOnly && !pipeWhole) {
         size_t freeB = 0, totalB = 0;
         CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
         const size_t held = (ctx->dW1.cap + ctx->dRing.cap) * sizeof(float);
@@ -1894,7 +1907,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         chunkPairsOf[q] =
             plain ? 1 : (int)std::max<long long>(1, std::min<long long>(4LL * G.warps, std::max(floorPairs, perCta)));
     }
-    for (size_t k = 0; k < n && !nullOnly && !pipe.clusters;) {
+    for (size_t k = 0; k < n && !nullOnly && !pipeWhole;) {
         Group &G = groups[groupOf(k)];
         size_t e = k;
         double cost = 0;
@@ -1975,13 +1988,15 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
             CK(cudaMemsetAsync(ctx->dPipeAbort.p, 0, ctx->dPipeAbort.cap * sizeof(int), ctx->stream), "zero abort flags");
             ctx->pipeClean = true;
         }
-        std::vector<int> list(n);
-        std::iota(list.begin(), list.end(), 0);
-        std::stable_sort(list.begin(), list.end(), [&](int x, int y) {
-            return (long long)(dp[x].M + 1) * dp[x].L > (long long)(dp[y].M + 1) * dp[y].L;
-        });
-        CK(ctx->dPipeList.ensure(n), "alloc pair list");
-        if ((st = upload(S.hPipeList, ctx->dPipeList.p, list.data(), n, "upload pair list"))) return st;
+        if (pipeWhole) {
+            std::vector<int> list(n);
+            std::iota(list.begin(), list.end(), 0);
+            std::stable_sort(list.begin(), list.end(), [&](int x, int y) {
+                return (long long)(dp[x].M + 1) * dp[x].L > (long long)(dp[y].M + 1) * dp[y].L;
+            });
+            CK(ctx->dPipeList.ensure(n), "alloc pair list");
+            if ((st = upload(S.hPipeList, ctx->dPipeList.p, list.data(), n, "upload pair list"))) return st;
+        }
     }
     CK(ctx->dRing.ensure(std::max<size_t>(slotsMax * ringSlot, 1), 0.25), "alloc ring slots");
     // one counter per group (search: the second wave's after them; the one-warp plain schedule: one per chunk)
@@ -2137,6 +2152,8 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         CK(S.hMask.ensure(n), "alloc survivors");
         CK(ctx->dMidChunks.ensure(std::max<size_t>(allChunks.size(), 1)), "alloc survivor chunks");
         CK(ctx->dSurvivors.ensure(std::max<size_t>(allChunks.size() * chunkStride, 1)), "alloc survivors");
+        CK(ctx->dSurvivorList.ensure(n), "alloc survivors");
+        CK(ctx->dSurvivorCount.ensure(2), "alloc survivors");
         CK(ctx->dMinBest.ensure(nProf), "alloc filter gates");
         if ((st = upload(S.hMinBest, ctx->dMinBest.p, minBest, nProf, "upload filter gates"))) return st;
     }
@@ -2191,36 +2208,60 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         CK(cudaGetLastError(), "null-model kernel");
         ++launches;
         CK(record(S.ev[1]), "event");
-        if (search) {
-            // the filter wave over every pair, then each chunk's survivors
-            for (int gi = 0; gi < kNumShapes; ++gi) {
-                Group &G = groups[gi];
-                if (G.chunks.empty()) continue;
-                DpArgs gk = g;
-                gk.out = S.dOutF.p;
-                gk.chunks = ctx->dChunks.p + G.chunkBase;
-                gk.nChunks = (int)G.chunks.size();
-                gk.chunkCounter = ctx->dCounter.p + gi;
-                G.kernF<<<G.grid, G.warps * kLanes, G.smem, ctx->stream>>>(gk, G.gt ? 0 : kNumCodes * G.maxRowPad);
-                CK(cudaGetLastError(), "filter kernel");
-                ++launches;
-            }
-            const int nc = (int)allChunks.size();
-            survivorKernel<<<(nc + 7) / 8, 256, 0, ctx->stream>>>(ctx->dChunks.p, nc, S.dOutF.p, ctx->dMinBest.p,
-                                                                  ctx->dMidChunks.p, ctx->dSurvivors.p, chunkStride,
-                                                                  S.dMask.p);
-            CK(cudaGetLastError(), "survivor kernel");
-            ++launches;
-        }
-        if (pipe.clusters) {
-            CK(cudaMemsetAsync(S.dOut.p, 0, n * sizeof(PairOut), ctx->stream), "zero results");
-            PipeArgs pa{ctx->dPipeList.p, nullptr, (int)n, g.pairs, g.profiles, g.emit, g.params, g.codes, g.seeds,
-                        g.scales, ctx->dW1.p, pipe.w1Slot, ctx->dPipeRing.p, pipe.ringSlot, ctx->dPipeAbort.p,
-                        S.dOut.p};
+        // the stripe pipeline over a list of pairs
+        auto pipeRun = [&](PipeKern kern, const int *list, const int *nList, int count, PairOut *out) -> int {
+            CK(cudaMemsetAsync(out, 0, n * sizeof(PairOut), ctx->stream), "zero results");
+            PipeArgs pa{list, nList, count, g.pairs, g.profiles, g.emit, g.params, g.codes, g.seeds,
+                        g.scales, ctx->dW1.p, pipe.w1Slot, ctx->dPipeRing.p, pipe.ringSlot, ctx->dPipeAbort.p, out};
             cudaLaunchAttribute at;
-            const cudaLaunchConfig_t cfg = clusterLaunch(pipe.C, pipe.W, pipe.smem, pipe.clusters * pipe.C, &at, ctx->stream);
-            CK(cudaLaunchKernelEx(&cfg, pipe.kern, pa), "stripe pipeline kernel");
+            const cudaLaunchConfig_t cfg =
+                clusterLaunch(pipe.C, pipe.W, pipe.smem, pipe.clusters * pipe.C, &at, ctx->stream);
+            CK(cudaLaunchKernelEx(&cfg, kern, pa), "stripe pipeline kernel");
             ++launches;
+            return DMST_OK;
+        };
+        int est = DMST_OK;
+        if (search) {
+            CK(cudaMemsetAsync(ctx->dSurvivorCount.p, 0, 2 * sizeof(int), ctx->stream), "zero survivors");
+            if (pipeWhole) {
+                if ((est = pipeRun(pipe.kernF, ctx->dPipeList.p, nullptr, (int)n, S.dOutF.p))) return est;
+                survivorListKernel<<<(int)((n + 255) / 256), 256, 0, ctx->stream>>>(
+                    ctx->dPipeList.p, (int)n, S.dPairs.p, S.dOutF.p, ctx->dMinBest.p, S.dMask.p, ctx->dSurvivorList.p,
+                    ctx->dSurvivorCount.p);
+                CK(cudaGetLastError(), "survivor kernel");
+                ++launches;
+            } else {
+                // the filter wave over every pair, then each chunk's survivors
+                for (int gi = 0; gi < kNumShapes; ++gi) {
+                    Group &G = groups[gi];
+                    if (G.chunks.empty()) continue;
+                    DpArgs gk = g;
+                    gk.out = S.dOutF.p;
+                    gk.chunks = ctx->dChunks.p + G.chunkBase;
+                    gk.nChunks = (int)G.chunks.size();
+                    gk.chunkCounter = ctx->dCounter.p + gi;
+                    G.kernF<<<G.grid, G.warps * kLanes, G.smem, ctx->stream>>>(gk, G.gt ? 0 : kNumCodes * G.maxRowPad);
+                    CK(cudaGetLastError(), "filter kernel");
+                    ++launches;
+                }
+                const int nc = (int)allChunks.size();
+                survivorKernel<<<(nc + 7) / 8, 256, 0, ctx->stream>>>(
+                    ctx->dChunks.p, nc, S.dOutF.p, ctx->dMinBest.p, ctx->dMidChunks.p, ctx->dSurvivors.p, chunkStride,
+                    S.dMask.p, ctx->dSurvivorList.p, ctx->dSurvivorCount.p);
+                CK(cudaGetLastError(), "survivor kernel");
+                ++launches;
+                if (pipe.clusters) {
+                    wavePlanKernel<<<(nc + 255) / 256, 256, 0, ctx->stream>>>(ctx->dMidChunks.p, nc, ctx->dSurvivorCount.p);
+                    CK(cudaGetLastError(), "survivor plan kernel");
+                    ++launches;
+                }
+            }
+            if (pipe.clusters && !forceExact &&
+                (est = pipeRun(pipe.kern, ctx->dSurvivorList.p, ctx->dSurvivorCount.p + 1, 0, S.dOut.p)))
+                return est;
+        }
+        if (pipeWhole && !search) {
+            if ((est = pipeRun(pipe.kern, ctx->dPipeList.p, nullptr, (int)n, S.dOut.p))) return est;
         } else if (!forceExact && !nullOnly) {
             for (int gi = 0; gi < kNumShapes; ++gi) {
                 Group &G = groups[gi];
@@ -2434,9 +2475,9 @@ static int completeCall(dmst_ctx *ctx) {
     const PairOut *pf = search ? S.hOutF.p : nullptr;
     if (S.pipe)
         for (size_t k = 0; k < n; ++k)
-            if (std::isnan(po[k].filt)) {  // a wait of the stripe pipeline ran out: its rings are not empty
-                ctx->pipeClean = false;
-                if (!mid) return ctx->fail(DMST_ETIMEOUT, "the stripe pipeline of pair %d gave up a wait", order[k]);
+            if (std::isnan(po[k].filt) || (search && std::isnan(pf[k].filt))) {
+                ctx->pipeClean = false;  // a wait of the stripe pipeline ran out: its rings are not empty
+                if (!mid || search) return ctx->fail(DMST_ETIMEOUT, "the stripe pipeline of pair %d gave up a wait", order[k]);
             }
     // Pairs outside the fast path's exact range go to the row-rescaled kernel.
     std::vector<int> flagged;

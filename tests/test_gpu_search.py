@@ -121,3 +121,27 @@ def test_search_equals_reference_two_waves(ref32, tmp_path):
             assert (r.mid.m, r.mid.e) == ref_mid[(p, s)], (p, s)
     assert got_surv == ref_surv
     assert 0 < len(ref_surv) < len(res)
+
+
+@pytest.mark.parametrize("reads,profiles", [(1, 1), (5, 2), (90, 10), (180, 10), (1100, 10)])
+def test_search_schedules_agree(reads, profiles):
+    """Both waves on the stripe pipeline (few pairs), its second wave only, and
+    (more than 8,192 survivors) the second wave as chunks: every result is the
+    filter and mid calls'."""
+    rng = np.random.default_rng(reads)
+    profs = [synth.make_profile(rng, int(M), f"w{k}") for k, M in enumerate(rng.integers(2, 200, profiles))]
+    txt = synth.hmmer3_text(profs)
+    seqs = synth.make_reads(rng, reads, 20, 260, profs, 0.3)
+    with d.Context() as ctx:
+        pids = ctx.load_hmm(txt)
+        sids = ctx.add_dna(seqs)
+        pr = _pairs(sids, pids)
+        flt = ctx.score_pairs_raw(pr, d.MODE_FILTER)
+        mid = ctx.score_pairs_raw(pr, d.MODE_MID)
+        for gate in (0.0, float(np.median([r.filter_f for r in flt]))):
+            got = ctx.search_raw(pr, np.full(len(pids), gate, np.float32))
+            for g, f, m in zip(got, flt, mid):
+                assert g.filter_f == f.filter_f
+                assert bool(g.flags & F.RES_SURVIVOR) == (f.filter_f >= gate and f.filter_f > 0)
+                if g.flags & F.RES_SURVIVOR:
+                    assert (g.mid.m, g.mid.e) == (m.mid.m, m.mid.e)
