@@ -546,6 +546,12 @@ void shapeOf(int M, int L, int forced, const Tuning &t, int &R, int &W) {
     W = t.forceWarps ? t.forceWarps : t.warps[c][rIndex(R)];
 }
 
+// CTA warps of the filter kernel (no W1, so fewer registers would do, but the
+// 8-warp build's 255 let it overlap more of a step): on the batched mix 11.2 ms
+// with four rows, 13.9 on 12 warps and 22.4 on 16; the same order for three and
+// two rows.
+constexpr int kFilterWarps = kCtaWarpsNarrow;
+
 }  // namespace
 
 // The per-call state of a scoring call in flight.  A context has two, so
@@ -1752,12 +1758,14 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         }
     }
     // The kernel shape of every pair (rows per lane and warps per CTA, from
-    // the profile's length and the read's length or its class).  A shape group too small to give every CTA two chunks would run as its
-    // own underfilled launch; its pairs join the largest group instead.
+    // the profile's length and the read's length or its class).  A shape group
+    // too small to give every CTA four chunks would run as its own underfilled
+    // launch; its pairs join the largest group instead.
     std::vector<int> pairShape(n);
     {
-        // tuned (or forced), the shape depends on the profile and the read's length class only
-        const bool byLength = !ctx->tune.tuned && !ctx->tune.forceR && ctx->opts.rows_per_lane == 0;
+        // tuned (or forced), the shape depends on the profile and the read's length class only; the filter
+        // kernel's rates are not the tuned ones (of the mid kernel)
+        const bool byLength = (!ctx->tune.tuned || !mid) && !ctx->tune.forceR && ctx->opts.rows_per_lane == 0;
         const size_t nProf = ctx->profiles.size();
         std::vector<int> shapeTab(2 * nProf);
         for (size_t q = 0; q < nProf; ++q)
@@ -1765,14 +1773,15 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                 int R, W;
                 shapeOf(ctx->profiles[q].M, c ? 0 : kShortRead, ctx->opts.rows_per_lane, ctx->tune, R, W);
                 if (plainStriped && R == 3) R = 4;  // the plain schedule's stripes take R = 4, 2 or 1
+                if (!mid) W = kFilterWarps;
                 shapeTab[2 * q + c] = rIndex(R) * 3 + wIndex(W);
             }
         long long groupPairs[kNumShapes] = {};
         for (size_t i = 0; i < n; ++i) {
             const int L = ctx->seqLen[pairs[i].seq];
             if (byLength) {
-                int R, W;
-                shapeOf(ctx->profiles[pairs[i].profile].M, L, 0, ctx->tune, R, W);
+                int R = untunedR(ctx->profiles[pairs[i].profile].M, L);
+                const int W = mid ? ctx->tune.warps[lengthClass(L)][rIndex(R)] : kFilterWarps;
                 if (plainStriped && R == 3) R = 4;
                 pairShape[i] = rIndex(R) * 3 + wIndex(W);
             } else {
@@ -1787,7 +1796,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
             int remap[kNumShapes];
             bool any = false;
             for (int q = 0; q < kNumShapes; ++q) {
-                const long long fill = 2LL * ctx->smCount * 4 * kShapeWarps[q % 3];
+                const long long fill = 4LL * ctx->smCount * 4 * kShapeWarps[q % 3];
                 remap[q] = (q != big && groupPairs[q] > 0 && groupPairs[q] < fill) ? big : q;
                 any |= remap[q] != q;
             }
@@ -1821,6 +1830,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     // costliest first within each group.
     struct Group {
         int R, warps;     // warps launched per CTA (<= kernWarps when shared memory is short)
+        int warpsF = 1;   // ... of a search's filter wave
         int kernWarps;    // the kernel's CTA shape (warp slots per CTA)
         DpKern kern;
         DpKern kernF = nullptr;  // search: the filter wave's kernel of the same shape
@@ -1898,7 +1908,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         const size_t winBytes = stagWindowBytes(G.R);
         G.gt = table + (size_t)G.kernWarps * winBytes > smemLimit;
         if (G.gt) G.kern = dpKernelFor(G.R, mid, G.kernWarps, true);
-        if (search) G.kernF = dpKernelFor(G.R, false, G.kernWarps, G.gt);
+        if (search) G.kernF = dpKernelFor(G.R, false, kFilterWarps, G.gt);
         G.warps = G.gt ? G.kernWarps : (int)std::min<size_t>(G.kernWarps, (smemLimit - table) / winBytes);
         G.warps = (int)std::max<size_t>(1, std::min<size_t>(G.warps, maxSlots / ctx->smCount));
         // Chunks of up to four pairs per launched warp, fewer when the group is
@@ -1907,9 +1917,13 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         // pairs leaves warps idle until the chunk's barrier).
         const long long perCta = groupPairs[q] / (4LL * ctx->smCount);
         const long long perSm = (groupPairs[q] + ctx->smCount - 1) / ctx->smCount;
-        const long long floorPairs = std::min<long long>(G.warps, perSm);
-        chunkPairsOf[q] =
-            plain ? 1 : (int)std::max<long long>(1, std::min<long long>(4LL * G.warps, std::max(floorPairs, perCta)));
+        const int warps = mid && !search ? G.warps : std::min(G.warps, kFilterWarps);
+        const long long floorPairs = std::min<long long>(warps, perSm);
+        // From two rounds of pairs on, whole rounds: a chunk of 27 pairs on 12
+        // warps takes as long as one of 36 (16,000 short pairs: 2.75 -> 2.30 ms).
+        long long chunk = std::max<long long>(1, std::min<long long>(4LL * warps, std::max(floorPairs, perCta)));
+        if (chunk >= 2 * warps) chunk = chunk / warps * warps;
+        chunkPairsOf[q] = plain ? 1 : (int)chunk;
     }
     for (size_t k = 0; k < n && !nullOnly && !pipeWhole;) {
         Group &G = groups[groupOf(k)];
@@ -1942,6 +1956,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         // Shared memory: the emission table, then one staging window per warp.
         const size_t table = (size_t)kNumCodes * G.maxRowPad * sizeof(float);
         G.smem = (G.gt ? 0 : table) + (size_t)G.warps * stagWindowBytes(G.R);
+        G.warpsF = std::min(G.warps, kFilterWarps);
         CK(cudaFuncSetAttribute(G.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G.smem),
            "smem attribute");
         if (search)
@@ -2244,7 +2259,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                     gk.chunks = ctx->dChunks.p + G.chunkBase;
                     gk.nChunks = (int)G.chunks.size();
                     gk.chunkCounter = ctx->dCounter.p + gi;
-                    G.kernF<<<G.grid, G.warps * kLanes, G.smem, ctx->stream>>>(gk, G.gt ? 0 : kNumCodes * G.maxRowPad);
+                    G.kernF<<<G.grid, G.warpsF * kLanes, G.smem, ctx->stream>>>(gk, G.gt ? 0 : kNumCodes * G.maxRowPad);
                     CK(cudaGetLastError(), "filter kernel");
                     ++launches;
                 }
