@@ -5,7 +5,7 @@
 // The reference decides each row's rescale after the whole row is known
 // (dummest-dp-backward.hh:560-573, dummest-dp-forward.hh:228-242), which a
 // wavefront cannot wait for.  So each direction runs twice (the kDiscover
-// and kReplay modes of the step functions in dp_wavefront.cuh):
+// and kReplay modes of the step functions below):
 //
 //  1. discovery: the same recurrence with a per-lane scale count that rises
 //     by one (values x 2^-64, exact) whenever a value passes 2^100, and that
@@ -35,11 +35,13 @@
 // every warp leaves its sweep, and the pair and those after it on the cluster
 // are marked failed.
 //
-// Bound: the latency of a step (the FP64 products and, in the replay, the
-// rescale factors add to the fast path's chain), so two rows per lane on as
-// many warps as there are stripes.  With four rows per lane on the 8 warps of
-// one CTA, 128-row stripes two to a warp, three pairs of M = 2000 x 10 kb took
-// 47 ms on three SMs.
+// Bound: the latency of a step, so two rows per lane, one column apart
+// (dp_stagger.cuh: neither waits for the other), on as many warps as there are
+// stripes; steps inside the read run without masks, and the FP64 products are
+// formed only for cells that can raise a row's best (rowBestFold).  Measured:
+// three windows of 10 kb against M = 2000 in 9.0 ms (170 ns a step), 18.7 with
+// two rows at one column and every product, 47 with four rows per lane on the
+// 8 warps of one CTA; 55 pairs of M = 400 x 2.2 kb in 2.0, 4.0 and 8.5 ms.
 #pragma once
 
 #include "dp_exact.cuh"
@@ -50,23 +52,21 @@ namespace dmst {
 
 constexpr int kExactRows = 2;  // rows per lane
 constexpr int kExactStripe = kLanes * kExactRows;
-constexpr int kExactMaxWarps = 16;
-// Steps of a block: a window entry per lane at most, and whole groups of the
-// step functions' three (six) phases.
-constexpr int kXBlock = 30;
-static_assert(kXBlock % 6 == 0 && kXBlock <= kLanes && 31 + 2 * kXBlock <= kWin, "window geometry");
-
+constexpr int kExactMaxWarps = 15;  // 227 KB of windows
+// Shared memory of a warp: the fast path's window, the discovery's ring counts
+// (mirrored like the ring), and the stripe's emission rows, code-major.
 struct WindowX {
-    Window w;
-    float emit[kNumCodes * kExactStripe];  // the stripe's emission rows, code-major
+    WindowS<kExactRows> s;
+    int cnt[kSRingWin + kSBlock];
+    float emit[kNumCodes * kExactStripe];
 };
 
 __host__ __device__ inline int exactStripes(int M) { return (M + kExactStripe) / kExactStripe; }
-// Scratch of a cluster (floats): W1 by stripe and diagonal, row maxima and
+// Scratch of a cluster (floats): W1 by stripe and step, row maxima and
 // counts of both discovery sweeps, reference counts, the warps' bests, and
 // with anchors the stripes' column partials.
 __host__ __device__ inline long long exactW1Floats(int M, int L) {
-    return (long long)exactStripes(M) * (L + kLanes - 1) * kExactStripe;
+    return exactStripes(M) * pipeStripeFloats(L, kExactRows);
 }
 __host__ __device__ inline long long exactPipeScratch(int M, int L, bool anchors) {
     const long long rows = 4LL * (M + 1) + 2LL * (M + 2);
@@ -106,47 +106,33 @@ struct ExactPipeArgs {
     int spinLimit;          // polls of a wait before it gives up
 };
 
-// A lane's operands of one window entry, as loaded.
+// A block's window entry of a lane, as loaded.
 struct FillX {
-    int code;
-    float suf, pre;
-    unsigned long long wy, cnt;
+    FillP p;
+    unsigned long long cnt;
 };
 
 template <bool BACKWARD, bool DISCOVER>
-__device__ __forceinline__ FillX fillLoadX(const SweepArgs &a, const unsigned long long *in, int first, int lane) {
-    FillX f{kPad, 0.0f, 0.0f, 0ull, 0ull};
-    const int u = first + lane;
-    if (lane < kXBlock && u < a.L) {
-        if (BACKWARD) {
-            const int j = a.L - 1 - u;
-            f.code = (j + 1 < a.L) ? (int)__ldg(a.codes() + j + 1) : kPad;
-            f.suf = __ldg(a.suf() + j);
-            f.pre = __ldg(a.pre() + j);
-        } else {
-            f.code = (u >= 2) ? (int)__ldg(a.codes() + u - 2) : kPad;
-            f.pre = __ldg(a.pre() + u);
-        }
-        if (in) {
-            f.wy = ringPeek(in + 2 * (size_t)u);
-            if (DISCOVER) f.cnt = ringPeek(in + 2 * (size_t)u + 1);
-        }
+__device__ __forceinline__ FillX fillLoadX(const SweepArgs &a, const unsigned long long *in, int u) {
+    FillX f{fillLoadP<BACKWARD>(a, nullptr, u), 0ull};
+    if (in && u < a.L) {
+        f.p.ring = ringPeek(in + 2 * (size_t)u);
+        if (DISCOVER) f.cnt = ringPeek(in + 2 * (size_t)u + 1);
     }
     return f;
 }
 
-// The window entries of a block, once their ring values are there; false:
+// The window entry of local time u, once its ring values are there; false:
 // given up.
 template <bool BACKWARD, bool DISCOVER>
-__device__ __forceinline__ bool fillStoreX(Window &w, const SweepArgs &a, FillX f, unsigned long long *in, int first,
-                                           int lane, int *abort, int spinLimit) {
-    const int u = first + lane;
+__device__ __forceinline__ bool fillStoreX(WindowX &w, const SweepArgs &a, FillX f, unsigned long long *in, int u,
+                                           int *abort, int spinLimit) {
     if (in) {
         int it = 0;
-        auto empty = [&]() { return f.wy == kRingEmpty || (DISCOVER && f.cnt == kRingEmpty); };
+        auto empty = [&]() { return f.p.ring == kRingEmpty || (DISCOVER && f.cnt == kRingEmpty); };
         while (__any_sync(kFull, empty())) {
             if (empty()) {
-                f.wy = ringPeek(in + 2 * (size_t)u);
+                f.p.ring = ringPeek(in + 2 * (size_t)u);
                 if (DISCOVER) f.cnt = ringPeek(in + 2 * (size_t)u + 1);
             }
             if (++it > spinLimit || (it & 63) == 0) {
@@ -157,101 +143,646 @@ __device__ __forceinline__ bool fillStoreX(Window &w, const SweepArgs &a, FillX 
                 }
             }
         }
-        if (lane < kXBlock && u < a.L) {
+        if (u < a.L) {
             ringPut(in + 2 * (size_t)u, kRingEmpty);
             if (DISCOVER) ringPut(in + 2 * (size_t)u + 1, kRingEmpty);
         }
     }
-    if (lane < kXBlock) {
-        const int e = u & (kWin - 1);
-        const float bg = a.smBg()[f.code], off = __int_as_float(f.code * a.rowPad);
-        w.col[e] = BACKWARD ? make_float4(off, bg, f.suf, f.pre) : make_float4(off, bg * a.sc().sC, f.pre, 0.0f);
-        w.ring[e] = make_float4(__uint_as_float((unsigned)f.wy), __uint_as_float((unsigned)(f.wy >> 32)),
-                                __uint_as_float((unsigned)f.cnt), 0.0f);
+    const FillRegs r{f.p.code, f.p.suf, f.p.pre, __uint_as_float((unsigned)f.p.ring),
+                     __uint_as_float((unsigned)(f.p.ring >> 32))};
+    fillStoreS<BACKWARD, kExactRows>(w.s, a, r, u);
+    if (DISCOVER) {
+        const int e = u & (kSRingWin - 1);
+        w.cnt[e] = (int)f.cnt;
+        if (e < kSBlock) w.cnt[e + kSRingWin] = (int)f.cnt;
     }
     return true;
 }
 
-// One stripe (b.sp = a.nS - 1 - s) of a backward sweep.
+// Two ring words of a column: (W, Y), and in the discovery its scale count.
+template <bool DISCOVER>
+__device__ __forceinline__ void ringPutX(unsigned long long *p, float w, float y, int cnt) {
+    ringPut(p, ((unsigned long long)__float_as_uint(y) << 32) | __float_as_uint(w));
+    if (DISCOVER) ringPut(p + 1, (unsigned)cnt);
+}
+
+// The largest exact product of a row, and the sum of its factors' bits as a
+// cheap upper test: the bits of a positive float are 2^23 times its binary
+// logarithm (biased) less at most 0.0861 2^23, so a product whose bit sum is
+// kBitSlack below the best's is smaller, and the double product, the
+// comparison and the select are left out for it (most cells).
+constexpr unsigned kBitSlack = 1445000;  // 2 x 0.0861 x 2^23, rounded up
+struct RowBest {
+    double v;
+    unsigned floor;
+};
+__device__ __forceinline__ void rowBestFold(RowBest &b, float x, float y) {
+    const unsigned bx = __float_as_uint(x), s = bx + __float_as_uint(y);
+    if (s >= b.floor && bx != 0) {
+        const double p = (double)x * (double)y;
+        if (p > b.v) {
+            b.v = p;
+            b.floor = s - kBitSlack;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The staggered steps of the exact path (dp_stagger.cuh's, two rows per lane,
+// with the discovery's scale counts or the replay's row factors).  GEN: steps
+// at which some lane is outside the read.
+// ---------------------------------------------------------------------------
+struct RunX {
+    const float4 *col;
+    const float2 *ring;
+    const int *cnt;
+    float *w1;
+    unsigned long long *out;
+};
+
 template <int MODE>
-__device__ bool exactBackward(const SweepArgs &a, Window &win, int s, int lane, unsigned long long *in, int *abort,
-                              int spinLimit, const ExactRows *x, ExactBest *exact) {
+struct BwdX {
+    Coef<kExactRows> c;
+    float h[4][2], z[4][2], rb[4], yPrev[2];
+    float ho[4];  // replay: row 1's W1 history as it leaves the row (after its rescale)
+    float bgH[4], sufH[4], preH[4], evH[4][2];
+    float sendW, sendY;
+    int u;
+    float *wp;
+    unsigned eS;
+    // discovery
+    int cnt, sendC;
+    float rmax[2];
+    // replay
+    float fOut[2];
+    int cOut[2];
+    RowBest best[2];
+    float *align;  // row-major W1 of the lane's row 0 at column L - 1 - u, or null
+};
+
+// Scales the lane's state by f and takes the count cnt (discovery).
+__device__ __forceinline__ void bwdRescaleX(BwdX<kDiscover> &b, float f, int cnt, int row, int M) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            b.h[q][k] *= f;
+            b.z[q][k] *= f;
+        }
+        b.rb[q] *= f;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        b.yPrev[k] *= f;
+        b.rmax[k] *= f;
+        b.c.rs[k] = seedCoef(row + k <= M, cnt);
+    }
+    b.cnt = cnt;
+}
+
+template <int MODE, int PH, bool GEN>
+__device__ __forceinline__ void bwdStepX(BwdX<MODE> &b, const SweepArgs &a, WindowX &w, int lane, int row, int M,
+                                         unsigned long long *out, const RunX &ip) {
     constexpr int R = kExactRows;
     constexpr bool kDisc = MODE == kDiscover;
-    BwdState<R, MODE> b;
-    b.sendW = b.sendY = b.filt = b.maxY = 0.0f;
-    b.sendC = b.cnt = 0;
-    b.u = -(kLanes - 1 - lane);  // lane 31 leads
-    b.sp = a.nS - 1 - s;
-    b.jj = 0;
-    backwardStart<R, MODE>(b, a, lane, s, x);
-    const int total = a.L;
-    const int T = (total + (kLanes - 1) + 2) / 3 * 3;
+    constexpr int SW = kLanes * R;
+    float inW = __shfl_down_sync(kFull, b.sendW, 1);
+    float inY = __shfl_down_sync(kFull, b.sendY, 1);
+    int inC = 0;
+    if (kDisc) inC = __shfl_down_sync(kFull, b.sendC, 1);
+    const float4 col = GEN ? w.s.col[b.u & (kSWin - 1)] : ip.col[PH];
+    if (lane == kLanes - 1) {
+        const float2 r = GEN ? w.s.ring[b.u & (kSRingWin - 1)] : ip.ring[PH];
+        inW = r.x;
+        inY = r.y;
+        if (kDisc) inC = GEN ? w.cnt[b.u & (kSRingWin - 1)] : ip.cnt[PH];
+    }
+    if constexpr (kDisc) {
+        // the incoming values and this lane to one scale
+        if ((!GEN || (b.u >= 0 && b.u < a.L + R)) && inC != b.cnt) {
+            if (inC > b.cnt) {
+                bwdRescaleX(b, stepsDown(inC - b.cnt), inC, row, M);
+            } else {
+                const float f = stepsDown(b.cnt - inC);
+                inW *= f;
+                inY *= f;
+            }
+        }
+    }
+    float ev[R];
+    loadEmitS<R>(ev, b.eS + 4u * (unsigned)__float_as_int(col.x));
+    b.bgH[PH] = col.y;
+    b.sufH[PH] = col.z;
+    b.preH[PH] = col.w;
+#pragma unroll
+    for (int k = 0; k < R; ++k) b.evH[PH][k] = ev[k];
+    b.rb[PH] = inW;
+    float nW[R], nY[R], nZ[R], pv[R];
+    bool act[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int D = R - 1 - k;
+        const int Q = (PH + 4 - D) & 3;
+        pv[k] = b.preH[Q];
+        float Wb1, Wb2, Wb3, Yb;  // the row below: W1 at columns j+1, j+2, j+3 and Y at j
+        if (k == R - 1) {
+            Wb1 = b.rb[(PH + 3) & 3];
+            Wb2 = b.rb[(PH + 2) & 3];
+            Wb3 = b.rb[(PH + 1) & 3];
+            Yb = inY;
+        } else if (kDisc) {
+            Wb1 = b.h[(PH + 2) & 3][k + 1];
+            Wb2 = b.h[(PH + 1) & 3][k + 1];
+            Wb3 = b.h[PH][k + 1];
+            Yb = b.yPrev[k + 1];
+        } else {
+            Wb1 = b.ho[(PH + 2) & 3];
+            Wb2 = b.ho[(PH + 1) & 3];
+            Wb3 = b.ho[PH];
+            Yb = b.yPrev[k + 1];
+        }
+        const float p = (Wb3 * b.evH[Q][k]) * b.c.enter[k];
+        float acc = __fmaf_rn(Yb, b.c.d0[k], p);
+        acc = __fmaf_rn(Wb2, b.c.d1[k], acc);
+        acc = __fmaf_rn(Wb1, b.c.d2[k], acc);
+        const float zbg = b.z[(PH + 1) & 3][k] * b.bgH[Q];
+        acc = __fmaf_rn(zbg, b.c.a0[k], acc);
+        acc = __fmaf_rn(b.h[(PH + 2) & 3][k], b.c.a2[k], acc);
+        acc = __fmaf_rn(b.h[(PH + 3) & 3][k], b.c.a1[k], acc);
+        float W = __fmaf_rn(b.sufH[Q], b.c.rs[k], acc);
+        float Y = __fmaf_rn(b.c.eps[k], Yb, W);
+        float Z = __fmaf_rn(b.c.b0[k], zbg, W);
+        act[k] = true;
+        if (GEN) {
+            act[k] = b.u >= D && b.u < a.L + D;
+            if (!act[k]) W = Y = Z = 0.0f;
+        }
+        nW[k] = W;
+        nY[k] = Y;
+        nZ[k] = Z;
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        b.h[PH][k] = nW[k];
+        b.z[PH][k] = nZ[k];
+        if (kDisc) {
+            b.rmax[k] = fmaxf(b.rmax[k], nY[k]);  // Y >= W1 at every cell
+            b.yPrev[k] = nY[k];
+        }
+    }
+    if constexpr (kDisc) {
+        if (fmaxf(nY[0], nY[1]) > kBump) bwdRescaleX(b, kStep, b.cnt + 1, row, M);
+        b.sendW = b.h[PH][0];
+        b.sendY = b.yPrev[0];
+        b.sendC = b.cnt;
+    } else {
+        if (b.align != nullptr) {
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+                if (act[k] && row + k <= M) b.align[(ptrdiff_t)k * a.L - (b.u - (R - 1 - k))] = nW[k];
+        }
+        // what leaves a row is scaled by the row's own decision
+        float oW[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            oW[k] = nW[k] * b.fOut[k];
+            b.yPrev[k] = nY[k] * b.fOut[k];
+            rowBestFold(b.best[k], oW[k], pv[k]);
+        }
+        b.ho[PH] = oW[1];
+        b.sendW = oW[0];
+        b.sendY = b.yPrev[0];
+        storeW1S<R>(GEN ? b.wp : ip.w1 + PH * SW, oW);
+    }
+    if (lane == 0 && out != nullptr) {
+        if (GEN) {
+            if (act[0]) ringPutX<kDisc>(out + 2 * (ptrdiff_t)(b.u - (R - 1)), b.sendW, b.sendY, b.cnt);
+        } else {
+            ringPutX<kDisc>(ip.out + 2 * PH, b.sendW, b.sendY, b.cnt);
+        }
+    }
+    if (GEN) {
+        b.wp += SW;
+        ++b.u;
+    } else if (!kDisc && b.align != nullptr) {
+        ++b.u;  // otherwise the run advances it
+    }
+}
+
+// One stripe of a backward sweep; `out`: its ring to the stripe below.
+template <int MODE>
+__device__ bool exactBackward(const SweepArgs &a, WindowX &w, int s, int lane, unsigned long long *in,
+                              unsigned long long *out, int *abort, int spinLimit, const ExactRows &x,
+                              ExactBest *exact) {
+    constexpr int R = kExactRows, S = kExactStripe, SW = kLanes * R;
+    constexpr bool kDisc = MODE == kDiscover;
+    const int M = a.M(), row = s * S + lane * R;
+    BwdX<MODE> b;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) b.h[q][k] = b.z[q][k] = b.evH[q][k] = 0.0f;
+        b.rb[q] = b.ho[q] = b.bgH[q] = b.sufH[q] = b.preH[q] = 0.0f;
+    }
+    loadBackwardCoef<R>(b.c, a, row);
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int i = row + k;
+        b.yPrev[k] = b.rmax[k] = 0.0f;
+        b.best[k] = RowBest{0.0, 0u};
+        b.fOut[k] = 1.0f;
+        b.cOut[k] = 0;
+        if (!kDisc) {
+            const int ci = i <= M ? i : M + 1;
+            const int cIn = __ldcg(x.cntB + min(ci + 1, M + 1));
+            b.cOut[k] = __ldcg(x.cntB + ci);
+            b.fOut[k] = stepsDown(b.cOut[k] - cIn);
+            b.c.rs[k] = seedCoef(i <= M, cIn);
+        }
+    }
+    b.sendW = b.sendY = 0.0f;
+    b.cnt = b.sendC = 0;
+    b.u = -(kLanes - 1 - lane) * R;
+    b.wp = a.w1 + lane * R;
+    b.eS = (unsigned)__cvta_generic_to_shared(a.smE + lane * R);
+    b.align = !kDisc && a.alignOut ? a.alignOut + (size_t)row * a.L + (a.L - 1) : nullptr;
+    const int T = (a.L - 1 + S + 3) / 4 * 4;
+    for (int v = -S + lane; v < 0; v += kLanes) fillStoreX<true, kDisc>(w, a, FillX{{kPad, 0.0f, 0.0f, 0ull}, 0ull}, nullptr, v, abort, 0);
     __syncwarp();
-    FillX f = fillLoadX<true, kDisc>(a, in, 0, lane);
-    if (!fillStoreX<true, kDisc>(win, a, f, in, 0, lane, abort, spinLimit)) return false;
-    f = fillLoadX<true, kDisc>(a, in, kXBlock, lane);
-    for (int t0 = 0; t0 < T; t0 += kXBlock) {
+    FillX f = fillLoadX<true, kDisc>(a, in, lane);
+    if (!fillStoreX<true, kDisc>(w, a, f, in, lane, abort, spinLimit)) return false;
+    f = fillLoadX<true, kDisc>(a, in, kSBlock + lane);
+    for (int t0 = 0; t0 < T; t0 += kSBlock) {
         __syncwarp();
-        if (!fillStoreX<true, kDisc>(win, a, f, in, t0 + kXBlock, lane, abort, spinLimit)) return false;
-        f = fillLoadX<true, kDisc>(a, in, t0 + 2 * kXBlock, lane);
+        if (!fillStoreX<true, kDisc>(w, a, f, in, t0 + kSBlock + lane, abort, spinLimit)) return false;
+        f = fillLoadX<true, kDisc>(a, in, t0 + 2 * kSBlock + lane);
         __syncwarp();
-        const int n = min(kXBlock, T - t0);
+        const int n = min(kSBlock, T - t0);
+        int gA, gB;
+        interiorRunS<4>(a, S, t0, n, gA, gB);
+        int g = 0;
+        RunX ip{nullptr, nullptr, nullptr, nullptr, nullptr};
 #pragma unroll 1
-        for (int g = 0; g < n; g += 3) {
-            backwardStep<R, MODE, 0, true, true, false>(b, a, win, lane, total, x, exact);
-            backwardStep<R, MODE, 1, true, true, false>(b, a, win, lane, total, x, exact);
-            backwardStep<R, MODE, 2, true, true, false>(b, a, win, lane, total, x, exact);
+        for (; g < gA; g += 4) {
+            bwdStepX<MODE, 0, true>(b, a, w, lane, row, M, out, ip);
+            bwdStepX<MODE, 1, true>(b, a, w, lane, row, M, out, ip);
+            bwdStepX<MODE, 2, true>(b, a, w, lane, row, M, out, ip);
+            bwdStepX<MODE, 3, true>(b, a, w, lane, row, M, out, ip);
+        }
+        if (gB > gA) {
+            const int u0 = b.u;
+            ip.col = w.s.col + (b.u & (kSWin - 1));
+            ip.ring = w.s.ring + (b.u & (kSRingWin - 1));
+            ip.cnt = w.cnt + (b.u & (kSRingWin - 1));
+            ip.w1 = b.wp;
+            ip.out = out + 2 * (ptrdiff_t)(b.u - (R - 1));
+#pragma unroll 1
+            for (; g < gB; g += 4) {
+                bwdStepX<MODE, 0, false>(b, a, w, lane, row, M, out, ip);
+                bwdStepX<MODE, 1, false>(b, a, w, lane, row, M, out, ip);
+                bwdStepX<MODE, 2, false>(b, a, w, lane, row, M, out, ip);
+                bwdStepX<MODE, 3, false>(b, a, w, lane, row, M, out, ip);
+                ip.col += 4;
+                ip.ring += 4;
+                ip.cnt += 4;
+                ip.w1 += 4 * SW;
+                ip.out += 8;
+            }
+            b.u = u0 + (gB - gA);
+            b.wp += (gB - gA) * SW;
+        }
+#pragma unroll 1
+        for (; g < n; g += 4) {
+            bwdStepX<MODE, 0, true>(b, a, w, lane, row, M, out, ip);
+            bwdStepX<MODE, 1, true>(b, a, w, lane, row, M, out, ip);
+            bwdStepX<MODE, 2, true>(b, a, w, lane, row, M, out, ip);
+            bwdStepX<MODE, 3, true>(b, a, w, lane, row, M, out, ip);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        if (row + k > M) continue;
+        if (kDisc) {
+            x.rowMax[row + k] = b.rmax[k];
+            x.rowCnt[row + k] = b.cnt;
+        } else {
+            foldBest(*exact, b.best[k].v, b.cOut[k]);
         }
     }
     return true;
 }
 
-// One stripe of a forward sweep.
-template <int MODE, bool ANCH>
-__device__ bool exactForward(const SweepArgs &a, Window &win, int s, int lane, unsigned long long *in, int *abort,
-                             int spinLimit, const ExactRows *x, ExactBest *exact) {
+// A column's best wMid on its way up the rows, and its row.
+struct Anchor {
+    float m;
+    int e, row;
+};
+
+template <int MODE>
+struct FwdX {
+    Coef<kExactRows> c;
+    float w[4][2], z[4][2], ninPrev[2], yPrev[2];
+    float bgH[4], preH[4], evH[4][2];
+    float sendIn, sendY;
+    int u;
+    unsigned eS;
+    const float *w1src;
+    int gAhead;
+    // discovery
+    int cnt, sendC;
+    float rmax[2];
+    // replay
+    float fOut[2];
+    int cSum[2];  // the row's forward count (before the row) plus its backward count
+    RowBest best[2];
+    Anchor an[2];  // anchors: per row, the column's best up to it
+    float *align;  // row-major W0 of the lane's row 0 at column u, or null
+};
+
+__device__ __forceinline__ void fwdRescaleX(FwdX<kDiscover> &f, float g, int cnt, int row, int M) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            f.w[q][k] *= g;
+            f.z[q][k] *= g;
+        }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        f.ninPrev[k] *= g;
+        f.yPrev[k] *= g;
+        f.rmax[k] *= g;
+        f.c.rs[k] = seedCoef(row + k <= M, cnt);
+    }
+    f.cnt = cnt;
+}
+
+template <int MODE, int PH, bool GEN, bool ANCH>
+__device__ __forceinline__ void fwdStepX(FwdX<MODE> &f, const SweepArgs &a, WindowX &w, int s, int lane, int row, int M,
+                                         unsigned long long *out, float *part, const RunX &ip) {
     constexpr int R = kExactRows;
     constexpr bool kDisc = MODE == kDiscover;
-    FwdState<R, MODE> f;
-    f.sendIn = f.sendY = f.best = f.mx = 0.0f;
-    f.sendC = f.cnt = 0;
-    f.sendAM = 0.0f;
-    f.sendAE = f.sendAR = 0;
-    f.u = -lane;  // lane 0 leads
-    f.s = s;
-    f.j = 0;
-    forwardStart<R, MODE>(f, a, lane, s, x);
-    const int total = a.L;
-    const int T = (total + (kLanes - 1) + 5) / 6 * 6;
-    W1Stage<R, true> st{-lane, s, 0};
-    if (MODE == kReplay) {
-#pragma unroll
-        for (int k = 0; k < kW1Ahead; ++k) st.issue(a, win, k, lane, total);
+    constexpr int SW = kLanes * R;
+    constexpr int H = PH & 3;
+    float q[R] = {0.0f, 0.0f};
+    if (!kDisc) {
+        cpAsyncWait<kSW1Ahead - 1>();
+        const float2 v = *reinterpret_cast<const float2 *>(&w.s.w1[PH][lane * 2]);
+        q[0] = v.x;
+        q[1] = v.y;
     }
-    __syncwarp();
-    FillX g = fillLoadX<false, kDisc>(a, in, 0, lane);
-    bool ok = fillStoreX<false, kDisc>(win, a, g, in, 0, lane, abort, spinLimit);
-    if (ok) g = fillLoadX<false, kDisc>(a, in, kXBlock, lane);
-    for (int t0 = 0; ok && t0 < T; t0 += kXBlock) {
-        __syncwarp();
-        ok = fillStoreX<false, kDisc>(win, a, g, in, t0 + kXBlock, lane, abort, spinLimit);
-        if (!ok) break;
-        g = fillLoadX<false, kDisc>(a, in, t0 + 2 * kXBlock, lane);
-        __syncwarp();
-        const int n = min(kXBlock, T - t0);
-#pragma unroll 1
-        for (int q = 0; q < n; q += 6) {
-            forwardStaged<R, MODE, 0, ANCH, true, true, false>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 1, ANCH, true, true, false>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 2, ANCH, true, true, false>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 3, ANCH, true, true, false>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 4, ANCH, true, true, false>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 5, ANCH, true, true, false>(f, a, win, lane, total, st, x, exact);
+    float inW = __shfl_up_sync(kFull, f.sendIn, 1);
+    float inY = __shfl_up_sync(kFull, f.sendY, 1);
+    int inC = 0;
+    if (kDisc) inC = __shfl_up_sync(kFull, f.sendC, 1);
+    Anchor inA{0.0f, 0, 0};
+    if (ANCH) {
+        inA.m = __shfl_up_sync(kFull, f.an[R - 1].m, 1);
+        inA.e = __shfl_up_sync(kFull, f.an[R - 1].e, 1);
+        inA.row = __shfl_up_sync(kFull, f.an[R - 1].row, 1);
+        if (lane == 0) inA = Anchor{0.0f, 0, 0};  // the rows below are another stripe's partial
+    }
+    const float4 col = GEN ? w.s.col[f.u & (kSWin - 1)] : ip.col[PH];
+    if (lane == 0) {
+        const float2 r = GEN ? w.s.ring[f.u & (kSRingWin - 1)] : ip.ring[PH];
+        inW = r.x;
+        inY = r.y;
+        if (kDisc) inC = GEN ? w.cnt[f.u & (kSRingWin - 1)] : ip.cnt[PH];
+    }
+    if constexpr (kDisc) {
+        if ((!GEN || (f.u >= 0 && f.u < a.L + R)) && inC != f.cnt) {
+            if (inC > f.cnt) {
+                fwdRescaleX(f, stepsDown(inC - f.cnt), inC, row, M);
+            } else {
+                const float g = stepsDown(f.cnt - inC);
+                inW *= g;
+                inY *= g;
+            }
         }
     }
-    if (MODE == kReplay) cpAsyncWait<0>();  // no copy outlives the sweep (the slots are reused)
-    return ok;
+    float ev[R];
+    loadEmitS<R>(ev, f.eS + 4u * (unsigned)__float_as_int(col.x));
+    f.bgH[H] = col.y;
+    f.preH[H] = col.z;
+#pragma unroll
+    for (int k = 0; k < R; ++k) f.evH[H][k] = ev[k];
+    float nW[R], nZ[R], nN[R], nY[R];
+    bool act[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int Q = (H + 4 - k) & 3;
+        const float win0 = k == 0 ? inW : f.ninPrev[k - 1];
+        const float yab = k == 0 ? inY : f.yPrev[k - 1];
+        const float w1 = f.w[(H + 3) & 3][k], w2 = f.w[(H + 2) & 3][k], w3 = f.w[(H + 1) & 3][k];
+        const float X = (f.c.enter[k] * f.evH[Q][k]) * w3;
+        float Z0 = f.bgH[Q] * __fmaf_rn(f.c.b0[k], f.z[(H + 1) & 3][k], f.c.a0[k] * w3);
+        const float zs = __fmaf_rn(f.c.a2[k], w2, __fmaf_rn(f.c.a1[k], w1, Z0));
+        float W0 = win0 + __fmaf_rn(f.preH[Q], f.c.rs[k], zs);
+        float Y0 = __fmaf_rn(f.c.eps[k], yab, f.c.d0[k] * W0);
+        float nin = __fmaf_rn(f.c.d2[k], w1, __fmaf_rn(f.c.d1[k], w2, X + Y0));
+        act[k] = true;
+        if (GEN) {
+            act[k] = f.u >= k && f.u < a.L + k;
+            if (!act[k]) W0 = Y0 = nin = Z0 = 0.0f;
+        }
+        nW[k] = W0;
+        nZ[k] = Z0;
+        nN[k] = nin;
+        nY[k] = Y0;
+    }
+    if constexpr (!kDisc) {
+        if (ANCH) {
+            // wMid = promote(W0) promote(W1): the exact double product, its
+            // mantissa rounded to float (dummest-batch.hh:216-235); rows in
+            // ascending order, the first row on ties (row k folds what row
+            // k - 1 left for its column a step ago)
+            const Anchor from[R] = {inA, f.an[0]};
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                Anchor an = from[k];
+                const unsigned bw = __float_as_uint(nW[k]), bq = __float_as_uint(q[k]);
+                if (act[k] && row + k <= M && bw != 0 && bq != 0 &&
+                    (an.m == 0.0f || (int)(bw >> 23) + (int)(bq >> 23) - 252 + kRescaleBits * f.cSum[k] >= an.e)) {
+                    const XS v = splitNorm((double)nW[k] * (double)q[k], kRescaleBits * f.cSum[k]);
+                    if (xsLessMe(an.m, an.e, v.m, v.e)) an = Anchor{v.m, v.e, row + k};
+                }
+                f.an[k] = an;
+            }
+            if (lane == kLanes - 1 && act[R - 1]) {
+                float *pp = part + ((size_t)s * a.L + (f.u - (R - 1))) * 3;
+                pp[0] = f.an[R - 1].m;
+                pp[1] = __int_as_float(f.an[R - 1].e);
+                pp[2] = __int_as_float(f.an[R - 1].row);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k) rowBestFold(f.best[k], nW[k], q[k]);
+        if (f.align != nullptr) {
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+                if (act[k] && row + k <= M) f.align[(ptrdiff_t)k * a.L + (f.u - k)] = nW[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        f.w[H][k] = nW[k];
+        f.z[H][k] = nZ[k];
+        f.ninPrev[k] = kDisc ? nN[k] : nN[k] * f.fOut[k];
+        f.yPrev[k] = kDisc ? nY[k] : nY[k] * f.fOut[k];
+        if (kDisc) f.rmax[k] = fmaxf(f.rmax[k], fmaxf(nW[k], nY[k]));
+    }
+    if constexpr (kDisc) {
+        if (fmaxf(fmaxf(fmaxf(nW[0], nY[0]), fmaxf(nW[1], nY[1])), fmaxf(nN[0], nN[1])) > kBump)
+            fwdRescaleX(f, kStep, f.cnt + 1, row, M);
+        f.sendC = f.cnt;
+    }
+    f.sendIn = f.ninPrev[R - 1];
+    f.sendY = f.yPrev[R - 1];
+    if (lane == kLanes - 1 && out != nullptr) {
+        if (GEN) {
+            if (act[R - 1]) ringPutX<kDisc>(out + 2 * (ptrdiff_t)(f.u - (R - 1)), f.sendIn, f.sendY, f.cnt);
+        } else {
+            ringPutX<kDisc>(ip.out + 2 * PH, f.sendIn, f.sendY, f.cnt);
+        }
+    }
+    if (!kDisc) {
+        float *slot = &w.s.w1[(PH + kSW1Ahead) % kSW1Slots][lane * R];
+        if (GEN) {
+            if (f.gAhead >= 0) cpAsyncStage<R>(slot, f.w1src);
+        } else {
+            cpAsyncStage<R>(slot, ip.w1 - PH * SW);
+        }
+        cpAsyncCommit();
+    }
+    if (GEN) {
+        f.w1src -= SW;
+        --f.gAhead;
+        ++f.u;
+    } else if (!kDisc && (ANCH || f.align != nullptr)) {
+        ++f.u;  // otherwise the run advances it
+    }
+}
+
+// One stripe of a forward sweep; part: the columns' partial anchors (ANCH).
+template <int MODE, bool ANCH>
+__device__ bool exactForward(const SweepArgs &a, WindowX &w, int s, int lane, unsigned long long *in,
+                             unsigned long long *out, int *abort, int spinLimit, const ExactRows &x, ExactBest *exact) {
+    constexpr int R = kExactRows, S = kExactStripe, SW = kLanes * R;
+    constexpr bool kDisc = MODE == kDiscover;
+    const int M = a.M(), row = s * S + lane * R;
+    FwdX<MODE> f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) f.w[q][k] = f.z[q][k] = f.evH[q][k] = 0.0f;
+        f.bgH[q] = f.preH[q] = 0.0f;
+    }
+    loadForwardCoef<R>(f.c, a, row);
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int i = row + k;
+        f.ninPrev[k] = f.yPrev[k] = f.rmax[k] = 0.0f;
+        f.best[k] = RowBest{0.0, 0u};
+        f.an[k] = Anchor{0.0f, 0, 0};
+        f.fOut[k] = 1.0f;
+        f.cSum[k] = 0;
+        if (!kDisc) {
+            const int ci = i <= M ? i : M;
+            const int cIn = __ldcg(x.cntF + ci);
+            f.fOut[k] = stepsDown(__ldcg(x.cntF + ci + 1) - cIn);
+            f.cSum[k] = cIn + __ldcg(x.cntB + ci);
+            f.c.rs[k] = seedCoef(i <= M, cIn);
+        }
+    }
+    f.sendIn = f.sendY = 0.0f;
+    f.cnt = f.sendC = 0;
+    f.u = -lane * R;
+    f.eS = (unsigned)__cvta_generic_to_shared(a.smE + lane * R);
+    f.align = !kDisc && a.alignOut ? a.alignOut + (size_t)row * a.L : nullptr;
+    const int steps = a.L - 1 + S;
+    const int T = (steps + kSW1Slots - 1) / kSW1Slots * kSW1Slots;
+    f.w1src = a.w1 + (size_t)(steps - 1) * SW + lane * R;
+    f.gAhead = steps - 1 - kSW1Ahead;
+    if (!kDisc) {
+#pragma unroll
+        for (int k = 0; k < kSW1Ahead; ++k) {
+            cpAsyncStage<R>(&w.s.w1[k][lane * R], f.w1src);
+            cpAsyncCommit();
+            f.w1src -= SW;
+        }
+    }
+    for (int v = -S + lane; v < 0; v += kLanes) fillStoreX<false, kDisc>(w, a, FillX{{kPad, 0.0f, 0.0f, 0ull}, 0ull}, nullptr, v, abort, 0);
+    __syncwarp();
+    FillX p = fillLoadX<false, kDisc>(a, in, lane);
+    bool ok = fillStoreX<false, kDisc>(w, a, p, in, lane, abort, spinLimit);
+    if (ok) p = fillLoadX<false, kDisc>(a, in, kSBlock + lane);
+    for (int t0 = 0; ok && t0 < T; t0 += kSBlock) {
+        __syncwarp();
+        ok = fillStoreX<false, kDisc>(w, a, p, in, t0 + kSBlock + lane, abort, spinLimit);
+        if (!ok) break;
+        p = fillLoadX<false, kDisc>(a, in, t0 + 2 * kSBlock + lane);
+        __syncwarp();
+        const int n = min(kSBlock, T - t0);
+        int gA, gB;
+        interiorRunS<8>(a, S, t0, n, gA, gB);
+        int g = 0;
+        RunX ip{nullptr, nullptr, nullptr, nullptr, nullptr};
+        auto general = [&](int end) {
+#pragma unroll 1
+            for (; g < end; g += 8) {
+                fwdStepX<MODE, 0, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 1, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 2, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 3, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 4, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 5, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 6, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 7, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+            }
+        };
+        if (gB > gA) {
+            general(gA);
+            const int u0 = f.u;
+            ip.col = w.s.col + (f.u & (kSWin - 1));
+            ip.ring = w.s.ring + (f.u & (kSRingWin - 1));
+            ip.cnt = w.cnt + (f.u & (kSRingWin - 1));
+            ip.w1 = const_cast<float *>(f.w1src);
+            ip.out = out + 2 * (ptrdiff_t)(f.u - (R - 1));
+#pragma unroll 1
+            for (; g < gB; g += 8) {
+                fwdStepX<MODE, 0, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 1, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 2, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 3, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 4, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 5, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 6, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                fwdStepX<MODE, 7, false, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
+                ip.col += 8;
+                ip.ring += 8;
+                ip.cnt += 8;
+                ip.w1 -= 8 * SW;
+                ip.out += 16;
+            }
+            f.u = u0 + (gB - gA);
+            f.w1src -= (gB - gA) * SW;
+            f.gAhead -= gB - gA;
+        }
+        general(n);
+    }
+    if (!kDisc) cpAsyncWait<0>();  // no copy outlives the sweep (the slots are reused)
+    if (!ok) return false;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        if (row + k > M) continue;
+        if (kDisc) {
+            x.rowMax[row + k] = f.rmax[k];
+            x.rowCnt[row + k] = f.cnt;
+        } else {
+            foldBest(*exact, f.best[k].v, f.cSum[k]);
+        }
+    }
+    return true;
 }
 
 __device__ __forceinline__ ExactBest warpBest(ExactBest b) {
@@ -355,7 +886,6 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
     __shared__ float smBg[32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WindowX &wx = reinterpret_cast<WindowX *>(smRaw)[warp];
-    Window &win = wx.w;
     const int C = clusterSize(), rank = clusterRank(), G = C * (blockDim.x >> 5);
     const int me = warp * C + rank;  // consecutive stripes on different CTAs
     const int cluster = blockIdx.x / C, nClusters = gridDim.x / C;
@@ -371,7 +901,7 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
         clusterSync(C);  // the previous pair's scratch, ring and background are done with
         if (warp == 0) smBg[lane] = lane < kNumCodes ? pr.bg[lane] : 0.0f;
         if (lane == 0) {
-            PairCold &c = win.cold;
+            PairCold &c = wx.s.cold;
             c.codes = g.codes + p.codeOff;
             c.pre = g.seeds + p.seedOff;
             c.suf = c.pre + p.L;
@@ -383,17 +913,15 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
         }
         __syncthreads();
         SweepArgs a;
-        a.cold = &win.cold;
+        a.cold = &wx.s.cold;
         a.L = p.L;
         a.rowPad = kExactStripe;
-        a.nS = nS;
+        a.nS = 1;
         a.P = INT_MAX / 4;  // a stripe's sweep never reaches another stripe
-        a.D = p.L + kLanes - 1;
-        a.sFirst = 0;
-        a.sStep = a.nMine = 1;
-        a.ringSlots = nS;
-        a.ringStride = 4LL * p.L;
-        a.w1 = base;
+        a.D = a.sFirst = 0;
+        a.sStep = a.nMine = a.ringSlots = 1;
+        a.ringStride = 0;
+        a.ring = nullptr;
         a.alignOut = nullptr;
         ExactRows x;
         float *rows = base + exactW1Floats(p.M, p.L);
@@ -404,7 +932,8 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
         double *bests = reinterpret_cast<double *>(
             base + (exactW1Floats(p.M, p.L) + 4LL * (p.M + 1) + 2LL * (p.M + 2) + 3) / 4 * 4);
         x.anchorPart = reinterpret_cast<float *>(bests + 4 * kPipeMaxCluster * kExactMaxWarps);
-        // The stripe's emission rows in shared memory, addressed by profile row.
+        const long long stripeFloats = pipeStripeFloats(p.L, kExactRows);
+        // The stripe's emission rows in shared memory, and its W1.
         auto stripe = [&](int s) {
             __syncwarp();
             const float *src = g.emit + pr.emitOff + (size_t)s * kExactStripe + lane * kExactRows;
@@ -413,29 +942,29 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
                 *reinterpret_cast<float2 *>(wx.emit + c * kExactStripe + lane * 2) =
                     __ldg(reinterpret_cast<const float2 *>(src + (size_t)c * pr.rowPad));
             __syncwarp();
-            a.smE = wx.emit - s * kExactStripe;
+            a.smE = wx.emit;
+            a.w1 = base + s * stripeFloats;
         };
         unsigned long long *rb = ring, *rf = ring + 2LL * nS * p.L;  // boundary rows downward and upward
         const int sLast = nS - 1 >= me ? me + (nS - 1 - me) / G * G : -1;
         bool ok = abortPeek(abort) == 0;  // a wait of an earlier pair ran out: no later pair is started
         ExactBest filt{0.0, 0}, mid{0.0, 0};
-        // Stripe s hands its row to the next through entry row sp of the
-        // step functions' numbering (the processing order).
-        auto backIn = [&](int s) { return s < nS - 1 ? rb + 2LL * (nS - 2 - s) * p.L : nullptr; };
+        // Stripe s hands its boundary row on through entry row s of a ring.
+        auto backIn = [&](int s) { return s < nS - 1 ? rb + 2LL * (s + 1) * p.L : nullptr; };
+        auto backOut = [&](int s) { return s > 0 ? rb + 2LL * s * p.L : nullptr; };
         auto foreIn = [&](int s) { return s > 0 ? rf + 2LL * (s - 1) * p.L : nullptr; };
-        a.ring = reinterpret_cast<float *>(rb);
+        auto foreOut = [&](int s) { return s < nS - 1 ? rf + 2LL * s * p.L : nullptr; };
         x.rowMax = maxB;
         x.rowCnt = rcB;
         for (int s = sLast; s >= 0 && ok; s -= G) {
             stripe(s);
-            ok = exactBackward<kDiscover>(a, win, s, lane, backIn(s), abort, g.spinLimit, &x, nullptr);
+            ok = exactBackward<kDiscover>(a, wx, s, lane, backIn(s), backOut(s), abort, g.spinLimit, x, nullptr);
         }
-        a.ring = reinterpret_cast<float *>(rf);
         x.rowMax = maxF;
         x.rowCnt = rcF;
         for (int s = me; s < nS && ok; s += G) {
             stripe(s);
-            ok = exactForward<kDiscover, false>(a, win, s, lane, foreIn(s), abort, g.spinLimit, &x, nullptr);
+            ok = exactForward<kDiscover, false>(a, wx, s, lane, foreIn(s), foreOut(s), abort, g.spinLimit, x, nullptr);
         }
         clusterSync(C);  // every row's maximum is written
         if (me == 0) exactScan<true>(maxB, rcB, x.cntB, p.M, lane);
@@ -449,17 +978,15 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
             alignW0 = g.alignCells + 2 * jb.cellOff;  // two floats per cell
             alignCnt = g.alignRows + jb.rowOff;
         }
-        a.ring = reinterpret_cast<float *>(rb);
         if (alignW0) a.alignOut = alignW0 + (size_t)(p.M + 1) * p.L;
         for (int s = sLast; s >= 0 && ok; s -= G) {
             stripe(s);
-            ok = exactBackward<kReplay>(a, win, s, lane, backIn(s), abort, g.spinLimit, &x, &filt);
+            ok = exactBackward<kReplay>(a, wx, s, lane, backIn(s), backOut(s), abort, g.spinLimit, x, &filt);
         }
-        a.ring = reinterpret_cast<float *>(rf);
         a.alignOut = alignW0;
         for (int s = me; s < nS && ok; s += G) {
             stripe(s);
-            ok = exactForward<kReplay, ANCH>(a, win, s, lane, foreIn(s), abort, g.spinLimit, &x, &mid);
+            ok = exactForward<kReplay, ANCH>(a, wx, s, lane, foreIn(s), foreOut(s), abort, g.spinLimit, x, &mid);
         }
         filt = warpBest(filt);
         mid = warpBest(mid);

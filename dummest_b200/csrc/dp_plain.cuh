@@ -2,7 +2,7 @@
 // baseline the batched persistent kernel is measured against.  The launch is
 // one CTA whose warps share the pair: its stripes (32 R profile rows each)
 // are dealt to the warps round-robin and run as a stripe pipeline with
-// the batched kernel's fast-path arithmetic (kMid or kFilter).  A pair of
+// the batched kernel's fast-path arithmetic.  A pair of
 // nS stripes keeps min(nS, 8) warps busy, so its time is that of the one
 // pair alone on the GPU, with none of the batching across pairs.  The
 // results are those of the batched kernel bit for bit; a pair whose wait
@@ -28,7 +28,7 @@
 
 namespace dmst {
 
-constexpr int kPipeWarps = 8;        // warps of the CTA
+constexpr int kPlainWarps = 8;       // warps of the CTA
 constexpr int kPipeExtra = 128;      // stripe period P' = P + kPipeExtra
 constexpr int kPipeSpinLimit = 1 << 24;  // default iterations of a wait (64 ns sleeps) before it gives up
 static_assert(kPipeExtra >= kLanes - 1 + 2 * kBlock, "a window never reaches the next stripe early");
@@ -36,7 +36,7 @@ static_assert(kPipeExtra >= kLanes - 1 + 2 * kBlock, "a window never reaches the
 __host__ __device__ inline int pipePeriod(int L) { return wavePeriod(L) + kPipeExtra; }
 
 struct PipeSync {
-    volatile int *progress;  // [kPipeWarps]: ring-writer position of each warp
+    volatile int *progress;  // [kPlainWarps]: ring-writer position of each warp
     volatile int *abort;     // the CTA's abort flag
     int W;                   // warps running stripes
     int spinLimit;           // iterations of a wait before it gives up (sets the abort flag)
@@ -103,30 +103,20 @@ __device__ __forceinline__ bool pipeReady(const PipeSync &ps, const SweepArgs &a
     return ok;
 }
 
-// The sweeps of one warp in a stripe pipeline.  The fast mode (kMid) also
-// gives the warp's share of the float maxima (filter best and largest Y in
-// the backward, mid and largest W0 / Y0 in the forward) through the optional
-// outputs; warps reduce them afterwards.
-template <int R, int MODE>
+// The sweeps of one warp in the stripe pipeline, with its share of the float
+// maxima (filter best and largest Y in the backward, mid and largest W0 / Y0
+// in the forward).
+template <int R, bool MID>
 __device__ bool backwardSweepPipe(const SweepArgs &a, Window &win, int warp, int lane, const PipeSync &ps,
-                                  const ExactRows *x, ExactBest *exact, float *filtOut = nullptr,
-                                  float *maxYOut = nullptr) {
-    BwdState<R, MODE> b;
+                                  float &filtOut, float &maxYOut) {
+    BwdState<R> b;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
 #pragma unroll
         for (int k = 0; k < R; ++k) b.h[q][k] = b.z[q][k] = 0.0f;
         b.rb[q] = 0.0f;
     }
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-        b.rmax[k] = 0.0f;
-        b.cOut[k] = 0;
-        b.fOut[k] = 1.0f;
-        b.rowBest[k] = 0.0;
-    }
     b.sendW = b.sendY = b.filt = b.maxY = 0.0f;
-    b.sendC = b.cnt = 0;
     b.u = -(kLanes - 1 - lane);  // lane 31 leads
     b.sp = a.sFirst;
     b.jj = 0;
@@ -134,82 +124,66 @@ __device__ bool backwardSweepPipe(const SweepArgs &a, Window &win, int warp, int
     const int total = a.nMine * a.P;
     const int T = (total + (kLanes - 1) + 2) / 3 * 3;
     if (!pipeReady(ps, a, -kBlock, 0, lane)) return false;
-    fillBlock<true, true>(win, a, 0, lane);
+    fillBlock<true>(win, a, 0, lane);
     for (int t0 = 0; t0 < T; t0 += kBlock) {
         pipePublish(ps, warp, pipePos(a, t0 - (kLanes - 1)), lane);
         if (!pipeReady(ps, a, t0, t0 + kBlock, lane)) return false;
-        fillBlock<true, true>(win, a, t0 + kBlock, lane);
+        fillBlock<true>(win, a, t0 + kBlock, lane);
         const int n = (t0 + kBlock < T ? kBlock : T - t0);
 #pragma unroll 1
         for (int g = 0; g < n; g += 3) {
-            backwardStep<R, MODE, 0, true>(b, a, win, lane, total, x, exact);
-            backwardStep<R, MODE, 1, true>(b, a, win, lane, total, x, exact);
-            backwardStep<R, MODE, 2, true>(b, a, win, lane, total, x, exact);
+            backwardStep<R, MID, 0>(b, a, win, lane, total);
+            backwardStep<R, MID, 1>(b, a, win, lane, total);
+            backwardStep<R, MID, 2>(b, a, win, lane, total);
         }
     }
     pipePublish(ps, warp, INT_MAX, lane);
-    if (filtOut) *filtOut = b.filt;
-    if (maxYOut) *maxYOut = b.maxY;
+    filtOut = b.filt;
+    maxYOut = b.maxY;
     return true;
 }
 
-template <int R, int MODE, bool ANCH = false>
+template <int R>
 __device__ bool forwardSweepPipe(const SweepArgs &a, Window &win, int warp, int lane, const PipeSync &ps,
-                                 const ExactRows *x, ExactBest *exact, float *bestOut = nullptr,
-                                 float *maxOut = nullptr) {
-    FwdState<R, MODE> f;
+                                 float &bestOut, float &maxOut) {
+    FwdState<R> f;
 #pragma unroll
     for (int h = 0; h < 3; ++h)
 #pragma unroll
         for (int k = 0; k < R; ++k) f.w[h][k] = f.z[h][k] = 0.0f;
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-        f.rmax[k] = 0.0f;
-        f.cIn[k] = f.cB[k] = 0;
-        f.fOut[k] = 1.0f;
-        f.rowBest[k] = 0.0;
-    }
     f.sendIn = f.sendY = f.best = f.mx = 0.0f;
-    f.sendC = f.cnt = 0;
-    f.sendAM = 0.0f;
-    f.sendAE = f.sendAR = 0;
     f.u = -lane;  // lane 0 leads
     f.s = a.sFirst;
     f.j = 0;
     const int total = a.nMine * a.P;
     const int T = (total + (kLanes - 1) + 5) / 6 * 6;
-    constexpr bool kReadW1 = MODE == kReplay || MODE == kMid;
-    W1Stage<R, true> st{-lane, a.sFirst, 0};
-    if (kReadW1) {
+    W1Stage<R> st{-lane, a.sFirst, 0};
 #pragma unroll
-        for (int k = 0; k < kW1Ahead; ++k) st.issue(a, win, k, lane, total);
-    }
+    for (int k = 0; k < kW1Ahead; ++k) st.issue(a, win, k, lane, total);
     bool ok = pipeReady(ps, a, -kBlock, 0, lane);
-    if (ok) fillBlock<false, true>(win, a, 0, lane);
+    if (ok) fillBlock<false>(win, a, 0, lane);
     for (int t0 = 0; ok && t0 < T; t0 += kBlock) {
         pipePublish(ps, warp, pipePos(a, t0 - (kLanes - 1)), lane);
         ok = pipeReady(ps, a, t0, t0 + kBlock, lane);
         if (!ok) break;
-        fillBlock<false, true>(win, a, t0 + kBlock, lane);
+        fillBlock<false>(win, a, t0 + kBlock, lane);
         const int n = (t0 + kBlock < T ? kBlock : T - t0);
 #pragma unroll 1
         for (int g = 0; g < n; g += 6) {
-            forwardStaged<R, MODE, 0, ANCH, true>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 1, ANCH, true>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 2, ANCH, true>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 3, ANCH, true>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 4, ANCH, true>(f, a, win, lane, total, st, x, exact);
-            forwardStaged<R, MODE, 5, ANCH, true>(f, a, win, lane, total, st, x, exact);
+            forwardStaged<R, 0>(f, a, win, lane, total, st);
+            forwardStaged<R, 1>(f, a, win, lane, total, st);
+            forwardStaged<R, 2>(f, a, win, lane, total, st);
+            forwardStaged<R, 3>(f, a, win, lane, total, st);
+            forwardStaged<R, 4>(f, a, win, lane, total, st);
+            forwardStaged<R, 5>(f, a, win, lane, total, st);
         }
     }
-    if (kReadW1) cpAsyncWait<0>();  // no copy outlives the sweep (the slots are reused)
+    cpAsyncWait<0>();  // no copy outlives the sweep (the slots are reused)
     if (ok) pipePublish(ps, warp, INT_MAX, lane);
-    if (bestOut) *bestOut = f.best;
-    if (maxOut) *maxOut = f.mx;
+    bestOut = f.best;
+    maxOut = f.mx;
     return ok;
 }
-
-constexpr int kPlainWarps = kPipeWarps;
 
 // Scratch of one pair (floats): W1 of every stripe (nS x D x 32 R) and the
 // 2W boundary rings of 4 P floats.
@@ -279,13 +253,13 @@ __global__ void __launch_bounds__(kPlainWarps * kLanes, 1)
     bool ok = true;
     if (lane == 0) progress[warp] = warp < W ? pipePos(a, -1) : INT_MAX;
     __syncthreads();
-    if (warp < W) ok = backwardSweepPipe<R, MID ? kMid : kFilter>(a, win, warp, lane, ps, nullptr, nullptr, &filt, &maxY);
+    if (warp < W) ok = backwardSweepPipe<R, MID>(a, win, warp, lane, ps, filt, maxY);
     __syncthreads();  // every stripe's W1 is stored; the rings are free
     ok = ok && abortFlag == 0;
     if (MID) {
         if (lane == 0) progress[warp] = warp < W ? pipePos(a, -1) : INT_MAX;
         __syncthreads();
-        if (warp < W && ok) ok = forwardSweepPipe<R, kMid>(a, win, warp, lane, ps, nullptr, nullptr, &mid, &maxFw);
+        if (warp < W && ok) ok = forwardSweepPipe<R>(a, win, warp, lane, ps, mid, maxFw);
         __syncthreads();
         ok = ok && abortFlag == 0;
     }

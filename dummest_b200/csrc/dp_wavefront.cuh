@@ -270,16 +270,8 @@ struct Window {
 __device__ __forceinline__ float4 ringLoad(const float *ring, int col) {
     return __ldcg(reinterpret_cast<const float4 *>(ring) + col);
 }
-// Each half in one 64-bit store: the exact path's readers (dp_exact_pipe.cuh)
-// see a half whole or not at all.
 __device__ __forceinline__ void ringStore(float *ring, int col, float w, float y) {
-    const unsigned long long v = ((unsigned long long)__float_as_uint(y) << 32) | __float_as_uint(w);
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(ring + 4 * (size_t)col), "l"(v) : "memory");
-}
-__device__ __forceinline__ void ringStore(float *ring, int col, float w, float y, int cnt) {
-    ringStore(ring, col, w, y);
-    const unsigned long long v = (unsigned)cnt;
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(ring + 4 * (size_t)col + 2), "l"(v) : "memory");
+    __stcg(reinterpret_cast<float2 *>(ring) + 2 * col, make_float2(w, y));
 }
 
 // max(a, b, c) in one instruction (the three-input max.f32 of sm_100).
@@ -306,19 +298,13 @@ __device__ __forceinline__ float stepFilt(float filt, const float (&wv)[R], floa
 }
 
 // The ring a stripe reads (written by the stripe before it in processing order).
-template <bool EXACT>
 __device__ __forceinline__ const float *ringOfPrev(const SweepArgs &a, int k) {
-    if (!EXACT) return a.ring;
     const int sp = a.sFirst + k * a.sStep;
     return a.ring + (size_t)((sp - 1) % a.ringSlots) * a.ringStride;
 }
-template <bool EXACT>
-__device__ __forceinline__ int stripeOf(const SweepArgs &a, int k) {
-    return EXACT ? a.sFirst + k * a.sStep : k;
-}
+__device__ __forceinline__ int stripeOf(const SweepArgs &a, int k) { return a.sFirst + k * a.sStep; }
 
 // Backward window entry for local time u (the column of u is L-1 - u mod P).
-template <bool EXACT>
 __device__ __forceinline__ void fillBackward(Window &w, const SweepArgs &a, int u) {
     const int e = u & (kWin - 1);
     float4 c = make_float4(__int_as_float(kPad * a.rowPad), 0.0f, 0.0f, 0.0f);
@@ -329,7 +315,7 @@ __device__ __forceinline__ void fillBackward(Window &w, const SweepArgs &a, int 
             const int j = a.L - 1 - jj;
             const int code = (j + 1 < a.L) ? (int)__ldg(a.codes() + j + 1) : kPad;
             c = make_float4(__int_as_float(code * a.rowPad), a.smBg()[code], __ldg(a.suf() + j), __ldg(a.pre() + j));
-            if (stripeOf<EXACT>(a, k) > 0) r = ringLoad(ringOfPrev<EXACT>(a, k), jj);
+            if (stripeOf(a, k) > 0) r = ringLoad(ringOfPrev(a, k), jj);
         }
     }
     w.col[e] = c;
@@ -337,7 +323,6 @@ __device__ __forceinline__ void fillBackward(Window &w, const SweepArgs &a, int 
 }
 
 // Forward window entry for local time u (the column of u is u mod P).
-template <bool EXACT>
 __device__ __forceinline__ void fillForward(Window &w, const SweepArgs &a, int u) {
     const int e = u & (kWin - 1);
     float4 c = make_float4(__int_as_float(kPad * a.rowPad), 0.0f, 0.0f, 0.0f);
@@ -347,7 +332,7 @@ __device__ __forceinline__ void fillForward(Window &w, const SweepArgs &a, int u
         if (j < a.L) {
             const int code = (j >= 2) ? (int)__ldg(a.codes() + j - 2) : kPad;
             c = make_float4(__int_as_float(code * a.rowPad), a.smBg()[code] * a.sc().sC, __ldg(a.pre() + j), 0.0f);
-            if (stripeOf<EXACT>(a, k) > 0) r = ringLoad(ringOfPrev<EXACT>(a, k), j);
+            if (stripeOf(a, k) > 0) r = ringLoad(ringOfPrev(a, k), j);
         }
     }
     w.col[e] = c;
@@ -355,14 +340,11 @@ __device__ __forceinline__ void fillForward(Window &w, const SweepArgs &a, int u
 }
 
 // ---------------------------------------------------------------------------
-// Sweep modes.
-//   kFilter    fast backward, no W1 kept: findSimilaritiesBackwardOnly
-//   kMid       fast backward keeping W1 / fast forward with the float mid
-//   kDiscover  exact path, pass 1: per-lane scale counts, row maxima
-//   kReplay    exact path, pass 2: the reference's counts, exact maxima
-// The fast modes compute with every rescale count at zero.
+// The exact path (dp_exact_pipe.cuh): sweep modes.
+//   kDiscover  pass 1: per-lane scale counts, row maxima
+//   kReplay    pass 2: the reference's counts, exact maxima
 // ---------------------------------------------------------------------------
-enum SweepMode { kFilter = 0, kMid = 1, kDiscover = 2, kReplay = 3 };
+enum SweepMode { kDiscover = 0, kReplay = 1 };
 
 constexpr float kBump = 0x1p100f;  // discovery: rescale a lane above this
 constexpr float kStep = 0x1p-64f;  // one rescale step, RESCALE_STEP (dummest-score.hh:87)
@@ -422,124 +404,55 @@ __device__ __forceinline__ bool xsLessMe(float am, int ae, float bm, int be) {
 // (5-PH)%3 column j+3, and the new value of column j replaces column j+3.  The
 // history then shifts by renaming, with no register copies.
 // ---------------------------------------------------------------------------
-template <int R, int MODE>
+template <int R>
 struct BwdState {
     Coef<R> c;
     float h[3][R], z[3][R];  // this lane's rows: W1 and Z history slots
     float rb[3];             // the row below (the next lane's top row): W1 history slots
     float sendW, sendY, filt, maxY;
-    int sendC;
     int u, sp, jj;           // lane-local time, stripe from the bottom, column from the right
     float *wp;               // W1 store pointer of the current step
-    // exact-path state
-    int cnt;                 // discovery: this lane's scale count
-    float rmax[R];           // discovery: per-row maxima at count cnt
-    int cOut[R];             // replay: count of each row after its decision
-    float fOut[R];           // replay: 1 or 2^-64, the row's own rescale
-    double rowBest[R];       // replay: per-row max of W1 * prefixSeed
 };
 
-// A lane takes up its rows of profile stripe s: coefficients, empty histories.
-template <int R, int MODE>
-__device__ __forceinline__ void backwardStart(BwdState<R, MODE> &b, const SweepArgs &a, int lane, int s,
-                                              const ExactRows *x) {
-    const int rowBase = s * kLanes * R + lane * R, lag = kLanes - 1 - lane;
-    loadBackwardCoef<R>(b.c, a, rowBase);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-#pragma unroll
-        for (int k = 0; k < R; ++k) b.h[q][k] = b.z[q][k] = 0.0f;
-        b.rb[q] = 0.0f;
-    }
-    b.wp = a.w1 + (((size_t)s * a.D + lag) * kLanes + lane) * R;
-    if (MODE == kDiscover) {
-        b.cnt = 0;
-#pragma unroll
-        for (int k = 0; k < R; ++k) b.rmax[k] = 0.0f;
-    }
-    if (MODE == kReplay) {
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const int i = rowBase + k;
-            const int ci = i <= a.M() ? i : a.M() + 1;
-            const int cIn = __ldcg(x->cntB + (ci + 1 <= a.M() + 1 ? ci + 1 : a.M() + 1));
-            b.cOut[k] = __ldcg(x->cntB + ci);
-            b.fOut[k] = stepsDown(b.cOut[k] - cIn);
-            b.c.rs[k] = seedCoef(i <= a.M(), cIn);
-            b.rowBest[k] = 0.0;
-        }
-    }
-}
-
-// PIPE: the sweep runs one of several warps' stripes of a pair (a stripe
-// pipeline: stripes sFirst, sFirst + sStep, ...; ring slot per stripe).
-// START: the lane takes up a stripe at its first column (false: the caller has
-// done so for the sweep's only stripe).
-template <int R, int MODE, int PH, bool PIPE = (MODE == kDiscover || MODE == kReplay), bool SH = false, bool START = true>
-__device__ __forceinline__ void backwardStep(BwdState<R, MODE> &b, const SweepArgs &a, Window &win, int lane,
-                                             int total, const ExactRows *x, ExactBest *exact) {
+template <int R, bool MID, int PH>
+__device__ __forceinline__ void backwardStep(BwdState<R> &b, const SweepArgs &a, Window &win, int lane, int total) {
     constexpr int S = kLanes * R;
-    constexpr bool kStore = MODE == kMid || MODE == kReplay;
-    constexpr bool kExactMode = MODE == kDiscover || MODE == kReplay;
     constexpr int I1 = (3 - PH) % 3, I2 = (4 - PH) % 3, I3 = (5 - PH) % 3;
     float inW = __shfl_down_sync(kFull, b.sendW, 1);
     float inY = __shfl_down_sync(kFull, b.sendY, 1);
-    int inC = 0;
-    if (MODE == kDiscover) inC = __shfl_down_sync(kFull, b.sendC, 1);
+    const int lag = kLanes - 1 - lane;
     if (b.u >= 0 && b.u < total && b.jj < a.L) {
         const int s = a.nS - 1 - b.sp;
         const int rowBase = s * S + lane * R;
-        if (START && b.jj == 0) backwardStart<R, MODE>(b, a, lane, s, x);
+        if (b.jj == 0) {
+            loadBackwardCoef<R>(b.c, a, rowBase);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+#pragma unroll
+                for (int k = 0; k < R; ++k) b.h[q][k] = b.z[q][k] = 0.0f;
+                b.rb[q] = 0.0f;
+            }
+            b.wp = a.w1 + (((size_t)s * a.D + lag) * kLanes + lane) * R;
+        }
         const int slot = b.u & (kWin - 1);
         const float4 col = win.col[slot];
         if (lane == kLanes - 1) {
             const float4 r = win.ring[slot];
             inW = r.x;
             inY = r.y;
-            if (MODE == kDiscover) inC = __float_as_int(r.z);
-        }
-        if (MODE == kDiscover) {
-            // Align the incoming values and this lane to one scale.
-            if (inC > b.cnt) {
-                const float f = stepsDown(inC - b.cnt);
-#pragma unroll
-                for (int k = 0; k < R; ++k) {
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        b.h[q][k] *= f;
-                        b.z[q][k] *= f;
-                    }
-                    b.rmax[k] *= f;
-                    b.c.rs[k] = seedCoef(rowBase + k <= a.M(), inC);
-                }
-#pragma unroll
-                for (int q = 0; q < 3; ++q) b.rb[q] *= f;
-                b.cnt = inC;
-            } else if (inC < b.cnt) {
-                const float f = stepsDown(b.cnt - inC);
-                inW *= f;
-                inY *= f;
-            }
         }
         const int eOff = __float_as_int(col.x);  // code * rowPad
         const float bgv = col.y, sufv = col.z, prev = col.w;
         float e[R];
-        if (SH)  // the table in shared memory: a plain shared load
-            loadEmitS<R>(e, (unsigned)__cvta_generic_to_shared(a.smE) + 4u * (unsigned)(eOff + rowBase));
-        else
-            loadEmit<R>(e, a.smE + eOff + rowBase);
+        loadEmit<R>(e, a.smE + eOff + rowBase);
         // First products (W1[i+1][j+3] * e) * enter, taken before any row of
         // this step overwrites its column-j+3 slot.
         float p[R];
         p[R - 1] = (b.rb[I3] * e[R - 1]) * b.c.enter[R - 1];
 #pragma unroll
-        for (int k = 0; k < R - 1; ++k) {
-            const float h3 = (MODE == kReplay) ? b.h[I3][k + 1] * b.fOut[k + 1] : b.h[I3][k + 1];
-            p[k] = (h3 * e[k]) * b.c.enter[k];
-        }
+        for (int k = 0; k < R - 1; ++k) p[k] = (b.h[I3][k + 1] * e[k]) * b.c.enter[k];
         float bW1 = b.rb[I1], bW2 = b.rb[I2], bY = inY;
         float wv[R], yv[R];
-        float stepMax = 0.0f;
 #pragma unroll
         for (int k = R - 1; k >= 0; --k) {
             float acc = p[k];
@@ -550,113 +463,56 @@ __device__ __forceinline__ void backwardStep(BwdState<R, MODE> &b, const SweepAr
             acc = __fmaf_rn(zbg, b.c.a0[k], acc);
             acc = __fmaf_rn(b.h[I2][k], b.c.a2[k], acc);
             acc = __fmaf_rn(b.h[I1][k], b.c.a1[k], acc);
-            // Seed term fma(suf, rs, acc): in the fast modes rs is 1 on real
-            // rows, where the fma is the exact sum suf + acc (one rounding, as
-            // the reference's add), and 0 on rows past M, which accumulate
-            // exactly 0 and must stay 0.
+            // Seed term fma(suf, rs, acc): rs is 1 on real rows, where the fma
+            // is the exact sum suf + acc (one rounding, as the reference's
+            // add), and 0 on rows past M, which accumulate exactly 0 and must
+            // stay 0.
             const float W = __fmaf_rn(sufv, b.c.rs[k], acc);
             const float Y = __fmaf_rn(b.c.eps[k], bY, W);
             const float Z = __fmaf_rn(b.c.b0[k], zbg, W);
-            if (MODE == kFilter || MODE == kMid) yv[k] = Y;
-            if (MODE == kDiscover) {
-                b.rmax[k] = fmaxf(b.rmax[k], Y);  // Y >= W1 at every cell
-                stepMax = fmaxf(stepMax, Y);
-            }
-            if (MODE == kReplay) {
-                if (a.alignOut != nullptr && rowBase + k <= a.M())
-                    a.alignOut[(size_t)(rowBase + k) * a.L + (a.L - 1 - b.jj)] = W;
-                // What leaves the row is scaled by the row's own decision.
-                const float Wo = W * b.fOut[k];
-                b.rowBest[k] = fmax(b.rowBest[k], (double)Wo * (double)prev);
-                bW1 = b.h[I1][k] * b.fOut[k];
-                bW2 = b.h[I2][k] * b.fOut[k];
-                bY = Y * b.fOut[k];
-                wv[k] = Wo;
-            } else {
-                bW1 = b.h[I1][k];
-                bW2 = b.h[I2][k];
-                bY = Y;
-                wv[k] = W;
-            }
+            yv[k] = Y;
+            bW1 = b.h[I1][k];
+            bW2 = b.h[I2][k];
+            bY = Y;
+            wv[k] = W;
             b.h[I3][k] = W;
             b.z[I3][k] = Z;
         }
-        if (MODE == kFilter || MODE == kMid) {
-            // running maxima, two rows per three-input max
+        // running maxima, two rows per three-input max
 #pragma unroll
-            for (int k = 0; k < R; k += 2) b.maxY = (k + 1 < R) ? fmax3(b.maxY, yv[k], yv[k + 1]) : fmaxf(b.maxY, yv[k]);
-            b.filt = stepFilt<R>(b.filt, wv, prev);
-        }
+        for (int k = 0; k < R; k += 2) b.maxY = (k + 1 < R) ? fmax3(b.maxY, yv[k], yv[k + 1]) : fmaxf(b.maxY, yv[k]);
+        b.filt = stepFilt<R>(b.filt, wv, prev);
         b.rb[I3] = inW;
         b.sendW = wv[0];
         b.sendY = bY;
-        if (MODE == kDiscover) {
-            if (stepMax > kBump) {
-#pragma unroll
-                for (int k = 0; k < R; ++k) {
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        b.h[q][k] *= kStep;
-                        b.z[q][k] *= kStep;
-                    }
-                    b.rmax[k] *= kStep;
-                    b.c.rs[k] = seedCoef(rowBase + k <= a.M(), b.cnt + 1);
-                }
-#pragma unroll
-                for (int q = 0; q < 3; ++q) b.rb[q] *= kStep;
-                b.sendW *= kStep;
-                b.sendY *= kStep;
-                ++b.cnt;
-            }
-            b.sendC = b.cnt;
-        }
-        if (kStore) {
+        if (MID) {
             storeW1<R>(b.wp, wv);
             b.wp += kLanes * R;
         }
-        if (lane == 0 && b.sp < a.nS - 1) {
-            float *rg = PIPE ? a.ring + (size_t)(b.sp % a.ringSlots) * a.ringStride : a.ring;
-            if (MODE == kDiscover)
-                ringStore(rg, b.jj, b.sendW, b.sendY, b.sendC);
-            else
-                ringStore(rg, b.jj, b.sendW, b.sendY);
-        }
-        if (b.jj == a.L - 1) {
-            // the last column of these rows
-#pragma unroll
-            for (int k = 0; k < R; ++k) {
-                const int i = rowBase + k;
-                if (i > a.M()) continue;
-                if (MODE == kDiscover) {
-                    x->rowMax[i] = b.rmax[k];
-                    x->rowCnt[i] = b.cnt;
-                }
-                if (MODE == kReplay) foldBest(*exact, b.rowBest[k], b.cOut[k]);
-            }
-        }
+        if (lane == 0 && b.sp < a.nS - 1)
+            ringStore(a.ring + (size_t)(b.sp % a.ringSlots) * a.ringStride, b.jj, b.sendW, b.sendY);
     } else {
         b.sendW = 0.0f;
         b.sendY = 0.0f;
-        b.sendC = 0;
     }
     if (b.u >= 0 && ++b.jj == a.P) {
         b.jj = 0;
-        b.sp += PIPE ? a.sStep : 1;
+        b.sp += a.sStep;
     }
     ++b.u;
 }
 
 // Window refills for a block of kBlock steps starting at t0: local times
 // [t0 + kBlock, t0 + 2 kBlock), one entry per lane and pass.
-template <bool BACKWARD, bool EXACT = false>
+template <bool BACKWARD>
 __device__ __forceinline__ void fillBlock(Window &win, const SweepArgs &a, int first, int lane) {
 #pragma unroll
     for (int o = 0; o < kBlock; o += kLanes) {
         if (o + lane < kBlock) {
             if (BACKWARD)
-                fillBackward<EXACT>(win, a, first + o + lane);
+                fillBackward(win, a, first + o + lane);
             else
-                fillForward<EXACT>(win, a, first + o + lane);
+                fillForward(win, a, first + o + lane);
         }
     }
 }
@@ -680,7 +536,7 @@ __device__ __forceinline__ void cpAsyncWait() {
 // W1 staging cursor of the forward sweep: the lane-local time whose W1 is
 // copied next (kW1Ahead steps ahead of the lane).  Every call commits one
 // group, empty for steps the lane does not compute.
-template <int R, bool EXACT = false>
+template <int R>
 struct W1Stage {
     int u, s, j;
     __device__ __forceinline__ void issue(const SweepArgs &a, Window &win, int slot, int lane, int total) {
@@ -691,129 +547,51 @@ struct W1Stage {
         cpAsyncCommit();
         if (u >= 0 && ++j == a.P) {
             j = 0;
-            s += EXACT ? a.sStep : 1;
+            s += a.sStep;
         }
         ++u;
     }
 };
 
-template <int R, int MODE>
+template <int R>
 struct FwdState {
     Coef<R> c;
     float w[3][R], z[3][R];  // W0 and Z0 history slots (rotating roles, see backwardStep)
     float sendIn, sendY, best, mx;
-    int sendC;
-    // anchors: the column's best wMid over the rows below and this lane's (mantissa, exponent, row)
-    float sendAM;
-    int sendAE, sendAR;
     int u, s, j;
-    // exact-path state (see BwdState)
-    int cnt;
-    float rmax[R];
-    int cIn[R], cB[R];
-    float fOut[R];
-    double rowBest[R];
 };
-
-template <int R, int MODE>
-__device__ __forceinline__ void forwardStart(FwdState<R, MODE> &f, const SweepArgs &a, int lane, int s,
-                                             const ExactRows *x) {
-    const int rowBase = s * kLanes * R + lane * R;
-    loadForwardCoef<R>(f.c, a, rowBase);
-#pragma unroll
-    for (int h = 0; h < 3; ++h)
-#pragma unroll
-        for (int k = 0; k < R; ++k) f.w[h][k] = f.z[h][k] = 0.0f;
-    if (MODE == kDiscover) {
-        f.cnt = 0;
-#pragma unroll
-        for (int k = 0; k < R; ++k) f.rmax[k] = 0.0f;
-    }
-    if (MODE == kReplay) {
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const int i = rowBase + k;
-            const int ci = i <= a.M() ? i : a.M();
-            f.cIn[k] = __ldcg(x->cntF + ci);
-            f.fOut[k] = stepsDown(__ldcg(x->cntF + ci + 1) - f.cIn[k]);
-            f.cB[k] = __ldcg(x->cntB + ci);
-            f.c.rs[k] = seedCoef(i <= a.M(), f.cIn[k]);
-            f.rowBest[k] = 0.0;
-        }
-    }
-}
 
 // One forward step of a lane (dummest-dp-forward.hh:112-223) at phase PH;
 // q holds the W1 values of this step.  Slot (3-PH)%3 holds column j-1,
 // (4-PH)%3 column j-2, (5-PH)%3 column j-3, which the new column j replaces.
-// ANCH (replay only): also the per-column anchors of the hit path
-// (dummest-dp-forward.hh:196-206): each column's best wMid over the rows and
-// its row passes up the lanes with the column, each lane folding its rows in
-// ascending order with scoreLess (the first row wins ties); the stripe's top
-// lane writes the stripe's partial, and the stripes are folded in order after
-// the sweep.
-template <int R, int MODE, int PH, bool ANCH = false, bool PIPE = (MODE == kDiscover || MODE == kReplay),
-          bool SH = false, bool START = true>
-__device__ __forceinline__ void forwardStep(FwdState<R, MODE> &f, const SweepArgs &a, Window &win, int lane,
-                                            int total, const float (&q)[R], const ExactRows *x, ExactBest *exact) {
+template <int R, int PH>
+__device__ __forceinline__ void forwardStep(FwdState<R> &f, const SweepArgs &a, Window &win, int lane, int total,
+                                            const float (&q)[R]) {
     constexpr int S = kLanes * R;
-    constexpr bool kExactMode = MODE == kDiscover || MODE == kReplay;
     constexpr int I1 = (3 - PH) % 3, I2 = (4 - PH) % 3, I3 = (5 - PH) % 3;
     float inW = __shfl_up_sync(kFull, f.sendIn, 1);
     float inY = __shfl_up_sync(kFull, f.sendY, 1);
-    float aM = 0.0f;
-    int aE = 0, aR = 0;
-    if (ANCH) {
-        aM = __shfl_up_sync(kFull, f.sendAM, 1);
-        aE = __shfl_up_sync(kFull, f.sendAE, 1);
-        aR = __shfl_up_sync(kFull, f.sendAR, 1);
-        if (lane == 0) {  // the rows below are the previous stripe's: a partial of this stripe
-            aM = 0.0f;
-            aE = aR = 0;
-        }
-    }
-    int inC = 0;
-    if (MODE == kDiscover) inC = __shfl_up_sync(kFull, f.sendC, 1);
     if (f.u >= 0 && f.u < total && f.j < a.L) {
         const int rowBase = f.s * S + lane * R;
-        if (START && f.j == 0) forwardStart<R, MODE>(f, a, lane, f.s, x);
+        if (f.j == 0) {
+            loadForwardCoef<R>(f.c, a, rowBase);
+#pragma unroll
+            for (int h = 0; h < 3; ++h)
+#pragma unroll
+                for (int k = 0; k < R; ++k) f.w[h][k] = f.z[h][k] = 0.0f;
+        }
         const int slot = f.u & (kWin - 1);
         const float4 col = win.col[slot];
         if (lane == 0) {
             const float4 r = win.ring[slot];
             inW = r.x;
             inY = r.y;
-            if (MODE == kDiscover) inC = __float_as_int(r.z);
-        }
-        if (MODE == kDiscover) {
-            if (inC > f.cnt) {
-                const float g = stepsDown(inC - f.cnt);
-#pragma unroll
-                for (int k = 0; k < R; ++k) {
-#pragma unroll
-                    for (int h = 0; h < 3; ++h) {
-                        f.w[h][k] *= g;
-                        f.z[h][k] *= g;
-                    }
-                    f.rmax[k] *= g;
-                    f.c.rs[k] = seedCoef(rowBase + k <= a.M(), inC);
-                }
-                f.cnt = inC;
-            } else if (inC < f.cnt) {
-                const float g = stepsDown(f.cnt - inC);
-                inW *= g;
-                inY *= g;
-            }
         }
         const int eOff = __float_as_int(col.x);  // code * rowPad
         const float bgsC = col.y, prev = col.z;
         float e[R];
-        if (SH)  // the table in shared memory: a plain shared load
-            loadEmitS<R>(e, (unsigned)__cvta_generic_to_shared(a.smE) + 4u * (unsigned)(eOff + rowBase));
-        else
-            loadEmit<R>(e, a.smE + eOff + rowBase);
+        loadEmit<R>(e, a.smE + eOff + rowBase);
         float win0 = inW, yab = inY;
-        float stepMax = 0.0f;
         float bv[R];
 #pragma unroll
         for (int k = 0; k < R; ++k) {
@@ -825,117 +603,31 @@ __device__ __forceinline__ void forwardStep(FwdState<R, MODE> &f, const SweepArg
             const float X = (f.c.enter[k] * e[k]) * w3;
             const float Z0 = bgsC * __fmaf_rn(f.c.b0[k], f.z[I3][k], f.c.a0[k] * w3);
             const float zs = __fmaf_rn(f.c.a2[k], w2, __fmaf_rn(f.c.a1[k], w1, Z0));
-            // fma(prev, 1, x) is prev + x; in the fast mode every row takes the
-            // seed: padding rows (past M, zero coefficients) then hold only
-            // their seed, which reaches no real row and multiplies a zero W1.
-            const float W0 = (MODE == kMid) ? win0 + __fadd_rn(zs, prev) : win0 + __fmaf_rn(prev, f.c.rs[k], zs);
-            if (MODE == kMid) bv[k] = W0 * q[k];
-            if (MODE == kReplay) {
-                f.rowBest[k] = fmax(f.rowBest[k], (double)W0 * (double)q[k]);
-                if (a.alignOut != nullptr && rowBase + k <= a.M()) a.alignOut[(size_t)(rowBase + k) * a.L + f.j] = W0;
-            }
-            if (ANCH) {
-                // wMid = promote(W0) * promote(W1): the exact double product,
-                // its mantissa rounded to float (dummest-batch.hh:216-235)
-                const double v = (double)W0 * (double)q[k];
-                if (rowBase + k <= a.M() && v > 0.0) {
-                    // frexp of v from its bits: v, a product of two positive
-                    // normal floats, is a normal double
-                    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
-                    const int ev = (int)((u >> 52) & 0x7FFULL) - 1022;
-                    const double mv = __longlong_as_double((long long)((u & 0xFFFFFFFFFFFFFULL) | (1022ULL << 52)));
-                    const float cm = __double2float_rn(mv);
-                    const int ce = ev + kRescaleBits * (f.cIn[k] + f.cB[k]);
-                    if (xsLessMe(aM, aE, cm, ce)) {
-                        aM = cm;
-                        aE = ce;
-                        aR = rowBase + k;
-                    }
-                }
-            }
+            // every row takes the seed: padding rows (past M, zero
+            // coefficients) then hold only their seed, which reaches no real
+            // row and multiplies a zero W1
+            const float W0 = win0 + __fadd_rn(zs, prev);
+            bv[k] = W0 * q[k];
             const float Y0 = __fmaf_rn(f.c.eps[k], yab, f.c.d0[k] * W0);
-            if (MODE == kMid) f.mx = fmax3(f.mx, W0, Y0);
-            const float nin = __fmaf_rn(f.c.d2[k], w1, __fmaf_rn(f.c.d1[k], w2, X + Y0));
-            if (MODE == kDiscover) {
-                f.rmax[k] = fmaxf(f.rmax[k], fmaxf(W0, Y0));
-                stepMax = fmaxf(stepMax, fmaxf(fmaxf(W0, Y0), nin));
-            }
+            f.mx = fmax3(f.mx, W0, Y0);
             f.w[I3][k] = W0;
             f.z[I3][k] = Z0;
-            if (MODE == kReplay) {
-                win0 = nin * f.fOut[k];
-                yab = Y0 * f.fOut[k];
-            } else {
-                win0 = nin;
-                yab = Y0;
-            }
+            win0 = __fmaf_rn(f.c.d2[k], w1, __fmaf_rn(f.c.d1[k], w2, X + Y0));
+            yab = Y0;
         }
-        if (MODE == kMid) {
 #pragma unroll
-            for (int k = 0; k < R; k += 2) f.best = (k + 1 < R) ? fmax3(f.best, bv[k], bv[k + 1]) : fmaxf(f.best, bv[k]);
-        }
-        if (MODE == kDiscover) {
-            if (stepMax > kBump) {
-#pragma unroll
-                for (int k = 0; k < R; ++k) {
-#pragma unroll
-                    for (int h = 0; h < 3; ++h) {
-                        f.w[h][k] *= kStep;
-                        f.z[h][k] *= kStep;
-                    }
-                    f.rmax[k] *= kStep;
-                    f.c.rs[k] = seedCoef(rowBase + k <= a.M(), f.cnt + 1);
-                }
-                win0 *= kStep;
-                yab *= kStep;
-                ++f.cnt;
-            }
-            f.sendC = f.cnt;
-        }
+        for (int k = 0; k < R; k += 2) f.best = (k + 1 < R) ? fmax3(f.best, bv[k], bv[k + 1]) : fmaxf(f.best, bv[k]);
         f.sendIn = win0;
         f.sendY = yab;
-        if (ANCH) {
-            f.sendAM = aM;
-            f.sendAE = aE;
-            f.sendAR = aR;
-            if (lane == kLanes - 1) {
-                float *pp = x->anchorPart + ((size_t)f.s * a.L + f.j) * 3;
-                pp[0] = aM;
-                pp[1] = __int_as_float(aE);
-                pp[2] = __int_as_float(aR);
-            }
-        }
-        if (lane == kLanes - 1 && f.s < a.nS - 1) {
-            float *rg = PIPE ? a.ring + (size_t)(f.s % a.ringSlots) * a.ringStride : a.ring;
-            if (MODE == kDiscover)
-                ringStore(rg, f.j, f.sendIn, f.sendY, f.sendC);
-            else
-                ringStore(rg, f.j, f.sendIn, f.sendY);
-        }
-        if (f.j == a.L - 1) {
-#pragma unroll
-            for (int k = 0; k < R; ++k) {
-                const int i = rowBase + k;
-                if (i > a.M()) continue;
-                if (MODE == kDiscover) {
-                    x->rowMax[i] = f.rmax[k];
-                    x->rowCnt[i] = f.cnt;
-                }
-                if (MODE == kReplay) foldBest(*exact, f.rowBest[k], f.cIn[k] + f.cB[k]);
-            }
-        }
+        if (lane == kLanes - 1 && f.s < a.nS - 1)
+            ringStore(a.ring + (size_t)(f.s % a.ringSlots) * a.ringStride, f.j, f.sendIn, f.sendY);
     } else {
         f.sendIn = 0.0f;
         f.sendY = 0.0f;
-        f.sendC = 0;
-        if (ANCH) {
-            f.sendAM = 0.0f;
-            f.sendAE = f.sendAR = 0;
-        }
     }
     if (f.u >= 0 && ++f.j == a.P) {
         f.j = 0;
-        f.s += PIPE ? a.sStep : 1;
+        f.s += a.sStep;
     }
     ++f.u;
 }
@@ -943,28 +635,20 @@ __device__ __forceinline__ void forwardStep(FwdState<R, MODE> &f, const SweepArg
 // One forward step at position P6 of a six-step group: wait for this step's
 // W1 copy, read it from the staging ring, run the step, and stage the W1 of
 // the step kW1Ahead later into the slot this lane read one step ago.
-template <int R, int MODE, int P6, bool ANCH = false, bool PIPE = (MODE == kDiscover || MODE == kReplay),
-          bool SH = false, bool START = true>
-__device__ __forceinline__ void forwardStaged(FwdState<R, MODE> &f, const SweepArgs &a, Window &win, int lane,
-                                              int total, W1Stage<R, PIPE> &st,
-                                              const ExactRows *x, ExactBest *exact) {
-    constexpr bool kReadW1 = MODE == kMid || MODE == kReplay;
+template <int R, int P6>
+__device__ __forceinline__ void forwardStaged(FwdState<R> &f, const SweepArgs &a, Window &win, int lane, int total,
+                                              W1Stage<R> &st) {
     float q[R];
-    if (kReadW1) {
-        cpAsyncWait<kW1Ahead - 1>();
-        const float4 v = win.w1[P6][lane];
-        q[0] = v.x;
-        if constexpr (R > 1) q[1] = v.y;
-        if constexpr (R > 2) {
-            q[2] = v.z;
-            q[3] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < R; ++k) q[k] = 0.0f;
+    cpAsyncWait<kW1Ahead - 1>();
+    const float4 v = win.w1[P6][lane];
+    q[0] = v.x;
+    if constexpr (R > 1) q[1] = v.y;
+    if constexpr (R > 2) {
+        q[2] = v.z;
+        q[3] = v.w;
     }
-    forwardStep<R, MODE, P6 % 3, ANCH, PIPE, SH, START>(f, a, win, lane, total, q, x, exact);
-    if (kReadW1) st.issue(a, win, (P6 + kW1Ahead) % kW1Slots, lane, total);
+    forwardStep<R, P6 % 3>(f, a, win, lane, total, q);
+    st.issue(a, win, (P6 + kW1Ahead) % kW1Slots, lane, total);
 }
 
 __device__ __forceinline__ float warpMax(float v) {
