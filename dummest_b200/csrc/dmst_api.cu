@@ -699,7 +699,7 @@ struct dmst_ctx {
     // dmst_align: the traceback buffers (dp_traceback.cuh) and the last call's results
     DevBuf<AlignJob> dAlignJobs;
     DevBuf<int> dAlignJobOf, dAlignRows, dAlignCand;
-    DevBuf<float> dAlignCells, dAlignColR, dAlignColF;
+    DevBuf<float> dAlignSteps, dAlignCells, dAlignColR, dAlignColF;
     DevBuf<XS> dAlignX, dAlignSuf, dAlignWork, dAlignRev, dAlignFwd;
     DevBuf<WalkSpan> dAlignSpan;
     DevBuf<WalkItem> dAlignItems;
@@ -867,6 +867,7 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
     ctx->dAlignJobOf.release();
     ctx->dAlignRows.release();
     ctx->dAlignCand.release();
+    ctx->dAlignSteps.release();
     ctx->dAlignCells.release();
     ctx->dAlignColR.release();
     ctx->dAlignColF.release();
@@ -2087,7 +2088,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         }
         const size_t expected =
             forceExact ? n : std::min<size_t>(n, std::max<size_t>(1, ctx->lastFlagged < 0 ? n / 64 : (size_t)ctx->lastFlagged));
-        pipeSpread(ctx, expected, exactStripes(maxM), kExactMaxWarps, kExactMaxWarps, 1, exactW, exactC);
+        pipeSpread(ctx, expected, 2 * exactStripes(maxM), kExactMaxWarps, kExactMaxWarps, 1, exactW, exactC);
         if (!ctx->exactAttrSet) {
             for (auto k : {exactPipeKernel<false>, exactPipeKernel<true>, exactPipeKernel<true, true>})
                 CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2406,7 +2407,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                                ctx->dCodes.p, S.dSeeds.p, S.dScales.p, ctx->dExactPool.p, poolSlot, ctx->dExactRing.p,
                                exactRing, ctx->dExactAbort.p, S.dExOut.p, anchors ? S.dAnchorOff.p : nullptr,
                                S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p, align ? ctx->dAlignJobOf.p : nullptr,
-                               align ? ctx->dAlignJobs.p : nullptr, align ? ctx->dAlignCells.p : nullptr,
+                               align ? ctx->dAlignJobs.p : nullptr, align ? ctx->dAlignSteps.p : nullptr,
                                align ? ctx->dAlignRows.p : nullptr, ctx->waitLimit > 0 ? ctx->waitLimit : kRingSpin};
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t cfg = clusterLaunch(exactC, exactW, exactW * sizeof(WindowX), exactC * exactClusters, &at, tail);
@@ -2725,7 +2726,7 @@ int dmst_anchors(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_score *be
 // anchors on the host (from the spans), and the store pass for the kept ones.
 static size_t alignJobBytes(int M, int L) {
     const size_t cells = (size_t)(M + 1) * L;
-    return cells * (8 + 8 + 8) + (size_t)L * (4 + 4 + 8 * kFlankArrays + 8 + 8 + 4 + sizeof(WalkSpan) + 2 * sizeof(Seg)) +
+    return cells * (8 + 8 + 8) + 2 * (size_t)exactW1Floats(M, L) * 4 + (size_t)L * (4 + 4 + 8 * kFlankArrays + 8 + 8 + 4 + sizeof(WalkSpan) + 2 * sizeof(Seg)) +
            (size_t)alignRowInts(M) * 4 + 256;
 }
 
@@ -2792,7 +2793,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
 
     size_t freeB = 0, totalB = 0;
     CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
-    const size_t held = ctx->dAlignCells.cap * sizeof(float) + (ctx->dAlignX.cap + ctx->dAlignSuf.cap) * sizeof(XS);
+    const size_t held = (ctx->dAlignCells.cap + ctx->dAlignSteps.cap) * sizeof(float) + (ctx->dAlignX.cap + ctx->dAlignSuf.cap) * sizeof(XS);
     const size_t budget = std::max<size_t>((freeB + held) / 2, (size_t)256 << 20);
     NullRates nr;
     nr.single = (double)(ctx->rates.insert1 + ctx->rates.delete2);
@@ -2800,7 +2801,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
     for (size_t b0 = 0; b0 < hits.size();) {
         // the batch: hits b0 .. b1-1
         size_t b1 = b0, bytes = 0;
-        while (b1 < hits.size() && b1 - b0 < 65535) {
+        while (b1 < hits.size() && b1 - b0 < 32767) {
             const dmst_pair &pp = pairs[hits[b1]];
             const size_t jb = alignJobBytes(ctx->profiles[pp.profile].M, ctx->seqLen[pp.seq]);
             if (b1 > b0 && bytes + jb > budget) break;
@@ -2810,7 +2811,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         const int nb = (int)(b1 - b0);
         std::vector<AlignJob> jobs(nb);
         std::vector<dmst_pair> bp(nb);
-        long long cells = 0, cols = 0, rowsN = 0;
+        long long cells = 0, cols = 0, rowsN = 0, steps = 0;
         int maxL = 0, maxM = 0;
         for (int j = 0; j < nb; ++j) {
             const dmst_pair &pp = pairs[hits[b0 + j]];
@@ -2823,17 +2824,20 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
             jb.cellOff = cells;
             jb.colOff = cols;
             jb.rowOff = rowsN;
+            jb.stepOff = steps;
             jb.minM = gates[b0 + j].m;
             jb.minE = gates[b0 + j].e;
             cells += (long long)(jb.M + 1) * jb.L;
             cols += jb.L;
             rowsN += alignRowInts(jb.M);
+            steps += 2 * exactW1Floats(jb.M, jb.L);
             maxL = std::max(maxL, jb.L);
             maxM = std::max(maxM, jb.M);
         }
         // headroom: calls whose hits differ a little reuse the buffers (a
         // reallocation synchronises the device and costs a cudaMalloc of GBs)
         CK(ctx->dAlignCells.ensure((size_t)cells * 2, 0.3), "alloc traceback tables");
+        CK(ctx->dAlignSteps.ensure((size_t)steps, 0.3), "alloc traceback tables");
         CK(ctx->dAlignX.ensure((size_t)cells, 0.3), "alloc traceback tables");
         CK(ctx->dAlignSuf.ensure((size_t)cells, 0.3), "alloc traceback tables");
         CK(ctx->dAlignRows.ensure((size_t)rowsN, 0.3), "alloc traceback rows");
@@ -2857,6 +2861,8 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
             return st;
         }
         CallSlot &S = ctx->slot[si];
+        alignRowsKernel<<<dim3((maxL + kExactStripe + kTileSteps - 2) / kTileSteps, exactStripes(maxM), 2 * nb), 256, 0,
+                          ctx->stream>>>(ctx->dAlignJobs.p, ctx->dAlignSteps.p, ctx->dAlignCells.p);
         sidesKernel<<<dim3((maxL + 127) / 128, nb), 128, 0, ctx->stream>>>(
             ctx->dAlignJobs.p, ctx->dAlignCells.p, ctx->dAlignRows.p, ctx->dAlignColR.p, ctx->dAlignColF.p);
         flankPrepKernel<<<dim3((maxL + 4 + 127) / 128, nb), 128, 0, ctx->stream>>>(
@@ -2877,7 +2883,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         if ((st = completeCall(ctx))) return st;
         CK(cudaStreamSynchronize(ctx->stream), "traceback tables");
         tm[2] += msSince(tPhase);
-        tm[8] += ctx->lastLaunches + 7;  // the traceback call's, then sides, 4 flank, X and optimal kernels
+        tm[8] += ctx->lastLaunches + 8;  // the traceback call's, then rows, sides, 4 flank, X and optimal kernels
         tPhase = Clock::now();
 
         // The reference's sort of each hit's anchors (std::ranges::sort with

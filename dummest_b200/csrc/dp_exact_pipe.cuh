@@ -29,8 +29,9 @@
 // pass through one 16-byte ring entry per column and stripe, each half its own
 // flag (dp_pipe.cuh): kRingEmpty until written, emptied again by its reader,
 // which loads a block ahead.  Both discovery sweeps follow each other without
-// a barrier (neither reads the other's values), then the counts are scanned,
-// then both replay sweeps.  Every wait is for an earlier stripe of the same
+// a barrier (neither reads the other's values), or run side by side on twice
+// as many warps as stripes; then the counts are scanned, then both replay
+// sweeps.  Every wait is for an earlier stripe of the same
 // cluster and bounded: a wait that runs out sets the cluster's abort flag,
 // every warp leaves its sweep, and the pair and those after it on the cluster
 // are marked failed.
@@ -39,9 +40,10 @@
 // (dp_stagger.cuh: neither waits for the other), on as many warps as there are
 // stripes; steps inside the read run without masks, and the FP64 products are
 // formed only for cells that can raise a row's best (rowBestFold).  Measured:
-// three windows of 10 kb against M = 2000 in 9.0 ms (170 ns a step), 18.7 with
-// two rows at one column and every product, 47 with four rows per lane on the
-// 8 warps of one CTA; 55 pairs of M = 400 x 2.2 kb in 2.0, 4.0 and 8.5 ms.
+// three windows of 10 kb against M = 2000 in 8.3 ms (170 ns a step), 10.8 with
+// the discovery sweeps in turn, 18.7 with two rows at one column and every
+// product, 47 with four rows per lane on the 8 warps of one CTA; 55 pairs of M
+// = 400 x 2.2 kb in 1.8, 2.0, 4.0 and 8.5 ms.
 #pragma once
 
 #include "dp_exact.cuh"
@@ -95,13 +97,14 @@ struct ExactPipeArgs {
     const long long *anchorOff;
     float *anchorM;
     int *anchorE, *anchorRow;
-    // traceback jobs (jobOf[pair] >= 0): the replay sweeps' row-major W0 and W1
-    // before each row's rescale (at float offset 2 AlignJob::cellOff: W0 at
-    // [0, (M+1) L), W1 after it) and the reference's rescale counts
-    // (AlignJob::rowOff in alignRows: cntB at [0, M+2), cntF after it)
+    // traceback jobs (jobOf[pair] >= 0): the replay sweeps' W0 and then W1
+    // before each row's rescale, by stripe and step (at AlignJob::stepOff in
+    // alignSteps; alignRowsKernel makes them row-major) and the reference's
+    // rescale counts (AlignJob::rowOff in alignRows: cntB at [0, M+2), cntF
+    // after it)
     const int *jobOf;
     const AlignJob *jobs;
-    float *alignCells;
+    float *alignSteps;
     int *alignRows;
     int spinLimit;          // polls of a wait before it gives up
 };
@@ -197,6 +200,7 @@ struct RunX {
     const float2 *ring;
     const int *cnt;
     float *w1;
+    float *align;
     unsigned long long *out;
 };
 
@@ -217,7 +221,7 @@ struct BwdX {
     float fOut[2];
     int cOut[2];
     RowBest best[2];
-    float *align;  // row-major W1 of the lane's row 0 at column L - 1 - u, or null
+    float *align;  // this step's W1 before the rows' rescale (traceback), or null
 };
 
 // Scales the lane's state by f and takes the count cnt (discovery).
@@ -336,11 +340,7 @@ __device__ __forceinline__ void bwdStepX(BwdX<MODE> &b, const SweepArgs &a, Wind
         b.sendY = b.yPrev[0];
         b.sendC = b.cnt;
     } else {
-        if (b.align != nullptr) {
-#pragma unroll
-            for (int k = 0; k < R; ++k)
-                if (act[k] && row + k <= M) b.align[(ptrdiff_t)k * a.L - (b.u - (R - 1 - k))] = nW[k];
-        }
+        if (b.align != nullptr) storeW1S<R>(GEN ? b.align : ip.align + PH * SW, nW);
         // what leaves a row is scaled by the row's own decision
         float oW[R];
 #pragma unroll
@@ -361,11 +361,10 @@ __device__ __forceinline__ void bwdStepX(BwdX<MODE> &b, const SweepArgs &a, Wind
             ringPutX<kDisc>(ip.out + 2 * PH, b.sendW, b.sendY, b.cnt);
         }
     }
-    if (GEN) {
+    if (GEN) {  // otherwise the run advances them
         b.wp += SW;
+        if (!kDisc && b.align != nullptr) b.align += SW;
         ++b.u;
-    } else if (!kDisc && b.align != nullptr) {
-        ++b.u;  // otherwise the run advances it
     }
 }
 
@@ -405,7 +404,7 @@ __device__ bool exactBackward(const SweepArgs &a, WindowX &w, int s, int lane, u
     b.u = -(kLanes - 1 - lane) * R;
     b.wp = a.w1 + lane * R;
     b.eS = (unsigned)__cvta_generic_to_shared(a.smE + lane * R);
-    b.align = !kDisc && a.alignOut ? a.alignOut + (size_t)row * a.L + (a.L - 1) : nullptr;
+    b.align = !kDisc && a.alignOut ? a.alignOut + lane * R : nullptr;
     const int T = (a.L - 1 + S + 3) / 4 * 4;
     for (int v = -S + lane; v < 0; v += kLanes) fillStoreX<true, kDisc>(w, a, FillX{{kPad, 0.0f, 0.0f, 0ull}, 0ull}, nullptr, v, abort, 0);
     __syncwarp();
@@ -421,7 +420,7 @@ __device__ bool exactBackward(const SweepArgs &a, WindowX &w, int s, int lane, u
         int gA, gB;
         interiorRunS<4>(a, S, t0, n, gA, gB);
         int g = 0;
-        RunX ip{nullptr, nullptr, nullptr, nullptr, nullptr};
+        RunX ip{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
 #pragma unroll 1
         for (; g < gA; g += 4) {
             bwdStepX<MODE, 0, true>(b, a, w, lane, row, M, out, ip);
@@ -430,11 +429,11 @@ __device__ bool exactBackward(const SweepArgs &a, WindowX &w, int s, int lane, u
             bwdStepX<MODE, 3, true>(b, a, w, lane, row, M, out, ip);
         }
         if (gB > gA) {
-            const int u0 = b.u;
             ip.col = w.s.col + (b.u & (kSWin - 1));
             ip.ring = w.s.ring + (b.u & (kSRingWin - 1));
             ip.cnt = w.cnt + (b.u & (kSRingWin - 1));
             ip.w1 = b.wp;
+            ip.align = b.align;
             ip.out = out + 2 * (ptrdiff_t)(b.u - (R - 1));
 #pragma unroll 1
             for (; g < gB; g += 4) {
@@ -446,10 +445,12 @@ __device__ bool exactBackward(const SweepArgs &a, WindowX &w, int s, int lane, u
                 ip.ring += 4;
                 ip.cnt += 4;
                 ip.w1 += 4 * SW;
+                ip.align += 4 * SW;
                 ip.out += 8;
             }
-            b.u = u0 + (gB - gA);
+            b.u += gB - gA;
             b.wp += (gB - gA) * SW;
+            if (b.align != nullptr) b.align += (gB - gA) * SW;
         }
 #pragma unroll 1
         for (; g < n; g += 4) {
@@ -496,7 +497,7 @@ struct FwdX {
     int cSum[2];  // the row's forward count (before the row) plus its backward count
     RowBest best[2];
     Anchor an[2];  // anchors: per row, the column's best up to it
-    float *align;  // row-major W0 of the lane's row 0 at column u, or null
+    float *align;  // this step's W0 (traceback), or null
 };
 
 __device__ __forceinline__ void fwdRescaleX(FwdX<kDiscover> &f, float g, int cnt, int row, int M) {
@@ -617,11 +618,7 @@ __device__ __forceinline__ void fwdStepX(FwdX<MODE> &f, const SweepArgs &a, Wind
         }
 #pragma unroll
         for (int k = 0; k < R; ++k) rowBestFold(f.best[k], nW[k], q[k]);
-        if (f.align != nullptr) {
-#pragma unroll
-            for (int k = 0; k < R; ++k)
-                if (act[k] && row + k <= M) f.align[(ptrdiff_t)k * a.L + (f.u - k)] = nW[k];
-        }
+        if (f.align != nullptr) storeW1S<R>(GEN ? f.align : ip.align + PH * SW, nW);
     }
 #pragma unroll
     for (int k = 0; k < R; ++k) {
@@ -657,8 +654,9 @@ __device__ __forceinline__ void fwdStepX(FwdX<MODE> &f, const SweepArgs &a, Wind
     if (GEN) {
         f.w1src -= SW;
         --f.gAhead;
+        if (!kDisc && f.align != nullptr) f.align += SW;
         ++f.u;
-    } else if (!kDisc && (ANCH || f.align != nullptr)) {
+    } else if (ANCH) {
         ++f.u;  // otherwise the run advances it
     }
 }
@@ -698,7 +696,7 @@ __device__ bool exactForward(const SweepArgs &a, WindowX &w, int s, int lane, un
     f.cnt = f.sendC = 0;
     f.u = -lane * R;
     f.eS = (unsigned)__cvta_generic_to_shared(a.smE + lane * R);
-    f.align = !kDisc && a.alignOut ? a.alignOut + (size_t)row * a.L : nullptr;
+    f.align = !kDisc && a.alignOut ? a.alignOut + lane * R : nullptr;
     const int steps = a.L - 1 + S;
     const int T = (steps + kSW1Slots - 1) / kSW1Slots * kSW1Slots;
     f.w1src = a.w1 + (size_t)(steps - 1) * SW + lane * R;
@@ -726,8 +724,12 @@ __device__ bool exactForward(const SweepArgs &a, WindowX &w, int s, int lane, un
         int gA, gB;
         interiorRunS<8>(a, S, t0, n, gA, gB);
         int g = 0;
-        RunX ip{nullptr, nullptr, nullptr, nullptr, nullptr};
-        auto general = [&](int end) {
+        RunX ip{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+        // the general steps before the interior ones (or all of them), then the interior, then the general ones after
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+            const bool inner = part == 0 && gB > gA;
+            const int end = inner ? gA : n;
 #pragma unroll 1
             for (; g < end; g += 8) {
                 fwdStepX<MODE, 0, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
@@ -739,14 +741,13 @@ __device__ bool exactForward(const SweepArgs &a, WindowX &w, int s, int lane, un
                 fwdStepX<MODE, 6, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
                 fwdStepX<MODE, 7, true, ANCH>(f, a, w, s, lane, row, M, out, x.anchorPart, ip);
             }
-        };
-        if (gB > gA) {
-            general(gA);
+            if (!inner) break;
             const int u0 = f.u;
             ip.col = w.s.col + (f.u & (kSWin - 1));
             ip.ring = w.s.ring + (f.u & (kSRingWin - 1));
             ip.cnt = w.cnt + (f.u & (kSRingWin - 1));
             ip.w1 = const_cast<float *>(f.w1src);
+            ip.align = f.align;
             ip.out = out + 2 * (ptrdiff_t)(f.u - (R - 1));
 #pragma unroll 1
             for (; g < gB; g += 8) {
@@ -762,13 +763,14 @@ __device__ bool exactForward(const SweepArgs &a, WindowX &w, int s, int lane, un
                 ip.ring += 8;
                 ip.cnt += 8;
                 ip.w1 -= 8 * SW;
+                ip.align += 8 * SW;
                 ip.out += 16;
             }
             f.u = u0 + (gB - gA);
+            if (f.align != nullptr) f.align += (gB - gA) * SW;
             f.w1src -= (gB - gA) * SW;
             f.gAhead -= gB - gA;
         }
-        general(n);
     }
     if (!kDisc) cpAsyncWait<0>();  // no copy outlives the sweep (the slots are reused)
     if (!ok) return false;
@@ -880,6 +882,36 @@ __global__ void __launch_bounds__(1024) queueSortKernel(int *queue, const int *q
     for (int i = threadIdx.x; i < cnt; i += blockDim.x) queue[i] = (int)(0x7fffffffu - (unsigned)(key[i] & 0xffffffffULL));
 }
 
+// The traceback's row-major W0 and W1 (row i at i L) from the replay's steps: a
+// tile of 128 steps of one stripe through shared memory, read and written in
+// whole lines.  (The sweeps storing each cell in place made 64 four-byte
+// stores a step, each in its own line: 4.6 ms for 55 hits of M = 400 x 2.2 kb.)
+constexpr int kTileSteps = 128;
+__global__ void __launch_bounds__(256) alignRowsKernel(const AlignJob *jobs, const float *steps, float *cells) {
+    __shared__ float tile[kTileSteps][kExactStripe + 1];
+    const AlignJob jb = jobs[blockIdx.z >> 1];
+    const bool backward = (blockIdx.z & 1) != 0;
+    const int s = blockIdx.y, nS = exactStripes(jb.M), t0 = blockIdx.x * kTileSteps, T = jb.L - 1 + kExactStripe;
+    if (s >= nS || t0 >= T) return;
+    const long long stripeFloats = pipeStripeFloats(jb.L, kExactRows);
+    const float *src = steps + jb.stepOff + (backward ? nS + s : s) * stripeFloats + (size_t)t0 * kExactStripe;
+    const int n = min(kTileSteps, T - t0);
+    for (int q = threadIdx.x; q < n * kExactStripe; q += blockDim.x)
+        tile[q / kExactStripe][q % kExactStripe] = __ldcs(src + q);
+    __syncthreads();
+    float *out = cells + 2 * jb.cellOff + (backward ? (size_t)(jb.M + 1) * jb.L : 0);
+    for (int r = threadIdx.x >> 5; r < kExactStripe; r += blockDim.x >> 5) {
+        const int i = s * kExactStripe + r, owner = r / kExactRows, k = r % kExactRows;
+        if (i > jb.M) break;
+        // the row's first column is at this step
+        const int lag = backward ? (kLanes - 1 - owner) * kExactRows + (kExactRows - 1 - k) : r;
+        for (int t = threadIdx.x & 31; t < n; t += kLanes) {
+            const int u = t0 + t - lag;
+            if (u >= 0 && u < jb.L) out[(size_t)i * jb.L + (backward ? jb.L - 1 - u : u)] = tile[t][r];
+        }
+    }
+}
+
 template <bool ANCH, bool ALIGN = false>
 __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(ExactPipeArgs g) {
     extern __shared__ float4 smRaw[];
@@ -954,6 +986,8 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
         auto backOut = [&](int s) { return s > 0 ? rb + 2LL * s * p.L : nullptr; };
         auto foreIn = [&](int s) { return s > 0 ? rf + 2LL * (s - 1) * p.L : nullptr; };
         auto foreOut = [&](int s) { return s < nS - 1 ? rf + 2LL * s * p.L : nullptr; };
+        // With twice as many warps as stripes the discovery sweeps run side by side.
+        const bool twin = G >= 2 * nS;
         x.rowMax = maxB;
         x.rowCnt = rcB;
         for (int s = sLast; s >= 0 && ok; s -= G) {
@@ -962,7 +996,8 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
         }
         x.rowMax = maxF;
         x.rowCnt = rcF;
-        for (int s = me; s < nS && ok; s += G) {
+        for (int s = twin ? me - nS : me; s < nS && ok; s += G) {
+            if (s < 0) break;
             stripe(s);
             ok = exactForward<kDiscover, false>(a, wx, s, lane, foreIn(s), foreOut(s), abort, g.spinLimit, x, nullptr);
         }
@@ -975,17 +1010,17 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
         float *alignW0 = nullptr;
         if (ALIGN && g.jobOf[pi] >= 0) {
             const AlignJob &jb = g.jobs[g.jobOf[pi]];
-            alignW0 = g.alignCells + 2 * jb.cellOff;  // two floats per cell
+            alignW0 = g.alignSteps + jb.stepOff;
             alignCnt = g.alignRows + jb.rowOff;
         }
-        if (alignW0) a.alignOut = alignW0 + (size_t)(p.M + 1) * p.L;
         for (int s = sLast; s >= 0 && ok; s -= G) {
             stripe(s);
+            if (ALIGN && alignW0) a.alignOut = alignW0 + (nS + s) * stripeFloats;
             ok = exactBackward<kReplay>(a, wx, s, lane, backIn(s), backOut(s), abort, g.spinLimit, x, &filt);
         }
-        a.alignOut = alignW0;
         for (int s = me; s < nS && ok; s += G) {
             stripe(s);
+            if (ALIGN && alignW0) a.alignOut = alignW0 + s * stripeFloats;
             ok = exactForward<kReplay, ANCH>(a, wx, s, lane, foreIn(s), foreOut(s), abort, g.spinLimit, x, &mid);
         }
         filt = warpBest(filt);

@@ -1,8 +1,8 @@
 // One traceback job: a hit pair (its best mid score passed the pair's gate)
 // whose alignments are traced (dummest-dp-forward.hh:471-535).  The offsets
 // place the job's pieces in the traceback buffers:
-//   cells  (M+1) x L row-major cells: the replay's W0 and W1 (floats, written
-//          by the exact kernel), later the prefix-optimal table in the same
+//   steps  the replay's W0 and W1 as the exact kernel stores them;
+//   cells  (M+1) x L row-major cells: W0 and W1 (floats), later the prefix-optimal table in the same
 //          bytes; the X table and the suffix-optimal table (one ExpScore per
 //          cell) in their own arrays at the same cell offset;
 //   cols   L entries per column array: anchors, column masses, flank scores,
@@ -20,6 +20,7 @@ struct AlignJob {
     long long cellOff;   // cells
     long long colOff;    // columns
     long long rowOff;    // ints
+    long long stepOff;   // the replay's W0 and W1 by stripe and step (floats)
     float minM;          // the gate, normalizeScore(minProbRatio, 0)
     int minE;
 };
