@@ -2876,7 +2876,9 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         xTableKernel<<<dim3((maxL + 127) / 128, (maxM + 1 + kXRows - 1) / kXRows, nb), 128, 0, ctx->stream>>>(
             ctx->dAlignJobs.p, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p, ctx->dCodes.p, S.dScales.p,
             ctx->dAlignCells.p, ctx->dAlignRows.p, ctx->dAlignX.p);
-        optimalKernel<<<nb, kOptThreads, 0, ctx->stream>>>(ctx->dAlignJobs.p, ctx->dAlignCells.p, ctx->dAlignRows.p,
+        CK(cudaFuncSetAttribute(optimalKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOptSmem), "smem attribute");
+        const int optThreads = std::min(kOptThreads, (maxL + 32 * kOptPer - 1) / (32 * kOptPer) * 32);
+        optimalKernel<<<dim3(nb, 2), optThreads, kOptSmem, ctx->stream>>>(ctx->dAlignJobs.p, ctx->dAlignCells.p, ctx->dAlignRows.p,
                                                           ctx->dAlignX.p, ctx->dAlignRev.p, ctx->dAlignFwd.p,
                                                           ctx->dAlignSuf.p);
         CK(cudaGetLastError(), "traceback table kernels");

@@ -14,8 +14,8 @@
 //                   each row's largest exponent;
 //   optimalKernel   the prefix- and suffix-optimal tables in the row-scaled
 //                   float form of dummest-scalerow.hh: each row is a running
-//                   maximum (a block-wide max scan) of candidates read from
-//                   the row before;
+//                   maximum (a block-wide max scan) of candidates from the row
+//                   before;
 //   spanKernel      the forward and reverse walks of every candidate anchor
 //                   at once (they do not depend on which anchors are kept):
 //                   each walk's sequence span and match counts; the host
@@ -164,7 +164,10 @@ __global__ void flankPrepKernel(const AlignJob *jobs, const DevPair *pairs, cons
 }
 
 // The three recurrences, one per warp (thread 0 of warps 0, 1, 2), inputs
-// loaded kFlankAhead columns at a time ahead of the chain.
+// loaded kFlankAhead columns at a time ahead of the chain, which is what
+// bounds them: in the float score algebra (null_model.cuh, the same bits) a
+// column takes a fraction of the 2400 cycles that double products and sums
+// with their conversions took (0.69 ms for reads of 2.2 kb, 2.7 before).
 constexpr int kFlankAhead = 8;
 __global__ void flankChainKernel(const AlignJob *jobs, const PairScales *scales, NullRates nr, XS *work) {
     const int t = blockIdx.x;
@@ -174,30 +177,36 @@ __global__ void flankChainKernel(const AlignJob *jobs, const PairScales *scales,
     const int L = jb.L;
     const PairScales sc = scales[jb.pair];
     const FlankRates r = flankRates(nr);
-    const XS aS1 = splitNorm((double)sc.s1, 0), aS2 = splitNorm((double)sc.s2, 0), aSC = splitNorm((double)sc.sC, 0);
+    const XS zero{0.0f, kZeroExp};
+    auto rate = [&](double f) { return f > 0.0 ? splitNorm(f, 0) : zero; };  // a float value
+    const XS aS1 = tagZero(splitNorm((double)sc.s1, 0)), aS2 = tagZero(splitNorm((double)sc.s2, 0)),
+             aSC = tagZero(splitNorm((double)sc.sC, 0));
+    const XS sr = rate(r.sr), dr = rate(r.dr);
+    const double keep = r.keep > 0.0 ? r.keep : 0.0;
     const XS *__restrict__ bgx = flankArray(work, jb, t, kFBg);
+    auto one = [&](XS v) { return scalarMulF(scalarMulF(v, sr), aS1); };
+    auto two = [&](XS v) { return scalarMulF(scalarMulF(v, dr), aS2); };
+    auto three = [&](XS v, XS bg) { return scalarMulF(scaleD(scalarMulF(v, aSC), keep), bg); };
     if (w == 0) {
         // middle entry masses, backward: mid[j] = colR[j] + cover of j+1.. continued
         const XS *__restrict__ cR = flankArray(work, jb, t, kFColR);
         XS *__restrict__ mid = flankArray(work, jb, t, kFMid);
-        XS m1 = xsZero(), m2 = xsZero(), m3 = xsZero();  // mid[j+1], mid[j+2], mid[j+3]
+        XS m1 = zero, m2 = zero, m3 = zero;  // mid[j+1], mid[j+2], mid[j+3]
         for (int q = L; q < L + 4; ++q) mid[q] = xsZero();
         for (int hi = L - 1; hi >= 0; hi -= kFlankAhead) {
             XS vc[kFlankAhead], vb[kFlankAhead];
 #pragma unroll
             for (int u = 0; u < kFlankAhead; ++u) {
                 const int j = hi - u;
-                vc[u] = j >= 0 ? ldXS(cR + j) : xsZero();
-                vb[u] = j >= 0 ? ldXS(bgx + j + 1) : xsZero();
+                vc[u] = j >= 0 ? tagZero(ldXS(cR + j)) : zero;
+                vb[u] = j >= 0 ? tagZero(ldXS(bgx + j + 1)) : zero;
             }
 #pragma unroll
             for (int u = 0; u < kFlankAhead; ++u) {
                 const int j = hi - u;
                 if (j < 0) break;
-                XS c = scalarMul(scaleScore(m1, r.sr), aS1);
-                c = scalarAdd(c, scalarMul(scaleScore(m2, r.dr), aS2));
-                c = scalarAdd(c, scalarMul(scaleScore(scalarMul(m3, aSC), r.keep), vb[u]));
-                const XS m = scalarAdd(vc[u], c);
+                const XS c = scalarAddF(scalarAddF(one(m1), two(m2)), three(m3, vb[u]));
+                const XS m = scalarAddF(vc[u], c);
                 stXS(mid + j, m);
                 m3 = m2;
                 m2 = m1;
@@ -208,27 +217,23 @@ __global__ void flankChainKernel(const AlignJob *jobs, const PairScales *scales,
         // cover of [j, end): the empty rest at the end counts 1
         XS *__restrict__ rest = flankArray(work, jb, t, kFRest);
         const XS bS1 = scaleScore(aS1, 4.0), bS2 = scaleScore(aS2, 16.0);
+        // the pieces cut off by the end, two and one bases long
+        const XS cut2 = tagZero(scaleScore(bS1, r.dr * 0.25)), cut3a = tagZero(scaleScore(bS2, r.keep * 0.0625)),
+                 cut3b = tagZero(scaleScore(bS1, r.keep * 0.25));
         for (int q = L; q < L + 4; ++q) rest[q] = xsZero();
         rest[L] = pow2Score(0);
-        XS r1 = pow2Score(0), r2 = xsZero(), r3 = xsZero();  // rest[j+1], rest[j+2], rest[j+3]
+        XS r1 = pow2Score(0), r2 = zero, r3 = zero;  // rest[j+1], rest[j+2], rest[j+3]
         for (int hi = L - 1; hi >= 0; hi -= kFlankAhead) {
             XS vb[kFlankAhead];
 #pragma unroll
-            for (int u = 0; u < kFlankAhead; ++u) vb[u] = hi - u >= 0 ? ldXS(bgx + hi - u) : xsZero();
+            for (int u = 0; u < kFlankAhead; ++u) vb[u] = hi - u >= 0 ? tagZero(ldXS(bgx + hi - u)) : zero;
 #pragma unroll
             for (int u = 0; u < kFlankAhead; ++u) {
                 const int j = hi - u;
                 if (j < 0) break;
-                const XS one = scalarMul(scaleScore(r1, r.sr), aS1);
-                const XS two = (j + 1 <= L - 1) ? scalarMul(scaleScore(r2, r.dr), aS2) : scaleScore(bS1, r.dr * 0.25);
-                XS three;
-                if (j + 2 <= L - 1)
-                    three = scalarMul(scaleScore(scalarMul(r3, aSC), r.keep), vb[u]);
-                else if (j + 1 <= L - 1)
-                    three = scaleScore(bS2, r.keep * 0.0625);
-                else
-                    three = scaleScore(bS1, r.keep * 0.25);
-                const XS v = scalarAdd(one, scalarAdd(two, three));
+                const XS b2 = j + 1 <= L - 1 ? two(r2) : cut2;
+                const XS b3 = j + 2 <= L - 1 ? three(r3, vb[u]) : (j + 1 <= L - 1 ? cut3a : cut3b);
+                const XS v = scalarAddF(one(r1), scalarAddF(b2, b3));
                 stXS(rest + j, v);
                 r3 = r2;
                 r2 = r1;
@@ -239,23 +244,20 @@ __global__ void flankChainKernel(const AlignJob *jobs, const PairScales *scales,
         // arrival masses, forward: cover ending at j grown from the cut masses
         const XS *__restrict__ cF = flankArray(work, jb, t, kFColF);
         XS *__restrict__ fa = flankArray(work, jb, t, kFArrival);
-        XS f1 = xsZero(), f2 = xsZero(), f3 = xsZero();  // arrival at j-1, j-2, j-3
+        XS f1 = zero, f2 = zero, f3 = zero;  // arrival at j-1, j-2, j-3
         for (int lo = 0; lo < L; lo += kFlankAhead) {
             XS vc[kFlankAhead], vb[kFlankAhead];
 #pragma unroll
             for (int u = 0; u < kFlankAhead; ++u) {
                 const int j = lo + u;
-                vc[u] = j < L ? ldXS(cF + j) : xsZero();
-                vb[u] = (j < L && j >= 2) ? ldXS(bgx + j - 2) : xsZero();
+                vc[u] = j < L ? tagZero(ldXS(cF + j)) : zero;
+                vb[u] = (j < L && j >= 2) ? tagZero(ldXS(bgx + j - 2)) : zero;
             }
 #pragma unroll
             for (int u = 0; u < kFlankAhead; ++u) {
                 const int j = lo + u;
                 if (j >= L) break;
-                XS a = vc[u];
-                if (j >= 1) a = scalarAdd(a, scalarMul(scaleScore(f1, r.sr), aS1));
-                if (j >= 2) a = scalarAdd(a, scalarMul(scaleScore(f2, r.dr), aS2));
-                if (j >= 3) a = scalarAdd(a, scalarMul(scaleScore(scalarMul(f3, aSC), r.keep), vb[u]));
+                const XS a = scalarAddF(scalarAddF(scalarAddF(vc[u], one(f1)), two(f2)), three(f3, vb[u]));
                 stXS(fa + j, a);
                 f3 = f2;
                 f2 = f1;
@@ -313,18 +315,18 @@ __global__ void flankSumKernel(const AlignJob *jobs, const XS *work, int *rows, 
     const int L = jb.L;
     const XS *__restrict__ u = flankArray(const_cast<XS *>(work), jb, t, kFUnified);
     int *sideMax = rows + jb.rowOff + 3 * (jb.M + 2);
-    XS cum = xsZero();
+    XS cum{0.0f, kZeroExp};
     int mx = INT_MIN;
     if (w == 0) {
         XS *__restrict__ rev = revEv + jb.colOff;
         for (int lo = 0; lo < L; lo += kFlankAhead) {
             XS v[kFlankAhead];
 #pragma unroll
-            for (int q = 0; q < kFlankAhead; ++q) v[q] = lo + q < L ? ldXS(u + lo + q) : xsZero();
+            for (int q = 0; q < kFlankAhead; ++q) v[q] = lo + q < L ? tagZero(ldXS(u + lo + q)) : cum;
 #pragma unroll
             for (int q = 0; q < kFlankAhead; ++q) {
                 if (lo + q >= L) break;
-                cum = scalarAdd(cum, v[q]);
+                cum = scalarAddF(cum, v[q]);
                 stXS(rev + lo + q, cum);
                 if (cum.m != 0.0f && cum.e > mx) mx = cum.e;
             }
@@ -335,11 +337,11 @@ __global__ void flankSumKernel(const AlignJob *jobs, const XS *work, int *rows, 
         for (int hi = L - 1; hi >= 0; hi -= kFlankAhead) {
             XS v[kFlankAhead];
 #pragma unroll
-            for (int q = 0; q < kFlankAhead; ++q) v[q] = hi - q >= 0 ? ldXS(u + hi - q) : xsZero();
+            for (int q = 0; q < kFlankAhead; ++q) v[q] = hi - q >= 0 ? tagZero(ldXS(u + hi - q)) : cum;
 #pragma unroll
             for (int q = 0; q < kFlankAhead; ++q) {
                 if (hi - q < 0) break;
-                cum = scalarAdd(cum, v[q]);
+                cum = scalarAddF(cum, v[q]);
                 stXS(fwd + hi - q, cum);
                 if (cum.m != 0.0f && cum.e > mx) mx = cum.e;
             }
@@ -424,15 +426,11 @@ __device__ __forceinline__ float blockExclusiveMax(float v, float *sm, bool reve
     return before;
 }
 
-// Prefix- and suffix-optimal tables of one job per CTA
-// (dummest-dp-forward.hh:295-451).  The prefix table overwrites the job's W0
-// and W1 (no longer read); the suffix table has its own array.
-__global__ void __launch_bounds__(kOptThreads) optimalKernel(const AlignJob *jobs, float *cells, const int *rows,
-                                                             const XS *X, const XS *revEv, const XS *fwdEv,
-                                                             XS *suffix) {
-    __shared__ float sm[kOptThreads / 32];
+// The tables of a read of more than kOptThreads x kOptPer columns, whose rows
+// are scanned in chunks, each row read back from the table.
+__device__ void optimalChunks(const AlignJob &jb, bool suffixTable, float *cells, const int *rows, const XS *X,
+                              const XS *revEv, const XS *fwdEv, XS *suffix, float *sm) {
     __shared__ float carry;
-    const AlignJob jb = jobs[blockIdx.x];
     const int M = jb.M, L = jb.L;
     const int *rowMaxX = rows + jb.rowOff + 2 * (M + 2);
     const int revMax = rows[jb.rowOff + 3 * (M + 2)], fwdMax = rows[jb.rowOff + 3 * (M + 2) + 1];
@@ -444,7 +442,7 @@ __global__ void __launch_bounds__(kOptThreads) optimalKernel(const AlignJob *job
 
     // prefix-optimal: rows 0..M, each a running maximum left to right
     int runMax = INT_MIN;
-    for (int i = 0; i <= M; ++i) {
+    for (int i = 0; i <= M && !suffixTable; ++i) {
         runMax = max(runMax, rowMaxX[i]);
         const int E = max(runMax, revMax) + 1;
         if (threadIdx.x == 0) carry = 0.0f;
@@ -486,7 +484,7 @@ __global__ void __launch_bounds__(kOptThreads) optimalKernel(const AlignJob *job
     // suffix-optimal: rows M..0, each a running maximum right to left
     runMax = INT_MIN;
     const int nChunks = (L + chunk - 1) / chunk;
-    for (int i = M; i >= 0; --i) {
+    for (int i = M; i >= 0 && suffixTable; --i) {
         runMax = max(runMax, rowMaxX[i]);
         const int E = max(runMax, fwdMax) + 1;
         if (threadIdx.x == 0) carry = 0.0f;
@@ -526,6 +524,111 @@ __global__ void __launch_bounds__(kOptThreads) optimalKernel(const AlignJob *job
             if (threadIdx.x == 0) carry = fmaxf(after, run);
             __syncthreads();
         }
+    }
+}
+
+// Prefix- (blockIdx.y = 0) and suffix-optimal (1) table of a job
+// (dummest-dp-forward.hh:295-451), one CTA each: neither reads the other.  The
+// prefix table overwrites the job's W0 and W1 (no longer read); the suffix
+// table has its own array.
+//
+// Bound: the chain of M+1 rows, each a block-wide scan.  So a row stays in
+// shared memory for the next one (in a read's own direction, position p = j or
+// L-1-j), a thread's flank scores stay in registers, the next row's X values
+// are loaded a row ahead, and a row takes two barriers.  With both tables on
+// one CTA, rows read back through L2 and five barriers a row, 55 hits of M =
+// 400 x 2.2 kb took 3.75 ms; now 1.25.
+constexpr int kOptCols = kOptThreads * kOptPer;
+constexpr size_t kOptSmem = 2 * (size_t)(kOptCols + kOptCols / kOptPer) * sizeof(XS);
+__device__ __forceinline__ int optSlot(int p) { return p + p / kOptPer; }  // a thread's run starts in its own bank
+
+__global__ void __launch_bounds__(kOptThreads) optimalKernel(const AlignJob *jobs, float *cells, const int *rows,
+                                                             const XS *X, const XS *revEv, const XS *fwdEv,
+                                                             XS *suffix) {
+    extern __shared__ XS optRows[];
+    __shared__ float sm[2][kOptThreads / 32];
+    const AlignJob jb = jobs[blockIdx.x];
+    const bool back = blockIdx.y != 0;
+    const int M = jb.M, L = jb.L;
+    if (L > kOptCols) {
+        optimalChunks(jb, back, cells, rows, X, revEv, fwdEv, suffix, sm[0]);
+        return;
+    }
+    const int *rowMaxX = rows + jb.rowOff + 2 * (M + 2);
+    const int flankMax = rows[jb.rowOff + 3 * (M + 2) + (back ? 1 : 0)];
+    XS *table = back ? suffix + jb.cellOff : reinterpret_cast<XS *>(cells + 2 * jb.cellOff);
+    const XS *Xj = X + jb.cellOff;
+    const XS *flank = (back ? fwdEv : revEv) + jb.colOff;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int p0 = threadIdx.x * kOptPer;
+    auto colOf = [&](int p) { return back ? L - 1 - p : p; };
+    // X of the match that ends (prefix) or starts (suffix) at position p: column
+    // j, or j + 3 (0 past the read)
+    auto loadX = [&](int i, int p) {
+        const int j = back ? L - 1 - p + 3 : p;
+        return p < L && j < L ? ldXS(Xj + (size_t)i * L + j) : xsZero();
+    };
+    XS fl[kOptPer], xv[kOptPer];
+    const int first = back ? M : 0, step = back ? -1 : 1;
+#pragma unroll
+    for (int q = 0; q < kOptPer; ++q) {
+        fl[q] = p0 + q < L ? ldXS(flank + colOf(p0 + q)) : xsZero();
+        xv[q] = loadX(first, p0 + q);
+    }
+    int runMax = INT_MIN, rowMax = rowMaxX[first];
+    for (int r = 0; r <= M; ++r) {
+        const int i = first + step * r;
+        XS *cur = optRows + (r & 1) * (kOptCols + kOptCols / kOptPer);
+        const XS *prev = optRows + ((r & 1) ^ 1) * (kOptCols + kOptCols / kOptPer);
+        runMax = max(runMax, rowMax);
+        const int E = max(runMax, flankMax) + 1;
+        float run = 0.0f, v[kOptPer];
+#pragma unroll
+        for (int q = 0; q < kOptPer; ++q) {
+            const int p = p0 + q;
+            float cand = 0.0f;
+            if (p < L) {
+                const float comb = toRow(xv[q], E), rs = toRow(fl[q], E);
+                if (r == 0) {
+                    cand = back ? rs : fmaxf(comb, rs);
+                } else {
+                    const float up = toRow(prev[optSlot(p)], E);
+                    const float succ = p >= 3 ? toRow(prev[optSlot(p - 3)], E) : 0.0f;
+                    // suffix: no match runs past the read's end
+                    const float match = back && p < 3 ? 0.0f : __fadd_rn(comb, succ);
+                    cand = fmaxf(fmaxf(up, match), rs);
+                }
+            }
+            run = fmaxf(run, cand);
+            v[q] = run;
+        }
+        if (r < M) {
+#pragma unroll
+            for (int q = 0; q < kOptPer; ++q) xv[q] = loadX(i + step, p0 + q);
+            rowMax = rowMaxX[i + step];
+        }
+        // the largest candidate of the threads before this one
+        float incl = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl = fmaxf(incl, t);
+        }
+        if (lane == 31) sm[r & 1][warp] = incl;
+        __syncthreads();
+        float before = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < warp ? __float_as_uint(sm[r & 1][lane]) : 0u));
+        const float left = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane >= 1) before = fmaxf(before, left);
+#pragma unroll
+        for (int q = 0; q < kOptPer; ++q) {
+            const int p = p0 + q;
+            if (p < L) {
+                const XS o = fromRow(fmaxf(before, v[q]), E);
+                cur[optSlot(p)] = o;
+                stXS(table + (size_t)i * L + colOf(p), o);
+            }
+        }
+        __syncthreads();
     }
 }
 

@@ -151,6 +151,24 @@ __device__ __forceinline__ XS scaleD(XS a, double f) {
     return XS{nz ? m : 0.0f, nz ? a.e + (hi >> 20) - 1022 : kZeroExp};
 }
 
+// mulScores and addScores, the scalar forms (dummest-score.hh:169-188), which
+// renormalise a product or sum of exactly 1 (the batch forms keep it) and
+// return the larger operand unchanged past 60 binades.  Zeros carry kZeroExp.
+__device__ __forceinline__ XS scalarMulF(XS a, XS b) {
+    const float p = __fmul_rn(a.m, b.m), z = __fmul_rz(a.m, b.m);
+    const bool lt = z < 0.5f, one = z >= 1.0f;
+    return XS{lt ? p + p : (one ? 0.5f : p), a.e + b.e + (one ? 1 : 0) - (lt ? 1 : 0)};
+}
+__device__ __forceinline__ XS scalarAddF(XS a, XS b) {
+    const bool ag = a.e >= b.e;
+    const float mh = ag ? a.m : b.m, ml = ag ? b.m : a.m;
+    const int eh = max(a.e, b.e), d = eh - min(a.e, b.e);
+    const float inv = __int_as_float((127 - min(d, 60)) << 23);
+    const float s = __fmaf_rn(ml, inv, mh);
+    const bool far = d > 60, ge = !far && __fmaf_rz(ml, inv, mh) >= 1.0f;
+    return XS{far ? mh : (ge ? s * 0.5f : s), eh + (ge ? 1 : 0)};
+}
+
 struct NullRates {
     double single;      // BACKGROUND_FRAMESHIFT_RATE (a float value)
     double dbl;         // BACKGROUND_FRAMESHIFT_RATE_2 (a float value)
