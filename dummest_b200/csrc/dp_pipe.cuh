@@ -167,7 +167,8 @@ __device__ bool pipeBackward(const SweepArgs &a, WindowS<R> &win, int lane, unsi
     b.filt = filt;
     b.maxY = maxY;
     b.u = -(kLanes - 1 - lane) * R;
-    b.jj = b.sp = 0;
+    b.jj = b.u;
+    b.sp = 0;
     b.wp = a.w1 + lane * stagLaneStride(R);
     const int rowBase = (a.nS - 1) * S + lane * R;
     loadBackwardCoef<R>(b.c, a, rowBase);
@@ -185,43 +186,7 @@ __device__ bool pipeBackward(const SweepArgs &a, WindowS<R> &win, int lane, unsi
         const int n = min(kSBlock, T - t0);
         int gA, gB;
         interiorRunS<4>(a, S, t0, n, gA, gB);
-        const bool ringWriter = lane == 0 && a.nS > 1;
-        int g = 0;
-        RunPtrs ip{nullptr, nullptr, nullptr, nullptr};
-#pragma unroll 1
-        for (; g < gA; g += 4) {
-            bwdStepS<R, MID, 0, true, true, true>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 1, true, true, true>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 2, true, true, true>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 3, true, true, true>(b, a, win, lane, false, ip);
-        }
-        if (gB > gA) {
-            ip.col = win.col + (b.u & (kSWin - 1));
-            ip.ring = win.ring + (b.u & (kSRingWin - 1));
-            ip.w1 = b.wp;
-            ip.ringOut = reinterpret_cast<float2 *>(a.ring) + (b.jj - (R - 1));
-#pragma unroll 1
-            for (; g < gB; g += 4) {
-                bwdStepS<R, MID, 0, false, true, true>(b, a, win, lane, ringWriter, ip);
-                bwdStepS<R, MID, 1, false, true, true>(b, a, win, lane, ringWriter, ip);
-                bwdStepS<R, MID, 2, false, true, true>(b, a, win, lane, ringWriter, ip);
-                bwdStepS<R, MID, 3, false, true, true>(b, a, win, lane, ringWriter, ip);
-                ip.col += 4;
-                ip.ring += 4;
-                ip.w1 += 4 * SW;
-                ip.ringOut += 4;
-            }
-            b.u += gB - gA;
-            b.jj += gB - gA;
-            b.wp += (gB - gA) * SW;
-        }
-#pragma unroll 1
-        for (; g < n; g += 4) {
-            bwdStepS<R, MID, 0, true, true, true>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 1, true, true, true>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 2, true, true, true>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 3, true, true, true>(b, a, win, lane, false, ip);
-        }
+        bwdBlockS<R, MID, true, true>(b, a, win, lane, n, gA, gB, lane == 0 && a.nS > 1);
     }
     filt = b.filt;
     maxY = b.maxY;
@@ -248,7 +213,8 @@ __device__ bool pipeForward(const SweepArgs &a, WindowS<R> &win, int lane, unsig
     f.best = best;
     f.mx = mx;
     f.u = -lane * R;
-    f.jj = f.sp = 0;
+    f.jj = f.u;
+    f.sp = 0;
     loadForwardCoef<R>(f.c, a, lane * R);
     f.eS = (unsigned)__cvta_generic_to_shared(a.smE + lane * R);
     f.eG = nullptr;
@@ -277,56 +243,7 @@ __device__ bool pipeForward(const SweepArgs &a, WindowS<R> &win, int lane, unsig
         const int n = min(kSBlock, T - t0);
         int gA, gB;
         interiorRunS<8>(a, S, t0, n, gA, gB);
-        const bool ringWriter = lane == kLanes - 1 && a.nS > 1;
-        int g = 0;
-        RunPtrs ip{nullptr, nullptr, nullptr, nullptr};
-#pragma unroll 1
-        for (; g < gA; g += 8) {
-            fwdStepS<R, 0, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 1, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 2, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 3, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 4, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 5, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 6, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 7, true, true, true>(f, a, win, lane, false, ip);
-        }
-        if (gB > gA) {
-            ip.col = win.col + (f.u & (kSWin - 1));
-            ip.ring = win.ring + (f.u & (kSRingWin - 1));
-            ip.w1 = const_cast<float *>(f.w1src);
-            ip.ringOut = reinterpret_cast<float2 *>(a.ring) + (f.jj - (R - 1));
-#pragma unroll 1
-            for (; g < gB; g += 8) {
-                fwdStepS<R, 0, false, true, true>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 1, false, true, true>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 2, false, true, true>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 3, false, true, true>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 4, false, true, true>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 5, false, true, true>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 6, false, true, true>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 7, false, true, true>(f, a, win, lane, ringWriter, ip);
-                ip.col += 8;
-                ip.ring += 8;
-                ip.w1 -= 8 * SW;
-                ip.ringOut += 8;
-            }
-            f.u += gB - gA;
-            f.jj += gB - gA;
-            f.w1src -= (gB - gA) * SW;
-            f.gAhead -= gB - gA;
-        }
-#pragma unroll 1
-        for (; g < n; g += 8) {
-            fwdStepS<R, 0, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 1, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 2, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 3, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 4, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 5, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 6, true, true, true>(f, a, win, lane, false, ip);
-            fwdStepS<R, 7, true, true, true>(f, a, win, lane, false, ip);
-        }
+        fwdBlockS<R, true, true>(f, a, win, lane, n, gA, gB, lane == kLanes - 1 && a.nS > 1);
     }
     cpAsyncWait<0>();  // no copy outlives the sweep (the staging slots are reused)
     best = f.best;

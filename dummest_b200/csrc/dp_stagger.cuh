@@ -29,7 +29,13 @@
 // next stripe is zero, and a lane's other rows are idle while its leading row
 // takes the next stripe's coefficients.  Idle steps are handled by masks in
 // the general steps; the interior steps (every row of every lane inside one
-// stripe) run without them.
+// stripe) run without them.  A general step's masks are the leading row's from
+// the last steps (row k sees the same columns later), only the values that are
+// not 0 by themselves are masked (an idle column's operands are 0), and the
+// window and W1 addresses are those of an interior run (with masks for every
+// row and value, and addresses of its own, it took 1.6 interior steps; 64
+// profiles x 2000 reads of 150-3000: 74.1 -> 70.6 ms; 16 x 1000 reads of
+// 75-300: 2.30 -> 2.10 ms).
 //
 // W1 is stored by warp step: the backward's step t writes the lane's R values
 // (its rows, each at its own column) to group t of the warp's slot, and the
@@ -53,6 +59,7 @@ constexpr int kSWin = 256;      // column window entries (lane-local times), a p
 constexpr int kSRingWin = 128;  // ring window entries (read by the stripe's leading lane only)
 constexpr int kSW1Slots = 8;    // forward W1 staging slots (cp.async, one group per step)
 constexpr int kSW1Ahead = kSW1Slots - 1;
+constexpr int kSDone = -(1 << 30);  // column of a lane after its last stripe: outside every read
 
 // Period of a stripe: L + 3 (three idle steps per row and stripe), and at
 // least S + 2 kSBlock + 31, so that the ring value a stripe's lowest row
@@ -216,7 +223,8 @@ struct BwdS {
     float h[4][R], z[4][R], rb[4], yPrev[R];
     float bgH[4], sufH[4], preH[4], evH[4][R];
     float sendW, sendY, filt, maxY;
-    int u, jj, sp;
+    bool act[4];      // whether the leading row's column of the last steps was inside the read (general steps)
+    int u, jj, sp;    // local time at the block's start, column of the leading row, stripe
     float *wp;        // W1 group of the current step (this lane's R values)
     unsigned eS;      // emission rows of the lane: 32-bit shared address (table in shared memory)
     const float *eG;  // or the global address (tall profiles)
@@ -227,12 +235,12 @@ struct BwdS {
 // coefficients when its leading row starts a stripe.
 template <int R, bool MID, int PH, bool GEN, bool SH, bool PIPE = false>
 __device__ __forceinline__ void bwdStepS(BwdS<R> &b, const SweepArgs &a, WindowS<R> &win, int lane,
-                                         bool ringWriter, const RunPtrs &ip) {
+                                         bool ringLane, const RunPtrs &ip) {
     constexpr int S = kLanes * R;
     constexpr int SW = kLanes * stagLaneStride(R);  // floats per W1 group
     float inW = __shfl_down_sync(kFull, b.sendW, 1);
     float inY = __shfl_down_sync(kFull, b.sendY, 1);
-    if (GEN && !PIPE && b.u >= 0 && b.jj == 0 && b.sp < a.nS) {
+    if (GEN && !PIPE && b.jj == 0) {
         // the leading row starts a stripe; the lane's other rows are idle
         const int rowBase = (a.nS - 1 - b.sp) * S + lane * R;
         loadBackwardCoef<R>(b.c, a, rowBase);
@@ -241,9 +249,10 @@ __device__ __forceinline__ void bwdStepS(BwdS<R> &b, const SweepArgs &a, WindowS
         else
             b.eG = a.smE + rowBase;
     }
-    const float4 col = GEN ? win.col[b.u & (kSWin - 1)] : ip.col[PH];
+    const float4 col = ip.col[PH];
+    if (GEN) b.act[PH] = (unsigned)b.jj < (unsigned)a.L;
     if (lane == kLanes - 1) {
-        const float2 r = GEN ? win.ring[b.u & (kSRingWin - 1)] : ip.ring[PH];
+        const float2 r = ip.ring[PH];
         inW = r.x;
         inY = r.y;
     }
@@ -289,12 +298,10 @@ __device__ __forceinline__ void bwdStepS(BwdS<R> &b, const SweepArgs &a, WindowS
         // seed term: rs is 1 on real rows (the fma is the exact sum) and 0 on
         // padding rows, which stay 0
         float W = __fmaf_rn(sufv, b.c.rs[k], acc);
-        float Y = __fmaf_rn(b.c.eps[k], Yb, W);
+        if (GEN && !b.act[Q]) W = 0.0f;
+        const float Y = __fmaf_rn(b.c.eps[k], Yb, W);  // idle: Yb is the idle row below's 0
         float Z = __fmaf_rn(b.c.b0[k], zbg, W);
-        if (GEN) {
-            const bool act = b.u >= 0 && b.sp < a.nS && b.jj >= D && b.jj < a.L + D;
-            if (!act) W = Y = Z = 0.0f;
-        }
+        if (GEN && !b.act[Q]) Z = 0.0f;
         nW[k] = W;
         nY[k] = Y;
         nZ[k] = Z;
@@ -324,21 +331,56 @@ __device__ __forceinline__ void bwdStepS(BwdS<R> &b, const SweepArgs &a, WindowS
     }
     b.sendW = nW[0];
     b.sendY = nY[0];
+    if (MID) storeW1S<R>(ip.w1 + PH * SW, nW);
     // the stripe's lowest row (lane 0, row 0) hands its row to the next stripe
     if (GEN) {
-        if (MID) storeW1S<R>(b.wp, nW);
-        b.wp += SW;
-        if (lane == 0 && b.u >= 0 && b.sp < a.nS - 1 && b.jj >= R - 1 && b.jj < a.L + R - 1)
+        if (ringLane && b.sp < a.nS - 1 && b.act[(PH + 4 - (R - 1)) & 3])
             ringStoreS<PIPE>(reinterpret_cast<float2 *>(a.ring) + (b.jj - (R - 1)), nW[0], nY[0]);
-        if (b.u >= 0 && ++b.jj == a.P) {
+        if (++b.jj == a.P) {
             b.jj = 0;
-            ++b.sp;
+            if (++b.sp == a.nS) b.jj = kSDone;
         }
-        ++b.u;
-    } else {  // the run advances u, jj and the W1 pointer
-        if (MID) storeW1S<R>(ip.w1 + PH * SW, nW);
-        if (ringWriter) ringStoreS<PIPE>(ip.ringOut + PH, nW[0], nY[0]);
+    } else {  // the run advances jj
+        if (ringLane) ringStoreS<PIPE>(ip.ringOut + PH, nW[0], nY[0]);
     }
+}
+
+// Four steps from phase 0, and the addresses and column of the next ones.
+template <int R, bool MID, bool GEN, bool SH, bool PIPE = false>
+__device__ __forceinline__ void bwdGroupS(BwdS<R> &b, const SweepArgs &a, WindowS<R> &win, int lane, bool ringLane,
+                                          RunPtrs &ip) {
+    constexpr int SW = kLanes * stagLaneStride(R);
+    if (GEN) {
+#pragma unroll
+        for (int d = 1; d < 4; ++d) b.act[4 - d] = (unsigned)(b.jj - d) < (unsigned)a.L;
+    }
+    bwdStepS<R, MID, 0, GEN, SH, PIPE>(b, a, win, lane, ringLane, ip);
+    bwdStepS<R, MID, 1, GEN, SH, PIPE>(b, a, win, lane, ringLane, ip);
+    bwdStepS<R, MID, 2, GEN, SH, PIPE>(b, a, win, lane, ringLane, ip);
+    bwdStepS<R, MID, 3, GEN, SH, PIPE>(b, a, win, lane, ringLane, ip);
+    ip.col += 4;
+    ip.ring += 4;
+    ip.w1 += 4 * SW;
+    if (!GEN) ip.ringOut += 4;
+}
+
+// The n steps of a block, of which [gA, gB) are interior; ringRun: this lane
+// writes the ring there.
+template <int R, bool MID, bool SH, bool PIPE = false>
+__device__ __forceinline__ void bwdBlockS(BwdS<R> &b, const SweepArgs &a, WindowS<R> &win, int lane, int n, int gA,
+                                          int gB, bool ringRun) {
+    RunPtrs ip{win.col + (b.u & (kSWin - 1)), win.ring + (b.u & (kSRingWin - 1)), b.wp, nullptr};
+    int g = 0;
+#pragma unroll 1
+    for (; g < gA; g += 4) bwdGroupS<R, MID, true, SH, PIPE>(b, a, win, lane, lane == 0, ip);
+    ip.ringOut = reinterpret_cast<float2 *>(a.ring) + (b.jj - (R - 1));  // used by the ring's writer only
+    if (gB > gA) b.jj += gB - gA;
+#pragma unroll 1
+    for (; g < gB; g += 4) bwdGroupS<R, MID, false, SH, PIPE>(b, a, win, lane, ringRun, ip);
+#pragma unroll 1
+    for (; g < n; g += 4) bwdGroupS<R, MID, true, SH, PIPE>(b, a, win, lane, lane == 0, ip);
+    b.u += n;
+    b.wp = ip.w1;
 }
 
 template <int R, bool MID, bool SH>
@@ -360,7 +402,8 @@ __device__ void backwardSweepS(const SweepArgs &a, WindowS<R> &win, int lane, fl
     }
     b.sendW = b.sendY = b.filt = b.maxY = 0.0f;
     b.u = -(kLanes - 1 - lane) * R;  // lane 31's leading row leads
-    b.jj = b.sp = 0;
+    b.jj = b.u;
+    b.sp = 0;
     b.wp = a.w1 + lane * stagLaneStride(R);
     {
         const int rowBase = (a.nS - 1) * S + lane * R;  // in bounds before the lane's first stripe
@@ -378,43 +421,7 @@ __device__ void backwardSweepS(const SweepArgs &a, WindowS<R> &win, int lane, fl
         const int n = min(kSBlock, T - t0);
         int gA, gB;
         const int sp = interiorRunS<4>(a, S, t0, n, gA, gB);
-        const bool ringWriter = lane == 0 && sp >= 0 && sp < a.nS - 1;
-        int g = 0;
-        RunPtrs ip{nullptr, nullptr, nullptr, nullptr};
-#pragma unroll 1
-        for (; g < gA; g += 4) {
-            bwdStepS<R, MID, 0, true, SH>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 1, true, SH>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 2, true, SH>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 3, true, SH>(b, a, win, lane, false, ip);
-        }
-        if (gB > gA) {
-            ip.col = win.col + (b.u & (kSWin - 1));
-            ip.ring = win.ring + (b.u & (kSRingWin - 1));
-            ip.w1 = b.wp;
-            ip.ringOut = reinterpret_cast<float2 *>(a.ring) + (b.jj - (R - 1));  // used by lane 0 only
-#pragma unroll 1
-            for (; g < gB; g += 4) {
-                bwdStepS<R, MID, 0, false, SH>(b, a, win, lane, ringWriter, ip);
-                bwdStepS<R, MID, 1, false, SH>(b, a, win, lane, ringWriter, ip);
-                bwdStepS<R, MID, 2, false, SH>(b, a, win, lane, ringWriter, ip);
-                bwdStepS<R, MID, 3, false, SH>(b, a, win, lane, ringWriter, ip);
-                ip.col += 4;
-                ip.ring += 4;
-                ip.w1 += 4 * SW;
-                ip.ringOut += 4;
-            }
-            b.u += gB - gA;
-            b.jj += gB - gA;
-            b.wp += (gB - gA) * SW;
-        }
-#pragma unroll 1
-        for (; g < n; g += 4) {
-            bwdStepS<R, MID, 0, true, SH>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 1, true, SH>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 2, true, SH>(b, a, win, lane, false, ip);
-            bwdStepS<R, MID, 3, true, SH>(b, a, win, lane, false, ip);
-        }
+        bwdBlockS<R, MID, SH>(b, a, win, lane, n, gA, gB, lane == 0 && sp >= 0 && sp < a.nS - 1);
     }
     filtOut = b.filt;
     maxYOut = b.maxY;
@@ -432,6 +439,7 @@ struct FwdS {
     float w[4][R], z[4][R], ninPrev[R], yPrev[R];
     float bgH[4], preH[4], evH[4][R];
     float sendIn, sendY, best, mx;
+    bool act[4];
     int u, jj, sp;
     unsigned eS;
     const float *eG;
@@ -451,7 +459,7 @@ __device__ __forceinline__ void cpAsyncStage(float *dst, const float *src) {
 
 template <int R, int PH, bool GEN, bool SH, bool PIPE = false>
 __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS<R> &win, int lane,
-                                         bool ringWriter, const RunPtrs &ip) {
+                                         bool ringLane, const RunPtrs &ip) {
     constexpr int S = kLanes * R;
     constexpr int SW = kLanes * stagLaneStride(R);  // floats per W1 group
     constexpr int H = PH & 3;
@@ -478,7 +486,7 @@ __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS
     }
     float inW = __shfl_up_sync(kFull, f.sendIn, 1);
     float inY = __shfl_up_sync(kFull, f.sendY, 1);
-    if (GEN && !PIPE && f.u >= 0 && f.jj == 0 && f.sp < a.nS) {
+    if (GEN && !PIPE && f.jj == 0) {
         const int rowBase = f.sp * S + lane * R;
         loadForwardCoef<R>(f.c, a, rowBase);
         if (SH)
@@ -486,9 +494,10 @@ __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS
         else
             f.eG = a.smE + rowBase;
     }
-    const float4 col = GEN ? win.col[f.u & (kSWin - 1)] : ip.col[PH];
+    const float4 col = ip.col[PH];
+    if (GEN) f.act[H] = (unsigned)f.jj < (unsigned)a.L;
     if (lane == 0) {
-        const float2 r = GEN ? win.ring[f.u & (kSRingWin - 1)] : ip.ring[PH];
+        const float2 r = ip.ring[PH];
         inW = r.x;
         inY = r.y;
     }
@@ -516,13 +525,11 @@ __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS
         float Z0 = bgsC * __fmaf_rn(f.c.b0[k], z3, f.c.a0[k] * w3);
         const float zs = __fmaf_rn(f.c.a2[k], w2, __fmaf_rn(f.c.a1[k], w1, Z0));
         float W0 = win0 + __fadd_rn(zs, prev);
-        float b = W0 * q[k];
-        float Y0 = __fmaf_rn(f.c.eps[k], yab, f.c.d0[k] * W0);
+        if (GEN && !f.act[Q]) W0 = 0.0f;
+        const float b = W0 * q[k];
+        const float Y0 = __fmaf_rn(f.c.eps[k], yab, f.c.d0[k] * W0);  // idle: yab is the idle row above's 0
         float nin = __fmaf_rn(f.c.d2[k], w1, __fmaf_rn(f.c.d1[k], w2, X + Y0));
-        if (GEN) {
-            const bool act = f.u >= 0 && f.sp < a.nS && f.jj >= k && f.jj < a.L + k;
-            if (!act) W0 = Y0 = nin = Z0 = b = 0.0f;
-        }
+        if (GEN && !f.act[Q]) nin = Z0 = 0.0f;
         f.mx = fmax3(f.mx, W0, Y0);
         nW[k] = W0;
         nZ[k] = Z0;
@@ -552,22 +559,66 @@ __device__ __forceinline__ void fwdStepS(FwdS<R> &f, const SweepArgs &a, WindowS
     f.sendY = nY[R - 1];
     // the stage for the step kSW1Ahead later goes into the slot read one step ago
     if (GEN) {
-        if (lane == kLanes - 1 && f.u >= 0 && f.sp < a.nS - 1 && f.jj >= R - 1 && f.jj < a.L + R - 1)
+        if (ringLane && f.sp < a.nS - 1 && f.act[(H + 4 - (R - 1)) & 3])
             ringStoreS<PIPE>(reinterpret_cast<float2 *>(a.ring) + (f.jj - (R - 1)), nN[R - 1], nY[R - 1]);
-        if (f.gAhead >= 0) cpAsyncStage<R>(&win.w1[(PH + kSW1Ahead) % kSW1Slots][lane * stagLaneStride(R)], f.w1src);
+        if (f.gAhead >= PH)
+            cpAsyncStage<R>(&win.w1[(PH + kSW1Ahead) % kSW1Slots][lane * stagLaneStride(R)], ip.w1 - PH * SW);
         cpAsyncCommit();
-        f.w1src -= SW;
-        --f.gAhead;
-        if (f.u >= 0 && ++f.jj == a.P) {
+        if (++f.jj == a.P) {
             f.jj = 0;
-            ++f.sp;
+            if (++f.sp == a.nS) f.jj = kSDone;
         }
-        ++f.u;
-    } else {  // the run advances u, jj and the staging cursor
-        if (ringWriter) ringStoreS<PIPE>(ip.ringOut + PH, nN[R - 1], nY[R - 1]);
+    } else {  // the run advances jj
+        if (ringLane) ringStoreS<PIPE>(ip.ringOut + PH, nN[R - 1], nY[R - 1]);
         cpAsyncStage<R>(&win.w1[(PH + kSW1Ahead) % kSW1Slots][lane * stagLaneStride(R)], ip.w1 - PH * SW);
         cpAsyncCommit();
     }
+}
+
+// Eight steps from phase 0, and the addresses and column of the next ones.
+template <int R, bool GEN, bool SH, bool PIPE = false>
+__device__ __forceinline__ void fwdGroupS(FwdS<R> &f, const SweepArgs &a, WindowS<R> &win, int lane, bool ringLane,
+                                          RunPtrs &ip) {
+    constexpr int SW = kLanes * stagLaneStride(R);
+    if (GEN) {
+#pragma unroll
+        for (int d = 1; d < 4; ++d) f.act[4 - d] = (unsigned)(f.jj - d) < (unsigned)a.L;
+    }
+    fwdStepS<R, 0, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    fwdStepS<R, 1, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    fwdStepS<R, 2, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    fwdStepS<R, 3, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    fwdStepS<R, 4, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    fwdStepS<R, 5, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    fwdStepS<R, 6, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    fwdStepS<R, 7, GEN, SH, PIPE>(f, a, win, lane, ringLane, ip);
+    ip.col += 8;
+    ip.ring += 8;
+    ip.w1 -= 8 * SW;
+    if (GEN)
+        f.gAhead -= 8;
+    else
+        ip.ringOut += 8;
+}
+
+template <int R, bool SH, bool PIPE = false>
+__device__ __forceinline__ void fwdBlockS(FwdS<R> &f, const SweepArgs &a, WindowS<R> &win, int lane, int n, int gA,
+                                          int gB, bool ringRun) {
+    RunPtrs ip{win.col + (f.u & (kSWin - 1)), win.ring + (f.u & (kSRingWin - 1)), const_cast<float *>(f.w1src), nullptr};
+    int g = 0;
+#pragma unroll 1
+    for (; g < gA; g += 8) fwdGroupS<R, true, SH, PIPE>(f, a, win, lane, lane == kLanes - 1, ip);
+    ip.ringOut = reinterpret_cast<float2 *>(a.ring) + (f.jj - (R - 1));  // used by the ring's writer only
+    if (gB > gA) {
+        f.jj += gB - gA;
+        f.gAhead -= gB - gA;
+    }
+#pragma unroll 1
+    for (; g < gB; g += 8) fwdGroupS<R, false, SH, PIPE>(f, a, win, lane, ringRun, ip);
+#pragma unroll 1
+    for (; g < n; g += 8) fwdGroupS<R, true, SH, PIPE>(f, a, win, lane, lane == kLanes - 1, ip);
+    f.u += n;
+    f.w1src = ip.w1;
 }
 
 template <int R, bool SH>
@@ -589,7 +640,8 @@ __device__ void forwardSweepS(const SweepArgs &a, WindowS<R> &win, int lane, flo
     }
     f.sendIn = f.sendY = f.best = f.mx = 0.0f;
     f.u = -lane * R;  // lane 0's row 0 leads
-    f.jj = f.sp = 0;
+    f.jj = f.u;
+    f.sp = 0;
     {
         const int rowBase = lane * R;
         f.eS = SH ? (unsigned)__cvta_generic_to_shared(a.smE + rowBase) : 0u;
@@ -618,56 +670,7 @@ __device__ void forwardSweepS(const SweepArgs &a, WindowS<R> &win, int lane, flo
         const int n = min(kSBlock, T - t0);
         int gA, gB;
         const int sp = interiorRunS<8>(a, S, t0, n, gA, gB);
-        const bool ringWriter = lane == kLanes - 1 && sp >= 0 && sp < a.nS - 1;
-        int g = 0;
-        RunPtrs ip{nullptr, nullptr, nullptr, nullptr};
-#pragma unroll 1
-        for (; g < gA; g += 8) {
-            fwdStepS<R, 0, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 1, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 2, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 3, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 4, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 5, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 6, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 7, true, SH>(f, a, win, lane, false, ip);
-        }
-        if (gB > gA) {
-            ip.col = win.col + (f.u & (kSWin - 1));
-            ip.ring = win.ring + (f.u & (kSRingWin - 1));
-            ip.w1 = const_cast<float *>(f.w1src);
-            ip.ringOut = reinterpret_cast<float2 *>(a.ring) + (f.jj - (R - 1));  // used by lane 31 only
-#pragma unroll 1
-            for (; g < gB; g += 8) {
-                fwdStepS<R, 0, false, SH>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 1, false, SH>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 2, false, SH>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 3, false, SH>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 4, false, SH>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 5, false, SH>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 6, false, SH>(f, a, win, lane, ringWriter, ip);
-                fwdStepS<R, 7, false, SH>(f, a, win, lane, ringWriter, ip);
-                ip.col += 8;
-                ip.ring += 8;
-                ip.w1 -= 8 * SW;
-                ip.ringOut += 8;
-            }
-            f.u += gB - gA;
-            f.jj += gB - gA;
-            f.w1src -= (gB - gA) * SW;
-            f.gAhead -= gB - gA;
-        }
-#pragma unroll 1
-        for (; g < n; g += 8) {
-            fwdStepS<R, 0, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 1, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 2, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 3, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 4, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 5, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 6, true, SH>(f, a, win, lane, false, ip);
-            fwdStepS<R, 7, true, SH>(f, a, win, lane, false, ip);
-        }
+        fwdBlockS<R, SH>(f, a, win, lane, n, gA, gB, lane == kLanes - 1 && sp >= 0 && sp < a.nS - 1);
     }
     cpAsyncWait<0>();  // no copy outlives the sweep (the staging slots are reused)
     bestOut = f.best;

@@ -56,3 +56,22 @@ def test_cluster_shapes_agree(n):
             got.append(c.score_pairs([sids[k % 40] for k in range(n)], pid, F.MODE_MID))
     for a, b in zip(*got):
         assert (a.mid, a.filter, a.filter_f) == (b.mid, b.filter, b.filter_f)
+
+
+@pytest.mark.parametrize("R", [1, 2, 3, 4])
+def test_batched_stripe_transitions_equal_oracle(R):
+    """The batched schedule with R rows per lane, whose lanes run from stripe
+    to stripe: one to several stripes, reads shorter than a period, around a
+    lane's lag, and longer than a stripe's fill."""
+    S = 32 * R
+    for M in (S - 1, S, 2 * S - 1, 3 * S + 5):
+        p, reads = _case(M, [3, 4, 5, 31, 32, 33, S - 1, S, S + 3, S + 92, S + 93, S + 130, 3 * S + 101], M)
+        with d.Context(rows_per_lane=R) as ctx:
+            pid = ctx.add_profile(*p)
+            sids = ctx.add_dna(reads)
+            mid = ctx.score_pairs(sids, pid, d.MODE_MID)
+            flt = ctx.score_pairs(sids, pid, d.MODE_FILTER)
+        for r, m, f in zip(reads, mid, flt):
+            want_mid, want_flt, _ = port.score_pair(*p, d.decode_dna(r))
+            assert (m.mid.m, m.mid.e) == want_mid and (m.filter.m, m.filter.e) == want_flt, (M, len(r))
+            assert f.filter_f == port.filter_pair(*p, d.decode_dna(r)), (M, len(r))
