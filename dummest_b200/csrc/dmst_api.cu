@@ -3659,13 +3659,13 @@ namespace {
 
 // Layout of the static scratch: a 2 KiB header (the kernel's profile, pair,
 // job and offset records), then the interleaved prefix and suffix
-// temporaries, 2 x 32 x (L+1) ExpScores.  The header is 2 KiB although its records take 192
+// temporaries, nullTmpEntries(L) ExpScores.  The header is 2 KiB although its records take 192
 // bytes so that a background lookup with any 8-bit code (bg[0..255] starts
 // 24 bytes into the profile record) stays inside the array.
 constexpr size_t kNaHeaderBytes = 2048;
 constexpr size_t kNaTmpEntries = (size_t)nullTmpEntries(DMST_NOALLOC_MAX_LEN);
-constexpr size_t kNaScratchBytes = kNaHeaderBytes + kNaTmpEntries * sizeof(XS);  // 8,391,168 bytes
-static_assert(kNaScratchBytes == 8391168, "documented scratch size");
+constexpr size_t kNaScratchBytes = kNaHeaderBytes + kNaTmpEntries * sizeof(XS);  // 8,399,360 bytes
+static_assert(kNaScratchBytes == 8399360, "documented scratch size");
 
 static __device__ __align__(256) unsigned char gNullScratch[kNaScratchBytes];
 

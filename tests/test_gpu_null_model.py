@@ -54,3 +54,27 @@ def test_jobs_of_ragged_reads_score_as_the_oracle():
             for r, got in zip(reads, res):
                 mid, flt, _ = port.score_pair(*p, d.decode_dna(r))
                 assert (got.mid.m, got.mid.e) == mid and (got.filter.m, got.filter.e) == flt
+
+
+@pytest.mark.parametrize("rates", [{}, {"insert1": 1e-4, "insert2": 1e-6, "delete1": 1e-6, "delete2": 1e-4},
+                                   {"insert1": 1e-25, "insert2": 1e-25, "delete1": 1e-25, "delete2": 1e-25}])
+def test_scaled_passes_equal_oracle(rates):
+    """Reads around the scaled passes' groups of 16 columns, reads whose
+    composition drives the seeds past both ends of the float range, reads
+    without a codon for long, and rates too small for the scaled passes."""
+    values, params, bg = _profile(60, 8)
+    rng = np.random.default_rng(12)
+    order = np.argsort(bg[:20])
+    aa = {d.decode_dna(a + b + c)[0]: a + b + c for a in "ACGT" for b in "ACGT" for c in "ACGT"}
+    rare, common = (aa[int(order[k])] for k in (0, 19))
+    reads = [synth.random_dna(rng, L, 0.5) for L in (18, 19, 20, 34, 35, 36, 50, 51, 66, 67)]
+    reads += [rare * 800 + common * 800, common * 800 + rare * 800, common * 300 + rare * 600 + common * 300,
+              "TAATAGTGA" * 60 + common * 300, synth.random_dna(rng, 9000, 0.35)]
+    with d.Context(rates=rates) as ctx:
+        pid = ctx.add_profile(values, params, bg)
+        for sid, r in zip(ctx.add_dna(reads), reads):
+            pre, suf, scales = ctx.null_model(sid, pid, len(r))
+            want = port.null_model(bg, d.decode_dna(r), port.rates(**rates))
+            np.testing.assert_array_equal(pre, want[0], err_msg=f"prefix seeds, L={len(r)}")
+            np.testing.assert_array_equal(suf, want[1], err_msg=f"suffix seeds, L={len(r)}")
+            np.testing.assert_array_equal(scales, np.asarray(want[2])[:3], err_msg=f"scales, L={len(r)}")
