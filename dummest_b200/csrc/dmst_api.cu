@@ -698,7 +698,7 @@ struct dmst_ctx {
     DevBuf<ExactOut> dExactOut;
     // dmst_align: the traceback buffers (dp_traceback.cuh) and the last call's results
     DevBuf<AlignJob> dAlignJobs;
-    DevBuf<int> dAlignJobOf, dAlignRows, dAlignCand;
+    DevBuf<int> dAlignJobOf, dAlignRows;
     DevBuf<float> dAlignSteps, dAlignCells, dAlignColR, dAlignColF;
     DevBuf<XS> dAlignX, dAlignSuf, dAlignWork, dAlignRev, dAlignFwd;
     DevBuf<WalkSpan> dAlignSpan;
@@ -866,7 +866,6 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
     ctx->dAlignJobs.release();
     ctx->dAlignJobOf.release();
     ctx->dAlignRows.release();
-    ctx->dAlignCand.release();
     ctx->dAlignSteps.release();
     ctx->dAlignCells.release();
     ctx->dAlignColR.release();
@@ -2846,7 +2845,6 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         CK(ctx->dAlignWork.ensure((size_t)kFlankArrays * (cols + 4LL * nb), 0.3), "alloc traceback columns");
         CK(ctx->dAlignRev.ensure((size_t)cols, 0.3), "alloc traceback columns");
         CK(ctx->dAlignFwd.ensure((size_t)cols, 0.3), "alloc traceback columns");
-        CK(ctx->dAlignCand.ensure((size_t)cols, 0.3), "alloc traceback columns");
         CK(ctx->dAlignSpan.ensure((size_t)cols, 0.3), "alloc traceback columns");
 
         // the exact path with the traceback stores, then the tables
@@ -2881,9 +2879,11 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         optimalKernel<<<dim3(nb, 2), optThreads, kOptSmem, ctx->stream>>>(ctx->dAlignJobs.p, ctx->dAlignCells.p, ctx->dAlignRows.p,
                                                           ctx->dAlignX.p, ctx->dAlignRev.p, ctx->dAlignFwd.p,
                                                           ctx->dAlignSuf.p);
+        spanKernel<<<dim3((maxL + 127) / 128, nb), 128, 0, ctx->stream>>>(
+            ctx->dAlignJobs.p, S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p, ctx->dAlignCells.p, ctx->dAlignX.p,
+            ctx->dAlignSuf.p, ctx->dAlignRev.p, ctx->dAlignFwd.p, ctx->dAlignSpan.p);
         CK(cudaGetLastError(), "traceback table kernels");
         if ((st = completeCall(ctx))) return st;
-        CK(cudaStreamSynchronize(ctx->stream), "traceback tables");
         tm[2] += msSince(tPhase);
         tm[8] += ctx->lastLaunches + 8;  // the traceback call's, then rows, sides, 4 flank, X and optimal kernels
         tPhase = Clock::now();
@@ -2896,7 +2896,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         // passing entries alone, sorted, are the candidates in order unless two
         // of them are equal scores: then where the reference's sort puts the
         // tied ones depends on all L entries, and the full sort runs.  Hits are
-        // shared among host threads.
+        // shared among host threads; the table and span kernels run meanwhile.
         struct Entry {
             dmst_score pair;
             int col;
@@ -2944,18 +2944,6 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         }
         tm[3] += msSince(tPhase);
         tPhase = Clock::now();
-        int maxCand = 1;
-        for (const AlignJob &jb : jobs) maxCand = std::max(maxCand, jb.nCand);
-        CK(cudaMemcpyAsync(ctx->dAlignJobs.p, jobs.data(), nb * sizeof(AlignJob), cudaMemcpyHostToDevice,
-                           ctx->stream),
-           "upload traceback jobs");
-        CK(cudaMemcpyAsync(ctx->dAlignCand.p, cand.data(), (size_t)cols * sizeof(int), cudaMemcpyHostToDevice,
-                           ctx->stream),
-           "upload traceback candidates");
-        spanKernel<<<dim3((maxCand + 127) / 128, nb), 128, 0, ctx->stream>>>(
-            ctx->dAlignJobs.p, ctx->dAlignCand.p, S.dAnchorRow.p, ctx->dAlignCells.p, ctx->dAlignX.p,
-            ctx->dAlignSuf.p, ctx->dAlignRev.p, ctx->dAlignFwd.p, ctx->dAlignSpan.p);
-        CK(cudaGetLastError(), "traceback span kernel");
         std::vector<WalkSpan> spans((size_t)cols);
         CK(cudaMemcpyAsync(spans.data(), ctx->dAlignSpan.p, (size_t)cols * sizeof(WalkSpan), cudaMemcpyDeviceToHost,
                            ctx->stream),
@@ -2980,7 +2968,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
             for (int c = 0; c < jb.nCand; ++c) {
                 const int a2 = cand[jb.colOff + c];
                 if (mark[a2]) continue;
-                const WalkSpan &w = spans[jb.colOff + c];
+                const WalkSpan &w = spans[jb.colOff + a2];
                 const int beg = std::max(w.beg, 0), end = std::min(w.end, jb.L);
                 if (beg < end && marked[end] - marked[beg] > 0) continue;
                 if (beg < end) {
@@ -3010,7 +2998,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
             CK(cudaMemcpyAsync(ctx->dAlignItems.p, items.data(), items.size() * sizeof(WalkItem),
                                cudaMemcpyHostToDevice, ctx->stream),
                "upload traceback walks");
-            storeWalkKernel<<<(int)((items.size() + 127) / 128), 128, 0, ctx->stream>>>(
+            storeWalkKernel<<<(int)((items.size() + kStoreWarps - 1) / kStoreWarps), kStoreWarps * 32, 0, ctx->stream>>>(
                 ctx->dAlignJobs.p, ctx->dAlignItems.p, (int)items.size(), S.dAnchorRow.p, ctx->dAlignCells.p,
                 ctx->dAlignX.p, ctx->dAlignSuf.p, ctx->dAlignRev.p, ctx->dAlignFwd.p, ctx->dAlignSegOut.p);
             CK(cudaGetLastError(), "traceback store kernel");

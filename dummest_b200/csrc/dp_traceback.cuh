@@ -16,8 +16,8 @@
 //                   float form of dummest-scalerow.hh: each row is a running
 //                   maximum (a block-wide max scan) of candidates from the row
 //                   before;
-//   spanKernel      the forward and reverse walks of every candidate anchor
-//                   at once (they do not depend on which anchors are kept):
+//   spanKernel      the forward and reverse walks of every column whose anchor
+//                   passes the gate (they do not depend on which are kept):
 //                   each walk's sequence span and match counts; the host
 //                   then takes the anchors in the reference's sorted order,
 //                   skipping those inside or overlapping kept ones;
@@ -642,6 +642,12 @@ struct WalkSpan {
     int beg, end, nf, nr;
 };
 
+// Bound: the latency of a step's loads, from tables of GBs that neither cache
+// holds.  Most steps are matches, so each step prefetches the cells of the
+// step kWalkAhead matches on (every candidate of 55 hits of M = 400 x 2.2 kb:
+// 0.83 ms, 1.27 without, in the candidates' order).
+constexpr int kWalkAhead = 8;
+
 // One anchor's walks (dummest-traceback.hh:35-118): forward from (anchor1,
 // anchor2) over the suffix-optimal table, then backward from (anchor1 - 1,
 // anchor2) over the prefix-optimal table, with the reference's merging of
@@ -657,6 +663,15 @@ __device__ WalkSpan walkAnchor(const AlignJob &jb, int a1, int a2, const XS *pre
     const int M = jb.M, L = jb.L;
     auto S = [&](int i, int j) { return (i <= M && j < L) ? ldXS(suf + (size_t)i * L + j) : xsZero(); };
     auto P = [&](int i, int j) { return ldXS(pre + (size_t)i * L + j); };
+    auto ahead = [&](const XS *t, int i, int j) {
+        if (i >= 0 && i <= M && j >= 0 && j < L) asm volatile("prefetch.global.L2 [%0];" ::"l"(t + (size_t)i * L + j));
+    };
+    for (int q = 0; q < kWalkAhead; ++q) {
+        ahead(Xj, a1 + q, a2 + 3 * q + 3);
+        ahead(suf, a1 + q + 1, a2 + 3 * q + 3);
+        ahead(Xj, a1 - 1 - q, a2 - 3 * q);
+        ahead(pre, a1 - 2 - q, a2 - 3 * q - 3);
+    }
     Seg fFirst{0, 0, 0}, fLast{0, 0, 0}, rFirst{0, 0, 0}, rFront{0, 0, 0};
     int nf = 0, nr = 0;
     {
@@ -665,8 +680,10 @@ __device__ WalkSpan walkAnchor(const AlignJob &jb, int a1, int a2, const XS *pre
             XS best = xsZero();
             int bi = INT_MAX, bj = INT_MAX;
             bool emit = false;
+            ahead(Xj, i + kWalkAhead, pos + 3 * kWalkAhead + 3);
+            ahead(suf, i + kWalkAhead + 1, pos + 3 * kWalkAhead + 3);
             if (pos + 3 < L) {
-                const XS cd = scalarAdd(ldXS(Xj + (size_t)i * L + pos + 3), S(i + 1, pos + 3));
+                const XS cd = scalarAddF(tagZero(ldXS(Xj + (size_t)i * L + pos + 3)), tagZero(S(i + 1, pos + 3)));
                 if (scoreLess(best, cd)) { best = cd; bi = i + 1; bj = pos + 3; emit = true; }
             }
             XS cd = S(i + 1, pos);
@@ -703,9 +720,11 @@ __device__ WalkSpan walkAnchor(const AlignJob &jb, int a1, int a2, const XS *pre
             XS best = xsZero();
             int bi = -1, bj = -1;
             bool emit = false;
+            ahead(Xj, i - kWalkAhead, pos - 3 * kWalkAhead);
+            ahead(pre, i - kWalkAhead - 1, pos - 3 * kWalkAhead - 3);
             if (pos >= 3) {
                 const XS succ = i >= 1 ? P(i - 1, pos - 3) : xsZero();
-                const XS cd = scalarAdd(ldXS(Xj + (size_t)i * L + pos), succ);
+                const XS cd = scalarAddF(tagZero(ldXS(Xj + (size_t)i * L + pos)), tagZero(succ));
                 if (scoreLess(best, cd)) { best = cd; bi = i - 1; bj = pos - 3; emit = true; }
             }
             if (i >= 1) {
@@ -761,18 +780,23 @@ __device__ WalkSpan walkAnchor(const AlignJob &jb, int a1, int a2, const XS *pre
     return w;
 }
 
-// The span pass: every candidate of every job at once, one thread each
-// (grid.y = job); spans[colOff + c] for candidate c.
-__global__ void spanKernel(const AlignJob *jobs, const int *cand, const int *anchorRow, const float *cells,
-                           const XS *X, const XS *suffix, const XS *revEv, const XS *fwdEv, WalkSpan *spans) {
+// The span pass: one thread per column of every job (grid.y = job), for the
+// columns whose anchor passes the job's gate; a walk does not depend on the
+// candidates' order, so this runs while the host sorts them.  Neighbouring
+// columns walk neighbouring cells.  The row is checked as well: after a failed
+// exact kernel the anchors are not its own.
+__global__ void spanKernel(const AlignJob *jobs, const float *anchorM, const int *anchorE, const int *anchorRow,
+                           const float *cells, const XS *X, const XS *suffix, const XS *revEv, const XS *fwdEv,
+                           WalkSpan *spans) {
     const AlignJob jb = jobs[blockIdx.y];
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= jb.nCand) return;
-    const int a2 = cand[jb.colOff + c];
+    const int a2 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a2 >= jb.L) return;
+    const XS a{anchorM[jb.colOff + a2], anchorE[jb.colOff + a2]};
     const int a1 = anchorRow[jb.colOff + a2];
-    spans[jb.colOff + c] = walkAnchor<false>(jb, a1, a2, reinterpret_cast<const XS *>(cells + 2 * jb.cellOff),
-                                             X + jb.cellOff, suffix + jb.cellOff, revEv + jb.colOff,
-                                             fwdEv + jb.colOff, nullptr, 0);
+    if (a.m == 0.0f || scoreLess(a, XS{jb.minM, jb.minE}) || a1 < 0 || a1 > jb.M) return;
+    spans[jb.colOff + a2] = walkAnchor<false>(jb, a1, a2, reinterpret_cast<const XS *>(cells + 2 * jb.cellOff),
+                                              X + jb.cellOff, suffix + jb.cellOff, revEv + jb.colOff,
+                                              fwdEv + jb.colOff, nullptr, 0);
 }
 
 // An accepted candidate whose segments are written.
@@ -782,12 +806,15 @@ struct WalkItem {
 };
 
 // The store pass: the accepted candidates' walks again, segments written in
-// place (the walks are deterministic, so the counts are the span pass's).
+// place (the walks are deterministic, so the counts are the span pass's).  One
+// walk per warp: few are kept, and walks that share a warp take their branches
+// in turn (37 kept walks of 55 hits on 2.2 kb: 0.46 ms, 1.52 on shared warps).
+constexpr int kStoreWarps = 4;
 __global__ void storeWalkKernel(const AlignJob *jobs, const WalkItem *items, int nItems, const int *anchorRow,
                                 const float *cells, const XS *X, const XS *suffix, const XS *revEv,
                                 const XS *fwdEv, Seg *segOut) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nItems) return;
+    const int t = blockIdx.x * kStoreWarps + (threadIdx.x >> 5);
+    if (t >= nItems || (threadIdx.x & 31) != 0) return;
     const WalkItem it = items[t];
     const AlignJob jb = jobs[it.job];
     const int a1 = anchorRow[jb.colOff + it.anchor2];

@@ -426,8 +426,9 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
 int dmst_align_fetch(const dmst_ctx *ctx, dmst_alignment *alignments, size_t cap_alignments,
                      dmst_segment *segments, size_t cap_segments);
 /* Wall-clock phases of the last dmst_align call (ms): out[0] the whole call,
- * [1] scoring every pair, [2] the hits' exact replay and traceback tables,
- * [3] the anchor sort, [4] the walks' span pass, [5] the choice of anchors,
+ * [1] scoring every pair, [2] the hits' exact replay, [3] the anchor sort
+ * (beside the traceback tables and the walks' span pass), [4] what of these
+ * the sort did not cover, [5] the choice of anchors,
  * [6] the kept walks and the segment copy, [7] hits traced, [8] kernel
  * launches of the call.  n <= 9. */
 int dmst_last_align_timing(const dmst_ctx *ctx, double *out, int n);
