@@ -1679,7 +1679,7 @@ def run_autograd(args, rank, world, local):
         "traffic": None,
         "peak_source": f"derived: {n_sm} SMs x 64 FP64 lanes x 2 x sm_max_mhz {sm_max:g} (of measured clock; "
                        "MEASURED_PEAKS.json has no FP64 figure)",
-        "kernel": "adjointKernel (forward, then backward with the gradient sums), CUDA events on the library "
+        "kernel": "adjointPipeKernel (forward, then backward with the gradient sums), CUDA events on the library "
                   "stream, summed over the step's launches",
         "algorithmic_flops_per_cell": AG_FLOPS_PER_CELL,
         "adjoint_gcups": total_cells / (adj_ms / 1e3) / 1e9,

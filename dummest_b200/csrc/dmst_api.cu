@@ -422,11 +422,11 @@ DpKern dpKernelFor(int R, bool mid, int warps, bool gt) {
 using PipeKern = void (*)(PipeArgs);
 template <bool MID>
 PipeKern pipeKernelByR(int R) {
-    return R == 4 ? pipeKernel<4, MID> : (R == 2 ? pipeKernel<2, MID> : pipeKernel<1, MID>);
+    return R == 2 ? pipeKernel<2, MID> : pipeKernel<1, MID>;
 }
 PipeKern pipeKernelFor(int R, bool mid) { return mid ? pipeKernelByR<true>(R) : pipeKernelByR<false>(R); }
 inline size_t pipeWindowBytes(int R) {
-    return R == 4 ? sizeof(WindowP<4>) : (R == 2 ? sizeof(WindowP<2>) : sizeof(WindowP<1>));
+    return R == 2 ? sizeof(WindowP<2>) : sizeof(WindowP<1>);
 }
 struct PipePlan {
     bool whole = false;  // the whole call runs on the pipeline (otherwise, a search's survivors)
@@ -1625,7 +1625,7 @@ static void pipeSpread(const dmst_ctx *ctx, size_t n, int stripes, int maxW, int
 // time of a step and the fill.  Twelve warps per SM.
 static int pipeShape(dmst_ctx *ctx, size_t n, double rows, int least, PipePlan &plan) {
     const int stripes = std::max(1, (int)std::ceil(rows / (kLanes * plan.R)));
-    const int maxW = (int)std::min<size_t>(pipeMaxWarps(plan.R), ((size_t)ctx->maxSmemOptin - 1024) / pipeWindowBytes(plan.R));
+    const int maxW = (int)std::min<size_t>(kPipeMaxWarps, ((size_t)ctx->maxSmemOptin - 1024) / pipeWindowBytes(plan.R));
     pipeSpread(ctx, n, stripes, maxW, 12, least, plan.W, plan.C);
     plan.smem = (size_t)plan.W * pipeWindowBytes(plan.R);
     CK(cudaFuncSetAttribute(plan.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem), "smem attribute");

@@ -277,11 +277,8 @@ __device__ __forceinline__ void atomicMaxPos(float *p, float v) {
     if (v > 0.0f) atomicMax(reinterpret_cast<int *>(p), __float_as_int(v));
 }
 
-// Warps of a CTA: four rows per lane need more than 128 registers.
-__host__ __device__ constexpr int pipeMaxWarps(int R) { return R == 4 ? 8 : kPipeMaxWarps; }
-
 template <int R, bool MID>
-__global__ void __launch_bounds__(pipeMaxWarps(R) * kLanes, 1) pipeKernel(PipeArgs g) {
+__global__ void __launch_bounds__(kPipeMaxWarps * kLanes, 1) pipeKernel(PipeArgs g) {
     extern __shared__ float4 smRaw[];
     WindowP<R> *wins = reinterpret_cast<WindowP<R> *>(smRaw);
     __shared__ float smBg[32];

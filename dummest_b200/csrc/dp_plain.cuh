@@ -33,8 +33,6 @@ constexpr int kPipeExtra = 128;      // stripe period P' = P + kPipeExtra
 constexpr int kPipeSpinLimit = 1 << 24;  // default iterations of a wait (64 ns sleeps) before it gives up
 static_assert(kPipeExtra >= kLanes - 1 + 2 * kBlock, "a window never reaches the next stripe early");
 
-__host__ __device__ inline int pipePeriod(int L) { return wavePeriod(L) + kPipeExtra; }
-
 struct PipeSync {
     volatile int *progress;  // [kPlainWarps]: ring-writer position of each warp
     volatile int *abort;     // the CTA's abort flag

@@ -219,21 +219,6 @@ __device__ __forceinline__ void storeW1(float *p, const float (&w)[R]) {
     }
 }
 
-// W1 values are read once, by the warp that wrote them: bypass L1 (the slot is
-// rewritten by the warp's next pair).
-template <int R>
-__device__ __forceinline__ void loadW1(float (&w)[R], const float *p) {
-    if constexpr (R == 4) {
-        float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
-        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else if constexpr (R == 2) {
-        float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
-        w[0] = v.x; w[1] = v.y;
-    } else {
-        w[0] = __ldcg(p);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Wavefront geometry.  Steps run in blocks of kBlock (a multiple of three);
 // the window holds the column operands of local times [t0 - 31, t0 + 2 kBlock)
