@@ -470,11 +470,12 @@ int dmst_tuned_rates_ex(const dmst_ctx *ctx, double *gcups, int n);
 int dmst_tuned_shape(const dmst_ctx *ctx, int M, int *rows_per_lane, int *warps_per_cta);
 
 /* The exact path's wait budget: a warp of the stripe-pipelined exact kernel
- * that waits for the stripe before its own (a flag in shared memory) gives up
- * after this many 64 ns sleeps, marks its pair failed and lets the CTA's
- * other warps leave at their next block; the call then returns DMST_ETIMEOUT
- * and the context stays usable.  iterations = 0 restores the default (2^24,
- * about a second); a small value makes a call with multi-stripe exact-path
+ * that waits for the stripe before its own (a ring entry in global memory)
+ * gives up after this many polls (of about half a microsecond; the plain
+ * schedule's waits: 64 ns sleeps), marks its pair failed and lets the
+ * cluster's other warps leave at their next block; the call then returns
+ * DMST_ETIMEOUT and the context stays usable.  iterations = 0 restores the
+ * default (2^24, some seconds); a small value makes a call with multi-stripe exact-path
  * pairs time out on purpose (the test of the timeout path).  No counterpart
  * in the reference (its threads never wait on one another inside a pair). */
 int dmst_set_wait_limit(dmst_ctx *ctx, int iterations);
