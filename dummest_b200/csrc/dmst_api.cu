@@ -669,8 +669,8 @@ struct dmst_ctx {
     DevBuf<int> dCounter;
     DevBuf<float> dW1, dRing;
     DevBuf<unsigned long long> dPipeRing;    // stripe pipeline: boundary rows, kRingEmpty between kernels
-    DevBuf<int> dPipeList, dPipeAbort;       // ... pair positions; an abort flag per cluster
-    bool pipeClean = false;                  // the ring and the flags are as a kernel expects them
+    DevBuf<int> dPipeList, dPipeAbort;       // ... pair positions; the ring's abort flag
+    bool pipeClean = false;                  // the ring and the flag are as a kernel expects them
     DevBuf<ExactJob> dJobs;
     DevBuf<AdjointJob> dAdjJobs;             // dmst_loglik_grad, dmst_posteriors
     DevBuf<int> dAdjStatus;                  // ... per job, then the launch's abort flag
@@ -688,8 +688,8 @@ struct dmst_ctx {
     int lastSlot = 0;                        // the slot of the last completed call
     DevBuf<float> dExactPool;                // exact-path scratch: one slot per cluster
     DevBuf<unsigned long long> dExactRing;   // exact path: boundary rows, kRingEmpty between kernels
-    DevBuf<int> dExactAbort;                 // ... an abort flag per cluster
-    bool exactClean = false;                 // the rings and the flags are as a kernel expects them
+    DevBuf<int> dExactAbort;                 // ... their abort flag
+    bool exactClean = false;                 // the rings and the flag are as a kernel expects them
     DevBuf<Chunk> dMidChunks;                // search: the survivors' chunks
     DevBuf<int> dSurvivors;                  // search: survivor pair indices by chunk
     DevBuf<int> dSurvivorList, dSurvivorCount;  // ... all of them; their number, and how many run from the list
@@ -1998,13 +1998,13 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
        "alloc W1 slots");
     if (pipe.clusters) {
         const size_t entries = (size_t)(pipe.clusters * pipe.ringSlot);
-        if (entries > ctx->dPipeRing.cap || (size_t)pipe.clusters > ctx->dPipeAbort.cap) ctx->pipeClean = false;
+        if (entries > ctx->dPipeRing.cap) ctx->pipeClean = false;
         CK(ctx->dPipeRing.ensure(entries, 0.25), "alloc stripe rings");
-        CK(ctx->dPipeAbort.ensure(pipe.clusters), "alloc stripe rings");
+        CK(ctx->dPipeAbort.ensure(1), "alloc stripe rings");
         if (!ctx->pipeClean) {
             CK(cudaMemsetAsync(ctx->dPipeRing.p, 0xff, ctx->dPipeRing.cap * sizeof(unsigned long long), ctx->stream),
                "empty stripe rings");
-            CK(cudaMemsetAsync(ctx->dPipeAbort.p, 0, ctx->dPipeAbort.cap * sizeof(int), ctx->stream), "zero abort flags");
+            CK(cudaMemsetAsync(ctx->dPipeAbort.p, 0, sizeof(int), ctx->stream), "zero abort flag");
             ctx->pipeClean = true;
         }
         if (pipeWhole) {
@@ -2108,15 +2108,14 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
             exactClusters = (int)std::max<size_t>(1, std::min<size_t>(exactClusters, poolBudget / slotBytes));
         }
         CK(ctx->dExactPool.ensure((size_t)exactClusters * poolSlot), "alloc exact scratch");
-        if ((size_t)(exactClusters * exactRing) > ctx->dExactRing.cap || (size_t)exactClusters > ctx->dExactAbort.cap)
-            ctx->exactClean = false;
+        if ((size_t)(exactClusters * exactRing) > ctx->dExactRing.cap) ctx->exactClean = false;
         CK(ctx->dExactRing.ensure((size_t)exactClusters * exactRing), "alloc exact rings");
-        CK(ctx->dExactAbort.ensure(exactClusters), "alloc exact rings");
+        CK(ctx->dExactAbort.ensure(1), "alloc exact rings");
         if (!ctx->exactClean) {
             CK(cudaStreamWaitEvent(ctx->stream, ctx->evExact, 0), "stream dependency");
             CK(cudaMemsetAsync(ctx->dExactRing.p, 0xff, ctx->dExactRing.cap * sizeof(unsigned long long), ctx->stream),
                "empty exact rings");
-            CK(cudaMemsetAsync(ctx->dExactAbort.p, 0, ctx->dExactAbort.cap * sizeof(int), ctx->stream), "zero abort flags");
+            CK(cudaMemsetAsync(ctx->dExactAbort.p, 0, sizeof(int), ctx->stream), "zero abort flag");
             ctx->exactClean = true;
         }
         CK(S.dExOut.ensure(n), "alloc exact out");

@@ -32,9 +32,9 @@
 // a barrier (neither reads the other's values), or run side by side on twice
 // as many warps as stripes; then the counts are scanned, then both replay
 // sweeps.  Every wait is for an earlier stripe of the same
-// cluster and bounded: a wait that runs out sets the cluster's abort flag,
-// every warp leaves its sweep, and the pair and those after it on the cluster
-// are marked failed.
+// cluster and bounded: a wait that runs out sets the ring buffer's abort flag
+// (dp_pipe.cuh), every warp leaves its sweep, and the pair and those started
+// after it are marked failed, also by a kernel queued before the host knows.
 //
 // Bound: the latency of a step, so two rows per lane, one column apart
 // (dp_stagger.cuh: neither waits for the other), on as many warps as there are
@@ -91,7 +91,7 @@ struct ExactPipeArgs {
     long long poolSlot;     // floats per cluster
     unsigned long long *ring;
     long long ringSlot;     // words per cluster
-    int *abort;             // one flag per cluster, 0 between kernels
+    int *abort;             // the ring buffer's flag, 0 while every word is empty between kernels
     ExactOut *out;
     // anchors: anchorOff[pair] >= 0 is the offset of its L columns
     const long long *anchorOff;
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
     const int cluster = blockIdx.x / C, nClusters = gridDim.x / C;
     float *base = g.pool + (size_t)cluster * g.poolSlot;
     unsigned long long *ring = g.ring + (size_t)cluster * g.ringSlot;
-    int *abort = g.abort + cluster;
+    int *abort = g.abort;
     const int n = *g.queueCount;
     for (int k = cluster; k < n; k += nClusters) {
         const int pi = g.queue[k];
@@ -983,7 +983,7 @@ __global__ void __launch_bounds__(kExactMaxWarps * kLanes, 1) exactPipeKernel(Ex
         };
         unsigned long long *rb = ring, *rf = ring + 2LL * nS * p.L;  // boundary rows downward and upward
         const int sLast = nS - 1 >= me ? me + (nS - 1 - me) / G * G : -1;
-        bool ok = abortPeek(abort) == 0;  // a wait of an earlier pair ran out: no later pair is started
+        bool ok = abortPeek(abort) == 0;  // a wait ran out, in this kernel or before it: no pair is started
         ExactBest filt{0.0, 0}, mid{0.0, 0};
         // Stripe s hands its boundary row on through entry row s of a ring.
         auto backIn = [&](int s) { return s < nS - 1 ? rb + 2LL * (s + 1) * p.L : nullptr; };

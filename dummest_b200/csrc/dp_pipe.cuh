@@ -18,9 +18,13 @@
 // a block ahead and look at them when they are needed; only then do they wait.
 // Every wait is for a stripe earlier in processing order, whose warp is in the
 // same cluster and hence resident, so the waits cannot form a cycle; each is
-// bounded (kRingSpin polls), after which the warp raises the cluster's abort
-// flag, every warp leaves its sweep at its next look at the ring, and the
-// pair's scores are NaN (the flag kernel sends such a pair to the exact path).
+// bounded (kRingSpin polls), after which the warp raises the abort flag, every
+// warp leaves its sweep at its next look at the ring, and the pair's scores are
+// NaN (the flag kernel sends such a pair to the exact path).  The flag is the
+// ring buffer's, not the cluster's: a warp that gives up leaves entries behind,
+// and the next kernel, which may be queued already, cuts the buffer into other
+// slots.  So no pair is started while the flag is up; the host empties the
+// buffer and lowers it.
 //
 // Why: one warp takes nS (L + 3) steps per sweep at about 290 cycles (one busy
 // warp per SM sub-partition), however empty the GPU is.  With G warps a sweep
@@ -69,7 +73,7 @@ struct PipeArgs {
     long long w1Slot;     // floats
     unsigned long long *ring;
     long long ringSlot;   // entries
-    int *abort;           // one flag per cluster, 0 between kernels
+    int *abort;           // the ring buffer's flag, 0 while every entry is empty between kernels
     PairOut *out;         // zeroed
 };
 
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(kPipeMaxWarps * kLanes, 1) pipeKernel(PipeArgs
     WindowS<R> &win = wp.s;
     float *w1 = g.w1 + (size_t)cluster * g.w1Slot;
     unsigned long long *ring = g.ring + (size_t)cluster * g.ringSlot;
-    int *abort = g.abort + cluster;
+    int *abort = g.abort;
     const int n = g.nList ? *g.nList : g.nPairs;
     for (int k = cluster; k < n; k += nClusters) {
         const int pi = g.list[k];
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(kPipeMaxWarps * kLanes, 1) pipeKernel(PipeArgs
             a.w1 = w1 + s * stripeFloats;
         };
         float filt = 0.0f, maxY = 0.0f, mid = 0.0f, maxFw = 0.0f;
-        bool ok = abortPeek(abort) == 0;  // a wait of an earlier pair ran out: no later pair is started
+        bool ok = abortPeek(abort) == 0;  // a wait ran out, in this kernel or before it: no pair is started
         const int sLast = nS - 1 >= me ? me + (nS - 1 - me) / G * G : -1;  // this warp's highest stripe
         for (int s = sLast; s >= 0 && ok; s -= G) {
             a.nS = s > 0 ? 2 : 1;
