@@ -713,7 +713,8 @@ struct dmst_ctx {
     int lastExactPairs = 0;
     int lastLaunches = 0;
     int lastFlagged = -1;  // pairs the last completed mid-score call sent to the exact path (-1: none yet)
-    int waitLimit = 0;    // exact path: iterations of a stripe wait before it gives up (0: the default)
+    int waitLimit = 0;    // polls of a stripe pipeline's wait before it gives up (0: the default)
+    int spinLimit() const { return waitLimit > 0 ? waitLimit : kRingSpin; }
 
     int fail(int status, const char *fmt, ...) {
         char buf[512];
@@ -2230,7 +2231,8 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
         auto pipeRun = [&](PipeKern kern, const int *list, const int *nList, int count, PairOut *out) -> int {
             CK(cudaMemsetAsync(out, 0, n * sizeof(PairOut), ctx->stream), "zero results");
             PipeArgs pa{list, nList, count, g.pairs, g.profiles, g.emit, g.params, g.codes, g.seeds,
-                        g.scales, ctx->dW1.p, pipe.w1Slot, ctx->dPipeRing.p, pipe.ringSlot, ctx->dPipeAbort.p, out};
+                        g.scales, ctx->dW1.p, pipe.w1Slot, ctx->dPipeRing.p, pipe.ringSlot, ctx->dPipeAbort.p, out,
+                        ctx->spinLimit()};
             cudaLaunchAttribute at;
             const cudaLaunchConfig_t cfg =
                 clusterLaunch(pipe.C, pipe.W, pipe.smem, pipe.clusters * pipe.C, &at, ctx->stream);
@@ -2345,7 +2347,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                                       (uintptr_t)S.hOut.p, (uintptr_t)S.hExOut.p};
         for (uintptr_t v : {(uintptr_t)pipe.kern, (uintptr_t)pipe.clusters, (uintptr_t)pipe.C, (uintptr_t)pipe.W,
                             (uintptr_t)pipe.w1Slot, (uintptr_t)pipe.ringSlot, (uintptr_t)ctx->dPipeRing.p,
-                            (uintptr_t)ctx->dPipeList.p, (uintptr_t)ctx->dPipeAbort.p})
+                            (uintptr_t)ctx->dPipeList.p, (uintptr_t)ctx->dPipeAbort.p, (uintptr_t)ctx->spinLimit()})
             key.push_back(v);
         for (const Group &G : groups) {
             const uintptr_t v[8] = {(uintptr_t)G.kern, (uintptr_t)G.grid,         (uintptr_t)G.warps,
@@ -2406,7 +2408,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                                exactRing, ctx->dExactAbort.p, S.dExOut.p, anchors ? S.dAnchorOff.p : nullptr,
                                S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p, align ? ctx->dAlignJobOf.p : nullptr,
                                align ? ctx->dAlignJobs.p : nullptr, align ? ctx->dAlignSteps.p : nullptr,
-                               align ? ctx->dAlignRows.p : nullptr, ctx->waitLimit > 0 ? ctx->waitLimit : kRingSpin};
+                               align ? ctx->dAlignRows.p : nullptr, ctx->spinLimit()};
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t cfg = clusterLaunch(exactC, exactW, exactW * sizeof(WindowX), exactC * exactClusters, &at, tail);
         CK(cudaLaunchKernelEx(&cfg, ek, ea), "exact kernel");
@@ -3330,7 +3332,8 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
                 AdjPipeArgs a{ctx->dAdjJobs.p, nj, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p,
                               ctx->dCodes.p, S.dSeeds.p, S.dScales.p, ctx->dAdjF.p,
                               reinterpret_cast<unsigned long long *>(ctx->dAdjB.p), ctx->dGrad.p, ctx->dLogT.p,
-                              tables ? ctx->dPost.p : nullptr, ctx->dAdjStatus.p, ctx->dAdjStatus.p + nj};
+                              tables ? ctx->dPost.p : nullptr, ctx->dAdjStatus.p, ctx->dAdjStatus.p + nj,
+                              ctx->spinLimit()};
                 cudaLaunchAttribute at;
                 const cudaLaunchConfig_t cfg = clusterLaunch(pC, pW, pW * sizeof(AdjWin), pC * std::min(pClusters, nj),
                                                              &at, ctx->stream);

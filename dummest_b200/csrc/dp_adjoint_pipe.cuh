@@ -92,6 +92,7 @@ struct AdjPipeArgs {
     double *post;
     int *status;                 // per job, AdjStatus, zeroed
     int *abort;                  // a wait of the launch ran out
+    int spinLimit;               // polls of a wait before it gives up
 };
 
 // The pair as every stripe sees it.
@@ -102,6 +103,7 @@ struct AdjPair {
     double sC, s1, s2;
     unsigned long long *fb, *bb;  // boundary entries: [stripe][column] x (W, Y)
     int *abort;
+    int spinLimit;
 };
 
 __device__ __forceinline__ double asD(unsigned long long v) { return __longlong_as_double((long long)v); }
@@ -119,14 +121,14 @@ __device__ __forceinline__ AdjEntry adjPeek(const unsigned long long *row, int c
     return e;
 }
 // Waits until no lane's entry is empty; false: given up.
-__device__ __forceinline__ bool adjWaitEntry(AdjEntry &e, const unsigned long long *row, int col, int *abort) {
+__device__ __forceinline__ bool adjWaitEntry(AdjEntry &e, const unsigned long long *row, int col, const AdjPair &p) {
     int it = 0;
     while (__any_sync(kFull, e.w == kAdjEmpty || e.y == kAdjEmpty)) {
         if (e.w == kAdjEmpty || e.y == kAdjEmpty) e = adjPeek(row, col, true);
-        if ((++it & 63) == 0) {
-            const bool gone = it > kRingSpin || abortPeek(abort) != 0;
+        if (++it > p.spinLimit || (it & 63) == 0) {
+            const bool gone = it > p.spinLimit || abortPeek(p.abort) != 0;
             if (__any_sync(kFull, gone)) {
-                *reinterpret_cast<volatile int *>(abort) = 1;
+                *reinterpret_cast<volatile int *>(p.abort) = 1;
                 return false;
             }
         }
@@ -236,7 +238,7 @@ __device__ bool adjForward(AdjWin &w, const AdjPair &p, int s, int lane, double 
     AdjEntry ent = adjPeek(in, lane, in && lane < p.L);
     float suf = lane < p.L ? __ldg(p.suf + lane) : 0.0f;
     for (int k0 = 0; k0 < nSteps; k0 += 32) {
-        if (in && !adjWaitEntry(ent, in, k0 + lane, p.abort)) return false;
+        if (in && !adjWaitEntry(ent, in, k0 + lane, p)) return false;
         __syncwarp();
         adjPutFCol(w, p, next, k0 + lane);
         w.fw[(k0 + lane) & 63] = asD(ent.w);
@@ -392,7 +394,7 @@ __device__ bool adjBackward(AdjWin &w, const AdjPair &p, int s, int lane, const 
     double zz1 = 0, zz2 = 0, zz3 = 0;  // own Z at j+1, j+2, j+3
     double pubW = 0, pubY = 0;
     for (int k0 = 0; k0 < nSteps; k0 += 32) {
-        if (in && !adjWaitEntry(ent, in, k0 + lane, p.abort)) {
+        if (in && !adjWaitEntry(ent, in, k0 + lane, p)) {
             adjWait<0>();
             return false;
         }
@@ -521,6 +523,7 @@ __global__ void __launch_bounds__(kAdjPipeWarps * kLanes, 1) adjointPipeKernel(A
         p.fb = g.bstore + job.bOff;
         p.bb = p.fb + 2 * (size_t)p.nS * p.L;
         p.abort = g.abort;
+        p.spinLimit = g.spinLimit;
         double *F = g.fstore + job.fOff;
         double *buf = F + adjPipeStates(d.M, d.L) + (size_t)me * 2 * kAdjCk * 96;
         double *parts = F + (CKPT ? adjPipeStates(d.M, d.L) + adjPipeBufs(d.M, G) : (long long)p.nS * (p.L + 31) * 96);

@@ -18,7 +18,7 @@
 // a block ahead and look at them when they are needed; only then do they wait.
 // Every wait is for a stripe earlier in processing order, whose warp is in the
 // same cluster and hence resident, so the waits cannot form a cycle; each is
-// bounded (kRingSpin polls), after which the warp raises the abort flag, every
+// bounded (spinLimit polls), after which the warp raises the abort flag, every
 // warp leaves its sweep at its next look at the ring, and the pair's scores are
 // NaN (the flag kernel sends such a pair to the exact path).  The flag is the
 // ring buffer's, not the cluster's: a warp that gives up leaves entries behind,
@@ -38,7 +38,7 @@
 namespace dmst {
 
 constexpr unsigned long long kRingEmpty = ~0ull;
-constexpr int kRingSpin = 1 << 24;   // polls of one wait before it gives up (about 0.5 us each)
+constexpr int kRingSpin = 1 << 24;   // default polls of one wait before it gives up (about 0.5 us each)
 constexpr int kPipeMaxWarps = 16;
 constexpr int kPipeMaxCluster = 8;   // CTAs of a cluster (portable size)
 
@@ -75,6 +75,7 @@ struct PipeArgs {
     long long ringSlot;   // entries
     int *abort;           // the ring buffer's flag, 0 while every entry is empty between kernels
     PairOut *out;         // zeroed
+    int spinLimit;        // polls of a wait before it gives up
 };
 
 __device__ __forceinline__ unsigned long long ringPeek(const unsigned long long *p) {
@@ -121,13 +122,13 @@ __device__ __forceinline__ FillP fillLoadP(const SweepArgs &a, const unsigned lo
 // window entries.  False: given up.
 template <bool BACKWARD, int R>
 __device__ __forceinline__ bool fillStoreP(WindowS<R> &w, const SweepArgs &a, FillP f, unsigned long long *ringIn, int u,
-                                           int *abort) {
+                                           int *abort, int spinLimit) {
     if (ringIn) {
         int it = 0;
         while (__any_sync(kFull, f.ring == kRingEmpty)) {
             if (f.ring == kRingEmpty) f.ring = ringPeek(ringIn + u);
-            if ((++it & 63) == 0) {
-                const bool gone = it > kRingSpin || abortPeek(abort) != 0;
+            if (++it > spinLimit || (it & 63) == 0) {
+                const bool gone = it > spinLimit || abortPeek(abort) != 0;
                 if (__any_sync(kFull, gone)) {
                     if (gone) *reinterpret_cast<volatile int *>(abort) = 1;
                     return false;
@@ -143,10 +144,10 @@ __device__ __forceinline__ bool fillStoreP(WindowS<R> &w, const SweepArgs &a, Fi
 
 template <bool BACKWARD, int R>
 __device__ __forceinline__ bool fillPrologueP(WindowS<R> &w, const SweepArgs &a, unsigned long long *ringIn, int lane,
-                                              int *abort, FillP &next) {
+                                              int *abort, int spinLimit, FillP &next) {
     constexpr int S = kLanes * R;
     for (int v = -S + lane; v < 0; v += kLanes) fillStoreS<BACKWARD, R>(w, a, FillRegs{kPad, 0.0f, 0.0f, 0.0f, 0.0f}, v);
-    if (!fillStoreP<BACKWARD, R>(w, a, fillLoadP<BACKWARD>(a, ringIn, lane), ringIn, lane, abort)) return false;
+    if (!fillStoreP<BACKWARD, R>(w, a, fillLoadP<BACKWARD>(a, ringIn, lane), ringIn, lane, abort, spinLimit)) return false;
     next = fillLoadP<BACKWARD>(a, ringIn, kSBlock + lane);
     return true;
 }
@@ -155,7 +156,7 @@ __device__ __forceinline__ bool fillPrologueP(WindowS<R> &w, const SweepArgs &a,
 // = 1), or as the first of two (nS = 2) when it hands its lowest row on.
 template <int R, bool MID>
 __device__ bool pipeBackward(const SweepArgs &a, WindowS<R> &win, int lane, unsigned long long *ringIn, int *abort,
-                             float &filt, float &maxY) {
+                             int spinLimit, float &filt, float &maxY) {
     constexpr int S = kLanes * R;
     constexpr int SW = kLanes * stagLaneStride(R);
     BwdS<R> b;
@@ -181,10 +182,10 @@ __device__ bool pipeBackward(const SweepArgs &a, WindowS<R> &win, int lane, unsi
     const int T = (a.L - 1 + S + 3) / 4 * 4;
     __syncwarp();
     FillP pf;
-    if (!fillPrologueP<true, R>(win, a, ringIn, lane, abort, pf)) return false;
+    if (!fillPrologueP<true, R>(win, a, ringIn, lane, abort, spinLimit, pf)) return false;
     for (int t0 = 0; t0 < T; t0 += kSBlock) {
         __syncwarp();
-        if (!fillStoreP<true, R>(win, a, pf, ringIn, t0 + kSBlock + lane, abort)) return false;
+        if (!fillStoreP<true, R>(win, a, pf, ringIn, t0 + kSBlock + lane, abort, spinLimit)) return false;
         pf = fillLoadP<true>(a, ringIn, t0 + 2 * kSBlock + lane);
         __syncwarp();
         const int n = min(kSBlock, T - t0);
@@ -201,7 +202,7 @@ __device__ bool pipeBackward(const SweepArgs &a, WindowS<R> &win, int lane, unsi
 // L - 2 + 32 R - t of the stripe.
 template <int R>
 __device__ bool pipeForward(const SweepArgs &a, WindowS<R> &win, int lane, unsigned long long *ringIn, int *abort,
-                            float &best, float &mx) {
+                            int spinLimit, float &best, float &mx) {
     constexpr int S = kLanes * R;
     constexpr int SW = kLanes * stagLaneStride(R);
     FwdS<R> f;
@@ -237,10 +238,10 @@ __device__ bool pipeForward(const SweepArgs &a, WindowS<R> &win, int lane, unsig
     }
     __syncwarp();
     FillP pf;
-    bool ok = fillPrologueP<false, R>(win, a, ringIn, lane, abort, pf);
+    bool ok = fillPrologueP<false, R>(win, a, ringIn, lane, abort, spinLimit, pf);
     for (int t0 = 0; ok && t0 < T; t0 += kSBlock) {
         __syncwarp();
-        ok = fillStoreP<false, R>(win, a, pf, ringIn, t0 + kSBlock + lane, abort);
+        ok = fillStoreP<false, R>(win, a, pf, ringIn, t0 + kSBlock + lane, abort, spinLimit);
         if (!ok) break;
         pf = fillLoadP<false>(a, ringIn, t0 + 2 * kSBlock + lane);
         __syncwarp();
@@ -354,7 +355,8 @@ __global__ void __launch_bounds__(kPipeMaxWarps * kLanes, 1) pipeKernel(PipeArgs
             a.nS = s > 0 ? 2 : 1;
             stripe(s, (a.nS - 1) * S);
             a.ring = reinterpret_cast<float *>(ring + (long long)s * p.L);
-            ok = pipeBackward<R, MID>(a, win, lane, s < nS - 1 ? ring + (long long)(s + 1) * p.L : nullptr, abort, filt, maxY);
+            ok = pipeBackward<R, MID>(a, win, lane, s < nS - 1 ? ring + (long long)(s + 1) * p.L : nullptr, abort, g.spinLimit, filt,
+                                      maxY);
         }
         if (MID) {
             unsigned long long *fr = ring + (long long)nS * p.L;
@@ -362,7 +364,8 @@ __global__ void __launch_bounds__(kPipeMaxWarps * kLanes, 1) pipeKernel(PipeArgs
                 a.nS = s < nS - 1 ? 2 : 1;
                 stripe(s, 0);
                 a.ring = reinterpret_cast<float *>(fr + (long long)s * p.L);
-                ok = pipeForward<R>(a, win, lane, s > 0 ? fr + (long long)(s - 1) * p.L : nullptr, abort, mid, maxFw);
+                ok = pipeForward<R>(a, win, lane, s > 0 ? fr + (long long)(s - 1) * p.L : nullptr, abort, g.spinLimit, mid,
+                                    maxFw);
             }
         }
         filt = warpMax(filt);

@@ -488,7 +488,7 @@ class Context:
         return {(r, w): out[base + i * 3 + j] for i, r in enumerate((4, 3, 2, 1)) for j, w in enumerate((16, 8, 12))}
 
     def set_wait_limit(self, iterations: int = 0) -> None:
-        """The exact path's wait budget in polls (plain schedule: 64 ns sleeps; dmst_set_wait_limit; 0: the default)."""
+        """The stripe pipelines' wait budget in polls (plain schedule: 64 ns sleeps; dmst_set_wait_limit; 0: the default)."""
         self._check(self.lib.dmst_set_wait_limit(self.h, int(iterations)), "dmst_set_wait_limit")
 
     def tuned_shape(self, M: int) -> tuple[int, int]:

@@ -469,15 +469,23 @@ int dmst_tuned_rates_ex(const dmst_ctx *ctx, double *gcups, int n);
 /* The shape a call would use for a profile of length M. */
 int dmst_tuned_shape(const dmst_ctx *ctx, int M, int *rows_per_lane, int *warps_per_cta);
 
-/* The exact path's wait budget: a warp of the stripe-pipelined exact kernel
- * that waits for the stripe before its own (a ring entry in global memory)
- * gives up after this many polls (of about half a microsecond; the plain
- * schedule's waits: 64 ns sleeps), marks its pair failed and lets the
- * cluster's other warps leave at their next block; the call then returns
- * DMST_ETIMEOUT and the context stays usable.  iterations = 0 restores the
- * default (2^24, some seconds); a small value makes a call with multi-stripe exact-path
- * pairs time out on purpose (the test of the timeout path).  No counterpart
- * in the reference (its threads never wait on one another inside a pair). */
+/* The stripe pipelines' wait budget: a warp that waits for the stripe before
+ * its own (an entry in global memory) gives up after this many polls (of about
+ * half a microsecond; the plain schedule's waits: 64 ns sleeps), and the other
+ * warps leave at their next block.  What follows depends on the pipeline:
+ *   exact path                     the call returns DMST_ETIMEOUT;
+ *   filter call, or either wave of
+ *   a search, of few pairs         the call returns DMST_ETIMEOUT;
+ *   mid call of few pairs, plain   its pairs run on the exact path (under the
+ *   schedule                       same budget) and the call returns its scores;
+ *   gradient, posteriors           every pair runs again on the one-warp kernel,
+ *                                  which waits for nothing.
+ * A call that was submitted behind one that gave up, before that one was
+ * completed, is treated alike.  The context stays usable.  iterations = 0
+ * restores the default (2^24, some seconds); a small value makes a wait of a
+ * multi-stripe pair run out on purpose (the test of these paths).  The value
+ * holds for calls submitted after it.  No counterpart in the reference (its
+ * threads never wait on one another inside a pair). */
 int dmst_set_wait_limit(dmst_ctx *ctx, int iterations);
 
 /* Column checkpointing of the adjoint's forward pass (dmst_loglik_grad,

@@ -73,3 +73,63 @@ def test_exact_call_behind_one_that_gave_up(first, second):
             assert got is None or _scores(got) == want_b
             assert _scores(ctx.score_pairs_raw(b, mode)) == want_b
             assert _scores(ctx.score_pairs_raw(a, mode)) == want_a
+
+
+def _case(M, lengths):
+    prof, p = _profile(M)
+    return p, _reads([prof] * len(lengths), lengths)
+
+
+def _gives_up(ctx, call):
+    """The call with a budget of one poll ends with DMST_ETIMEOUT."""
+    ctx.set_wait_limit(1)
+    with pytest.raises(d.DmstError) as err:
+        call()
+    assert err.value.status == F.DMST_ETIMEOUT
+    ctx.set_wait_limit(0)
+
+
+# two stripes of 64 rows (and R = 1: two of 32), many; one pair (a cluster of CTAs), one warp or more a stripe
+@pytest.mark.parametrize("M,lengths", [(64, [700, 900]), (600, [1500, 1200]), (200, [400] * 300), (2000, [3000])])
+def test_pipelined_calls_that_give_up(M, lengths):
+    """Filter, mid, graph and search calls of few pairs: DMST_ETIMEOUT (the mid
+    call's pairs go to the exact path, which has the same budget), and the same
+    results as before once the budget is restored."""
+    p, reads = _case(M, lengths)
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        a = _pairs(ctx.add_dna(reads), [pid] * len(reads))
+        gate = np.zeros(1, np.float32)
+        calls = [lambda: ctx.score_pairs_raw(a, d.MODE_FILTER), lambda: ctx.score_pairs_raw(a, d.MODE_MID),
+                 lambda: ctx.score_pairs_raw(a, d.MODE_MID | d.MODE_GRAPH), lambda: ctx.search_raw(a, gate)]
+        results = lambda res: list(zip(_scores(res), [r.filter_f for r in res]))
+        before = [results(call()) for call in calls]
+        for call, want in zip(calls, before):
+            for _ in range(2):
+                _gives_up(ctx, call)
+                assert results(call()) == want
+
+
+@pytest.mark.parametrize("M,lengths", [(32, [300, 350]), (200, [700, 500, 900]), (130, [400] * 200)])
+def test_adjoint_that_gives_up(M, lengths):
+    """Gradients and posteriors run again on the one-warp kernel: the same log T
+    and tables bit for bit, the gradient up to the order of its sums."""
+    p, reads = _case(M, lengths)
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        sids = ctx.add_dna(reads)
+        for mode in (F.ADJ_CKPT_OFF, F.ADJ_CKPT_ON):
+            ctx.adjoint_checkpoint(mode)
+            got, launches = [], []
+            for limit in (0, 1, 0):
+                ctx.set_wait_limit(limit)
+                got.append((ctx.loglik_grad(sids, pid), ctx.posterior_summary(sids, pid)))
+                ctx.loglik_grad(sids, pid)
+                launches.append(ctx.last_timing()["launches"])
+            assert launches[0] == launches[2] == launches[1] - 1  # the pipeline's and the one-warp kernel's
+            (lt, gp, ge), (plt, tracks) = got[0]
+            for (l2, gp2, ge2), (pl2, tr2) in got[1:]:
+                assert np.array_equal(lt, l2) and np.array_equal(plt, pl2)
+                for x, y in ((gp, gp2), (ge, ge2)):
+                    np.testing.assert_allclose(x, y, rtol=1e-11, atol=1e-13 * np.abs(x).max())
+                assert all(np.array_equal(u, v) for t, t2 in zip(tracks, tr2) for u, v in zip(t, t2))
