@@ -2493,11 +2493,14 @@ static int completeCall(dmst_ctx *ctx) {
     const bool search = S.search;
     const uint8_t *survived = search ? S.hMask.p : nullptr;
     const PairOut *pf = search ? S.hOutF.p : nullptr;
+    // Waits that ran out: the rings of that pipeline are not empty.  Both are
+    // looked at before the call fails for either.
+    int gaveUp = -1, exactGaveUp = -1;  // a pair of the caller's order
     if (S.pipe)
         for (size_t k = 0; k < n; ++k)
             if (std::isnan(po[k].filt) || (search && std::isnan(pf[k].filt))) {
-                ctx->pipeClean = false;  // a wait of the stripe pipeline ran out: its rings are not empty
-                if (!mid || search) return ctx->fail(DMST_ETIMEOUT, "the stripe pipeline of pair %d gave up a wait", order[k]);
+                ctx->pipeClean = false;
+                if (!mid || search) gaveUp = order[k];  // a mid call's pair is on the exact path
             }
     // Pairs outside the fast path's exact range go to the row-rescaled kernel.
     std::vector<int> flagged;
@@ -2559,10 +2562,12 @@ static int completeCall(dmst_ctx *ctx) {
     }
     for (size_t f = 0; f < eo.size(); ++f)
         if (eo[f].failed) {
-            ctx->exactClean = false;  // its rings are not empty
-            return ctx->fail(DMST_ETIMEOUT, "exact path: the stripe pipeline of pair %d gave up a wait",
-                             order[flagged[f]]);
+            ctx->exactClean = false;
+            exactGaveUp = order[flagged[f]];
         }
+    if (gaveUp >= 0) return ctx->fail(DMST_ETIMEOUT, "the stripe pipeline of pair %d gave up a wait", gaveUp);
+    if (exactGaveUp >= 0)
+        return ctx->fail(DMST_ETIMEOUT, "exact path: the stripe pipeline of pair %d gave up a wait", exactGaveUp);
     ctx->lastExactMs = exactMs;
     ctx->lastExactPairs = (int)flagged.size();
     if (mid) ctx->lastFlagged = (int)flagged.size();

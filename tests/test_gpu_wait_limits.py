@@ -133,3 +133,19 @@ def test_adjoint_that_gives_up(M, lengths):
                 for x, y in ((gp, gp2), (ge, ge2)):
                     np.testing.assert_allclose(x, y, rtol=1e-11, atol=1e-13 * np.abs(x).max())
                 assert all(np.array_equal(u, v) for t, t2 in zip(tracks, tr2) for u, v in zip(t, t2))
+
+
+def test_search_whose_two_pipelines_give_up():
+    """A search's survivors run on the few-pair pipeline (the filter wave of 1,000
+    pairs does not), and those it gives up go to the exact path, which gives up
+    too: both rings are emptied before the next call that uses them."""
+    p, reads = _case(300, [950] * 40 + [300] * 960)
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        a = _pairs(ctx.add_dna(reads), [pid] * len(reads))
+        gate = np.zeros(1, np.float32)
+        want = _scores(ctx.search_raw(a, gate))
+        assert ctx.last_timing()["exact_pairs"] > 0
+        for _ in range(2):
+            _gives_up(ctx, lambda: ctx.search_raw(a, gate))
+            assert _scores(ctx.search_raw(a, gate)) == want
