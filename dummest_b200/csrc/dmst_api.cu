@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -1586,6 +1587,13 @@ static void scoreToResult(XS s, dmst_score *dst, double *ln) {
     *ln = (s.m == 0.0f) ? -INFINITY : scoreLn(s.m, s.e);
 }
 
+// A score as the float pass has it: infinite beyond the float range, and zero
+// below the normal floats (flush to zero).
+static float scoreFloat(XS s) {
+    const float f = (float)std::ldexp((double)s.m, s.e);
+    return f < FLT_MIN ? 0.0f : f;
+}
+
 // Milliseconds between two recorded events; a timing failure is noted in the
 // context's error text and cleared (it must not surface as the error of a
 // later launch check), and reads as -1.
@@ -2496,12 +2504,13 @@ static int completeCall(dmst_ctx *ctx) {
     // Waits that ran out: the rings of that pipeline are not empty.  Both are
     // looked at before the call fails for either.
     int gaveUp = -1, exactGaveUp = -1;  // a pair of the caller's order
-    if (S.pipe)
-        for (size_t k = 0; k < n; ++k)
-            if (std::isnan(po[k].filt) || (search && std::isnan(pf[k].filt))) {
-                ctx->pipeClean = false;
-                if (!mid || search) gaveUp = order[k];  // a mid call's pair is on the exact path
-            }
+    // The float pass ran for these pairs; its scores are never NaN otherwise.
+    auto floatPass = [&](size_t k) { return !forceExact && (!survived || survived[k]); };
+    for (size_t k = 0; k < n; ++k)
+        if ((floatPass(k) && std::isnan(po[k].filt)) || (search && std::isnan(pf[k].filt))) {
+            if (S.pipe) ctx->pipeClean = false;
+            if (!mid || search) gaveUp = order[k];  // a mid call's pair is on the exact path
+        }
     // Pairs outside the fast path's exact range go to the row-rescaled kernel.
     std::vector<int> flagged;
     for (size_t k = 0; k < n; ++k) {
@@ -2600,7 +2609,7 @@ static int completeCall(dmst_ctx *ctx) {
                 fillResult(r, po[k].mid, false, &r.mid, &r.mid_ln);
                 fillResult(r, po[k].filt, false, &r.filter, &r.filter_ln);
             }
-            r.filter_f = po[k].filt;
+            r.filter_f = floatPass(k) && !std::isnan(po[k].filt) ? po[k].filt : scoreFloat(eo[flagAt[k]].filt);
             if (search) {
                 r.filter_f = pf[k].filt;  // the float filter of the first wave
                 r.flags |= DMST_RES_SURVIVOR;

@@ -121,7 +121,9 @@ typedef struct dmst_result {
     dmst_score filter; /* max_{i,j} W1*prefixSeed (exact pair, MODE_MID)     */
     double mid_ln;     /* ln(mid) = scoreToLog(mid); -inf for zero            */
     double filter_ln;  /* ln(filter) (MODE_MID) or ln of the float filter     */
-    float filter_f;    /* MODE_FILTER: the float filter score as the reference returns it */
+    float filter_f;    /* the float filter score as the reference returns it (inf beyond float range);
+                        * in mid calls the same, or the exact filter score as a float where only the
+                        * exact path scored the pair */
     int32_t flags;     /* DMST_RES_*                                          */
 } dmst_result;
 

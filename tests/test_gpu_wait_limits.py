@@ -149,3 +149,41 @@ def test_search_whose_two_pipelines_give_up():
         for _ in range(2):
             _gives_up(ctx, lambda: ctx.search_raw(a, gate))
             assert _scores(ctx.search_raw(a, gate)) == want
+
+
+def test_pairs_that_the_exact_path_takes_over():
+    """A mid call in flight behind a filter call that gave up finds the ring not
+    empty: its pairs are scored on the exact path, with every field as ever."""
+    p, reads = _case(600, [1900, 1500, 400, 90])
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        a = _pairs(ctx.add_dna(reads), [pid] * len(reads))
+        b = _pairs([r.seq for r in a][::-1], [pid] * len(reads))
+        fields = lambda res: [(s, r.mid_ln, r.filter_ln, r.filter_f) for s, r in zip(_scores(res), res)]
+        want = fields(ctx.score_pairs_raw(b, d.MODE_MID))
+        ctx.set_wait_limit(1)
+        ctx.submit_raw(a, d.MODE_FILTER)
+        ctx.set_wait_limit(0)
+        ctx.submit_raw(b, d.MODE_MID)
+        assert _status(ctx) is None
+        got = _status(ctx)
+        assert got is not None and fields(got) == want
+        assert all(r.flags & F.RES_EXACT_PATH for r in got)
+        assert fields(ctx.score_pairs_raw(b, d.MODE_MID | d.MODE_FORCE_EXACT)) == want
+
+
+def test_plain_schedule_that_gives_up():
+    """Two stripes of 32 rows on two warps, one of 64 on the exact path: the mid
+    call's pairs are taken over, the filter call ends with DMST_ETIMEOUT."""
+    p, reads = _case(50, [400, 300])
+    with d.Context(rows_per_lane=1) as ctx:
+        pid = ctx.add_profile(*p)
+        a = _pairs(ctx.add_dna(reads), [pid] * len(reads))
+        plain = lambda mode: [(s, r.filter_f) for res in [ctx.score_pairs_raw(a, mode | d.MODE_PLAIN)]
+                              for s, r in zip(_scores(res), res)]
+        want = [plain(m) for m in (d.MODE_MID, d.MODE_FILTER)]
+        ctx.set_wait_limit(1)
+        assert plain(d.MODE_MID) == want[0]
+        assert ctx.last_timing()["exact_pairs"] == len(reads)
+        _gives_up(ctx, lambda: plain(d.MODE_FILTER))
+        assert [plain(m) for m in (d.MODE_MID, d.MODE_FILTER)] == want
