@@ -1719,10 +1719,11 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
     // the plain schedule's kernel: the pair's stripes on the CTA's warps, or
     // (DMST_MODE_PLAIN_1WARP) the batched kernel's one warp per pair
     const bool plainStriped = plain && !(mode & DMST_MODE_PLAIN_1WARP);
-    const bool forceExact = (mode & (DMST_MODE_FORCE_EXACT | DMST_MODE_EXACT_SEQUENTIAL)) != 0;
-    const bool sequentialExact = (mode & DMST_MODE_EXACT_SEQUENTIAL) != 0;
     if (base != DMST_MODE_MID && base != DMST_MODE_FILTER) return DMST_EINVAL;
     const bool mid = base == DMST_MODE_MID;
+    // (a filter call has the float pass only, whatever the exact-path flags)
+    const bool forceExact = mid && (mode & (DMST_MODE_FORCE_EXACT | DMST_MODE_EXACT_SEQUENTIAL)) != 0;
+    const bool sequentialExact = (mode & DMST_MODE_EXACT_SEQUENTIAL) != 0;
     const auto hostT0 = std::chrono::steady_clock::now();
     const int si = ctx->nextSlot;
     CallSlot &S = ctx->slot[si];
@@ -2480,7 +2481,7 @@ static int completeCall(dmst_ctx *ctx) {
     ctx->lastOrder = S.order;
     const size_t n = S.n;
     const bool mid = S.mid, nullOnly = S.nullOnly;
-    const bool forceExact = (S.mode & (DMST_MODE_FORCE_EXACT | DMST_MODE_EXACT_SEQUENTIAL)) != 0;
+    const bool forceExact = mid && (S.mode & (DMST_MODE_FORCE_EXACT | DMST_MODE_EXACT_SEQUENTIAL)) != 0;
     const std::vector<int> &order = S.order;
     const std::vector<DevPair> &dp = S.dp;
     dmst_result *out = S.out;

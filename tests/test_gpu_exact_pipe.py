@@ -79,3 +79,17 @@ def test_calls_in_flight_share_the_scratch():
             pass
     for (_, res), w in zip(arrays, want):
         assert [(d.Score(r.mid.m, r.mid.e), d.Score(r.filter.m, r.filter.e)) for r in res] == w
+
+
+@pytest.mark.parametrize("flag", [d.MODE_FORCE_EXACT, d.MODE_EXACT_SEQUENTIAL])
+def test_filter_calls_have_no_exact_path(flag):
+    """A filter call scores in float, whatever the exact-path flags."""
+    p, reads = _case(90, [300, 200, 100, 310, 210, 110], 8)
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        sids = ctx.add_dna(reads)
+        got = []
+        for mode in (d.MODE_FILTER, d.MODE_FILTER | flag, d.MODE_FILTER):
+            ctx.score_pairs(sids[3:], pid, d.MODE_FILTER)  # other results in the buffers
+            got.append([(r.filter_f, r.filter_ln, r.exact_path) for r in ctx.score_pairs(sids[:3], pid, mode)])
+    assert got[0] == got[1] == got[2] and not any(g[2] for g in got[1])
