@@ -2875,6 +2875,10 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
             return st;
         }
         CallSlot &S = ctx->slot[si];
+        // after a replay that gave up a wait, the stores and anchors are not the pairs' own: no tables
+        CK(cudaEventSynchronize(S.ev[4]), "traceback replay");
+        if (std::any_of(S.hExOut.p, S.hExOut.p + nb, [](const ExactOut &e) { return e.failed != 0; }))
+            return completeCall(ctx);
         alignRowsKernel<<<dim3((maxL + kExactStripe + kTileSteps - 2) / kTileSteps, exactStripes(maxM), 2 * nb), 256, 0,
                           ctx->stream>>>(ctx->dAlignJobs.p, ctx->dAlignSteps.p, ctx->dAlignCells.p);
         sidesKernel<<<dim3((maxL + 127) / 128, nb), 128, 0, ctx->stream>>>(

@@ -783,8 +783,7 @@ __device__ WalkSpan walkAnchor(const AlignJob &jb, int a1, int a2, const XS *pre
 // The span pass: one thread per column of every job (grid.y = job), for the
 // columns whose anchor passes the job's gate; a walk does not depend on the
 // candidates' order, so this runs while the host sorts them.  Neighbouring
-// columns walk neighbouring cells.  The row is checked as well: after a failed
-// exact kernel the anchors are not its own.
+// columns walk neighbouring cells.
 __global__ void spanKernel(const AlignJob *jobs, const float *anchorM, const int *anchorE, const int *anchorRow,
                            const float *cells, const XS *X, const XS *suffix, const XS *revEv, const XS *fwdEv,
                            WalkSpan *spans) {
@@ -792,11 +791,10 @@ __global__ void spanKernel(const AlignJob *jobs, const float *anchorM, const int
     const int a2 = blockIdx.x * blockDim.x + threadIdx.x;
     if (a2 >= jb.L) return;
     const XS a{anchorM[jb.colOff + a2], anchorE[jb.colOff + a2]};
-    const int a1 = anchorRow[jb.colOff + a2];
-    if (a.m == 0.0f || scoreLess(a, XS{jb.minM, jb.minE}) || a1 < 0 || a1 > jb.M) return;
-    spans[jb.colOff + a2] = walkAnchor<false>(jb, a1, a2, reinterpret_cast<const XS *>(cells + 2 * jb.cellOff),
-                                              X + jb.cellOff, suffix + jb.cellOff, revEv + jb.colOff,
-                                              fwdEv + jb.colOff, nullptr, 0);
+    if (a.m == 0.0f || scoreLess(a, XS{jb.minM, jb.minE})) return;
+    spans[jb.colOff + a2] = walkAnchor<false>(jb, anchorRow[jb.colOff + a2], a2,
+                                              reinterpret_cast<const XS *>(cells + 2 * jb.cellOff), X + jb.cellOff,
+                                              suffix + jb.cellOff, revEv + jb.colOff, fwdEv + jb.colOff, nullptr, 0);
 }
 
 // An accepted candidate whose segments are written.

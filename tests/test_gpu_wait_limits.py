@@ -187,3 +187,24 @@ def test_plain_schedule_that_gives_up():
         assert ctx.last_timing()["exact_pairs"] == len(reads)
         _gives_up(ctx, lambda: plain(d.MODE_FILTER))
         assert [plain(m) for m in (d.MODE_MID, d.MODE_FILTER)] == want
+
+
+def test_traceback_whose_replay_gives_up():
+    """950 pairs score on the batched schedule, which waits for nothing; the hits'
+    replay gives up, and no traceback table is made from its stores."""
+    prof, p = _profile(100)
+    rng = np.random.default_rng(5)
+    reads = [synth.sample_homolog(rng, prof, max_aa=30)[:200] + synth.random_dna(rng, 300 + 7 * k, 0.5) for k in range(4)]
+    reads += [synth.random_dna(rng, 250, 0.5)] * 946
+    flat = lambda sims: [[(s[:5], s[5].tolist()) for s in q] for q in sims]
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        sids = ctx.add_dna(reads)
+        gates = [100.0] * 4 + [-1.0] * 946
+        want = flat(ctx.align(sids, pid, gates)[0])
+        assert any(want) and ctx.last_align_timing()["hits"] > 0
+        for _ in range(2):
+            _gives_up(ctx, lambda: ctx.align(sids, pid, gates))
+            t = ctx.last_align_timing()
+            assert t["hits"] > 0 and t["tables_ms"] == 0.0  # scored, not traced
+            assert flat(ctx.align(sids, pid, gates)[0]) == want
