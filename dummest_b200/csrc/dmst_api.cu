@@ -3256,8 +3256,9 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
     }
     // Batches of pairs under the device budget.  The full forward store is
     // 24 bytes per cell; the checkpointed one keeps a checkpoint every kAdjCk
-    // columns (about 1/12 of it) and recomputes.  Auto: the full store when
-    // every pair's fits the budget at once.
+    // columns (about 1/12 of it) and recomputes; both keep the boundary rows
+    // (one byte per cell).  Auto: the full store when every pair's fits the
+    // budget at once, in the pipelined kernel's sizes.
     CK(cudaSetDevice(ctx->device), "set device");
     size_t budget = ctx->opts.device_budget_bytes;
     if (!budget) {
@@ -3268,7 +3269,7 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
     long long fullAll = 0;
     for (size_t k = 0; k < n; ++k) {
         const int L = ctx->seqLen[pairs[order[k]].seq];
-        fullAll += ((adjStoreDoubles(M, L) + 31) & ~31LL) + adjBoundDoubles(L) + (tables ? 2LL * (M + 1) * L : 0);
+        fullAll += ((adjPipeFull(M, L) + 31) & ~31LL) + adjPipeBound(M, L) + (tables ? 2LL * (M + 1) * L : 0);
     }
     const bool ckpt = ctx->adjCheckpoint == DMST_ADJ_CKPT_ON ||
                       (ctx->adjCheckpoint == DMST_ADJ_CKPT_AUTO && (size_t)fullAll * 8 > budget);

@@ -3,6 +3,8 @@ around its 32-row stripes, reads around its 32-column blocks and 64-column
 checkpoints, from one pair (a cluster of CTAs) to more pairs than clusters, and
 a call that mixes pairs inside the range of its unscaled values with one far
 beyond it (log T above 900 bits), which the scaled kernel takes."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -72,3 +74,23 @@ def test_pairs_beyond_the_unscaled_range():
     reads.append(synth.sample_homolog(rng, prof, max_aa=60) + synth.random_dna(rng, 50, 0.5))
     assert port.log_total(p[0].astype(np.float64), p[1].astype(np.float64), p[2], d.decode_dna(reads[0])) > 900 * np.log(2)
     _check(*p, reads)
+
+
+@pytest.mark.parametrize("M,L,n", [(100, 900, 6), (31, 300, 1), (32, 301, 3)])
+def test_automatic_store_follows_what_the_pipeline_holds(M, L, n):
+    """The full forward store is taken when the budget holds it at once: 3 x 32
+    doubles per stripe and step and a share of T per stripe, in units of 32, and
+    two boundary rows of two doubles per stripe and column in each direction."""
+    rng, prof, p = _profile(M, 5)
+    reads = [synth.random_dna(rng, L, 0.5) for _ in range(n)]
+    stripes = (M + 32) // 32
+    need = 8 * n * ((stripes * (L + 31) * 96 + stripes + 31) // 32 * 32 + 4 * stripes * L)
+    for budget, checkpointed in ((need, False), (need - 1, True)):
+        with d.Context() as ctx:
+            ctx.opts.device_budget_bytes = budget
+            ctx.close()  # the same context anew, with the budget
+            ctx.h = C.c_void_p()
+            assert ctx.lib.dmst_ctx_create(C.byref(ctx.opts), C.byref(ctx.h)) == F.DMST_OK
+            pid = ctx.add_profile(*p)
+            ctx.loglik_grad(ctx.add_dna(reads), pid)
+            assert ctx.adjoint_checkpoint() == checkpointed
