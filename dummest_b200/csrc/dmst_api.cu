@@ -700,8 +700,9 @@ struct dmst_ctx {
     // dmst_align: the traceback buffers (dp_traceback.cuh) and the last call's results
     DevBuf<AlignJob> dAlignJobs;
     DevBuf<int> dAlignJobOf, dAlignRows;
-    DevBuf<float> dAlignSteps, dAlignCells, dAlignColR, dAlignColF;
-    DevBuf<XS> dAlignX, dAlignSuf, dAlignWork, dAlignRev, dAlignFwd;
+    DevBuf<float> dAlignCells, dAlignColR, dAlignColF;
+    DevBuf<XS> dAlignTables;                 // the replay's steps (floats), then the X and the suffix tables
+    DevBuf<XS> dAlignWork, dAlignRev, dAlignFwd;
     DevBuf<WalkSpan> dAlignSpan;
     DevBuf<WalkItem> dAlignItems;
     DevBuf<Seg> dAlignSegOut;
@@ -868,12 +869,10 @@ void dmst_ctx_destroy(dmst_ctx *ctx) {
     ctx->dAlignJobs.release();
     ctx->dAlignJobOf.release();
     ctx->dAlignRows.release();
-    ctx->dAlignSteps.release();
     ctx->dAlignCells.release();
     ctx->dAlignColR.release();
     ctx->dAlignColF.release();
-    ctx->dAlignX.release();
-    ctx->dAlignSuf.release();
+    ctx->dAlignTables.release();
     ctx->dAlignWork.release();
     ctx->dAlignRev.release();
     ctx->dAlignFwd.release();
@@ -2416,7 +2415,7 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                                ctx->dCodes.p, S.dSeeds.p, S.dScales.p, ctx->dExactPool.p, poolSlot, ctx->dExactRing.p,
                                exactRing, ctx->dExactAbort.p, S.dExOut.p, anchors ? S.dAnchorOff.p : nullptr,
                                S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p, align ? ctx->dAlignJobOf.p : nullptr,
-                               align ? ctx->dAlignJobs.p : nullptr, align ? ctx->dAlignSteps.p : nullptr,
+                               align ? ctx->dAlignJobs.p : nullptr, align ? reinterpret_cast<float *>(ctx->dAlignTables.p) : nullptr,
                                align ? ctx->dAlignRows.p : nullptr, ctx->spinLimit()};
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t cfg = clusterLaunch(exactC, exactW, exactW * sizeof(WindowX), exactC * exactClusters, &at, tail);
@@ -2741,7 +2740,8 @@ int dmst_anchors(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_score *be
 // anchors on the host (from the spans), and the store pass for the kept ones.
 static size_t alignJobBytes(int M, int L) {
     const size_t cells = (size_t)(M + 1) * L;
-    return cells * (8 + 8 + 8) + 2 * (size_t)exactW1Floats(M, L) * 4 + (size_t)L * (4 + 4 + 8 * kFlankArrays + 8 + 8 + 4 + sizeof(WalkSpan) + 2 * sizeof(Seg)) +
+    return cells * 8 + std::max(cells * (8 + 8), 2 * (size_t)exactW1Floats(M, L) * 4) +
+           (size_t)L * (4 + 4 + 8 * kFlankArrays + 8 + 8 + 4 + sizeof(WalkSpan) + 2 * sizeof(Seg)) +
            (size_t)alignRowInts(M) * 4 + 256;
 }
 
@@ -2808,7 +2808,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
 
     size_t freeB = 0, totalB = 0;
     CK(cudaMemGetInfo(&freeB, &totalB), "memory info");
-    const size_t held = (ctx->dAlignCells.cap + ctx->dAlignSteps.cap) * sizeof(float) + (ctx->dAlignX.cap + ctx->dAlignSuf.cap) * sizeof(XS);
+    const size_t held = ctx->dAlignCells.cap * sizeof(float) + ctx->dAlignTables.cap * sizeof(XS);
     const size_t budget = std::max<size_t>((freeB + held) / 2, (size_t)256 << 20);
     NullRates nr;
     nr.single = (double)(ctx->rates.insert1 + ctx->rates.delete2);
@@ -2852,9 +2852,9 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         // headroom: calls whose hits differ a little reuse the buffers (a
         // reallocation synchronises the device and costs a cudaMalloc of GBs)
         CK(ctx->dAlignCells.ensure((size_t)cells * 2, 0.3), "alloc traceback tables");
-        CK(ctx->dAlignSteps.ensure((size_t)steps, 0.3), "alloc traceback tables");
-        CK(ctx->dAlignX.ensure((size_t)cells, 0.3), "alloc traceback tables");
-        CK(ctx->dAlignSuf.ensure((size_t)cells, 0.3), "alloc traceback tables");
+        // the steps are row-major cells before the X and suffix tables are made: one buffer
+        CK(ctx->dAlignTables.ensure(std::max((size_t)cells * 2, ((size_t)steps + 1) / 2), 0.3), "alloc traceback tables");
+        XS *alignX = ctx->dAlignTables.p, *alignSuf = alignX + cells;
         CK(ctx->dAlignRows.ensure((size_t)rowsN, 0.3), "alloc traceback rows");
         CK(ctx->dAlignColR.ensure((size_t)cols, 0.3), "alloc traceback columns");
         CK(ctx->dAlignColF.ensure((size_t)cols, 0.3), "alloc traceback columns");
@@ -2880,7 +2880,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
         if (std::any_of(S.hExOut.p, S.hExOut.p + nb, [](const ExactOut &e) { return e.failed != 0; }))
             return completeCall(ctx);
         alignRowsKernel<<<dim3((maxL + kExactStripe + kTileSteps - 2) / kTileSteps, exactStripes(maxM), 2 * nb), 256, 0,
-                          ctx->stream>>>(ctx->dAlignJobs.p, ctx->dAlignSteps.p, ctx->dAlignCells.p);
+                          ctx->stream>>>(ctx->dAlignJobs.p, reinterpret_cast<const float *>(alignX), ctx->dAlignCells.p);
         sidesKernel<<<dim3((maxL + 127) / 128, nb), 128, 0, ctx->stream>>>(
             ctx->dAlignJobs.p, ctx->dAlignCells.p, ctx->dAlignRows.p, ctx->dAlignColR.p, ctx->dAlignColF.p);
         flankPrepKernel<<<dim3((maxL + 4 + 127) / 128, nb), 128, 0, ctx->stream>>>(
@@ -2893,15 +2893,14 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
                                                    ctx->dAlignRev.p, ctx->dAlignFwd.p);
         xTableKernel<<<dim3((maxL + 127) / 128, (maxM + 1 + kXRows - 1) / kXRows, nb), 128, 0, ctx->stream>>>(
             ctx->dAlignJobs.p, S.dPairs.p, ctx->dProfiles.p, ctx->dEmit.p, ctx->dParams.p, ctx->dCodes.p, S.dScales.p,
-            ctx->dAlignCells.p, ctx->dAlignRows.p, ctx->dAlignX.p);
+            ctx->dAlignCells.p, ctx->dAlignRows.p, alignX);
         CK(cudaFuncSetAttribute(optimalKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOptSmem), "smem attribute");
         const int optThreads = std::min(kOptThreads, (maxL + 32 * kOptPer - 1) / (32 * kOptPer) * 32);
         optimalKernel<<<dim3(nb, 2), optThreads, kOptSmem, ctx->stream>>>(ctx->dAlignJobs.p, ctx->dAlignCells.p, ctx->dAlignRows.p,
-                                                          ctx->dAlignX.p, ctx->dAlignRev.p, ctx->dAlignFwd.p,
-                                                          ctx->dAlignSuf.p);
+                                                          alignX, ctx->dAlignRev.p, ctx->dAlignFwd.p, alignSuf);
         spanKernel<<<dim3((maxL + 127) / 128, nb), 128, 0, ctx->stream>>>(
-            ctx->dAlignJobs.p, S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p, ctx->dAlignCells.p, ctx->dAlignX.p,
-            ctx->dAlignSuf.p, ctx->dAlignRev.p, ctx->dAlignFwd.p, ctx->dAlignSpan.p);
+            ctx->dAlignJobs.p, S.dAnchorM.p, S.dAnchorE.p, S.dAnchorRow.p, ctx->dAlignCells.p, alignX,
+            alignSuf, ctx->dAlignRev.p, ctx->dAlignFwd.p, ctx->dAlignSpan.p);
         CK(cudaGetLastError(), "traceback table kernels");
         if ((st = completeCall(ctx))) return st;
         tm[2] += msSince(tPhase);
@@ -3020,7 +3019,7 @@ int dmst_align(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, dmst_result *out
                "upload traceback walks");
             storeWalkKernel<<<(int)((items.size() + kStoreWarps - 1) / kStoreWarps), kStoreWarps * 32, 0, ctx->stream>>>(
                 ctx->dAlignJobs.p, ctx->dAlignItems.p, (int)items.size(), S.dAnchorRow.p, ctx->dAlignCells.p,
-                ctx->dAlignX.p, ctx->dAlignSuf.p, ctx->dAlignRev.p, ctx->dAlignFwd.p, ctx->dAlignSegOut.p);
+                alignX, alignSuf, ctx->dAlignRev.p, ctx->dAlignFwd.p, ctx->dAlignSegOut.p);
             CK(cudaGetLastError(), "traceback store kernel");
             const size_t first = ctx->alignSegOut.size();
             ctx->alignSegOut.resize(first + (size_t)ng);

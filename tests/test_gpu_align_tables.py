@@ -37,3 +37,26 @@ def test_a_hit_alone_equals_the_hit_in_company(M, lengths):
     assert M < 31 or all(alone)
     for k, got in zip(idx, many):
         assert _flat(got) == _flat(alone[k]), (M, len(reads[k]))
+
+
+def test_a_long_hit_holds_24_bytes_per_cell():
+    """The tables of a traced hit take 24 bytes per cell, and headroom of 30%."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(3)
+    M, L = 1000, 50000
+    prof = synth.make_profile(rng, M, "long")
+    h = synth.sample_homolog(rng, prof, max_aa=M, fs_rate=0.001)
+    read = synth.random_dna(rng, 20000, 0.5) + h
+    read += synth.random_dna(rng, L - len(read), 0.5)
+    p = d.finalize_hmm(synth.hmmer3_text([prof]))[1:]
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        sids = ctx.add_dna([read])
+        ctx.anchors(sids, pid)
+        ctx.align(sids, [pid], [-1.0])  # scored, not traced: every other buffer of the call
+        free = torch.cuda.mem_get_info()[0]
+        sims, _ = ctx.align(sids, [pid], [3e38])
+        held = free - torch.cuda.mem_get_info()[0]
+    assert sims[0]
+    cells, per_column = (M + 1) * L, 400
+    assert held <= 1.3 * (24 * cells + per_column * L) + (64 << 20), held / cells
