@@ -3307,34 +3307,40 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
         CK(cudaOccupancyMaxActiveClusters(&pClusters, pipeKern, &cfg), "cluster occupancy");
         if (pClusters < 1) return ctx->fail(DMST_ERANGE, "adjoint kernel does not fit on an SM");
     }
+    // Doubles of the stores of the pair at position k: forward, boundary rows, tables.
+    struct Need {
+        long long f, b, p;
+        size_t bytes() const { return (size_t)(f + b + p) * sizeof(double); }
+    };
+    auto needOf = [&](int k, bool pipe) {
+        const int L = ctx->seqLen[pairs[order[k]].seq];
+        const long long f = pipe ? (ckpt ? adjPipeCkpt(M, L, pW * pC) : adjPipeFull(M, L))
+                                 : (ckpt ? adjCkptDoubles(M, L) : adjStoreDoubles(M, L));
+        // 256-byte aligned stores (cp.async)
+        return Need{(f + 31) & ~31LL, pipe ? adjPipeBound(M, L) : adjBoundDoubles(L), tables ? 2LL * (M + 1) * L : 0};
+    };
     // Runs the adjoint over the positions `which` (longest read first) in
     // batches under the budget; pipe: the pipelined kernel, whose per-job
     // status goes to `status`.
     auto runBatches = [&](const std::vector<int> &which, bool pipe, std::vector<int> &status) -> int {
         const size_t m = which.size();
         std::vector<AdjointJob> jobs(m);
-        std::vector<long long> needF(m), needB(m), needP(m);
+        std::vector<Need> need(m);
         for (size_t q = 0; q < m; ++q) {
-            const int L = ctx->seqLen[pairs[order[which[q]]].seq];
             jobs[q] = AdjointJob{which[q], 0, 0, 0, tables ? 0 : -1};
-            // 256-byte aligned stores (cp.async)
-            needF[q] = ((pipe ? (ckpt ? adjPipeCkpt(M, L, pW * pC) : adjPipeFull(M, L))
-                              : (ckpt ? adjCkptDoubles(M, L) : adjStoreDoubles(M, L))) +
-                        31) & ~31LL;
-            needB[q] = pipe ? adjPipeBound(M, L) : adjBoundDoubles(L);
-            needP[q] = tables ? 2LL * (M + 1) * L : 0;
+            need[q] = needOf(which[q], pipe);
         }
         status.assign(m + 1, 0);
         for (size_t k0 = 0; k0 < m;) {
             size_t k1 = k0;
             long long f = 0, b = 0, pp = 0;
-            while (k1 < m && (k1 == k0 || (size_t)(f + needF[k1] + b + needB[k1] + pp + needP[k1]) * 8 <= budget)) {
+            while (k1 < m && (k1 == k0 || (size_t)(f + b + pp) * sizeof(double) + need[k1].bytes() <= budget)) {
                 jobs[k1].fOff = f;
                 jobs[k1].bOff = b;
                 if (tables) jobs[k1].pOff = pp;
-                f += needF[k1];
-                b += needB[k1];
-                pp += needP[k1];
+                f += need[k1].f;
+                b += need[k1].b;
+                pp += need[k1].p;
                 ++k1;
             }
             const int nj = (int)(k1 - k0);
@@ -3398,7 +3404,7 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
             if (post)
                 for (size_t k = k0; k < k1; ++k)
                     CK(cudaMemcpyAsync(post + postOff[order[which[k]]], ctx->dPost.p + jobs[k].pOff,
-                                       (size_t)needP[k] * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
+                                       (size_t)need[k].p * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
                        "download posterior tables");
             std::vector<double> blt(nj);
             CK(cudaMemcpyAsync(blt.data(), ctx->dLogT.p, nj * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
@@ -3420,20 +3426,28 @@ static int runAdjoint(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, double *l
         return DMST_OK;
     };
     CK(cudaMemsetAsync(ctx->dGrad.p, 0, gN * sizeof(double), ctx->stream), "zero gradient");
-    std::vector<int> all(n), beyond, status;
-    std::iota(all.begin(), all.end(), 0);
-    if ((st = runBatches(all, true, status))) return st;
-    bool redo = false;
-    for (size_t k = 0; k <= n; ++k) {
-        redo |= status[k] == kAdjRedo;
-        if (k < n && status[k] == kAdjRange) beyond.push_back((int)k);
+    // A pair whose stores alone are beyond the memory there is (the caller's
+    // budget, or all that is free) runs on the one-warp kernel when that one's
+    // are not: it keeps two boundary rows, the pipeline two per stripe.
+    const size_t most = ctx->opts.device_budget_bytes ? ctx->opts.device_budget_bytes : 2 * budget;
+    std::vector<int> piped, oneWarp, status;
+    for (int k = 0; k < (int)n; ++k)
+        (needOf(k, true).bytes() > most && needOf(k, false).bytes() <= most ? oneWarp : piped).push_back(k);
+    if (!piped.empty()) {
+        if ((st = runBatches(piped, true, status))) return st;
+        bool redo = false;
+        for (size_t q = 0; q < status.size(); ++q) {
+            redo |= status[q] == kAdjRedo;
+            if (status[q] == kAdjRange) oneWarp.push_back(piped[q]);  // values that need the stripe offsets
+        }
+        if (redo) {  // part of a gradient is in the sums: every pair again
+            CK(cudaMemsetAsync(ctx->dGrad.p, 0, gN * sizeof(double), ctx->stream), "zero gradient");
+            oneWarp.resize(n);
+            std::iota(oneWarp.begin(), oneWarp.end(), 0);
+        }
+        std::sort(oneWarp.begin(), oneWarp.end());
     }
-    if (redo) {  // part of a gradient is in the sums: every pair again
-        CK(cudaMemsetAsync(ctx->dGrad.p, 0, gN * sizeof(double), ctx->stream), "zero gradient");
-        beyond = all;
-    }
-    // pairs whose values need the stripe offsets
-    if (!beyond.empty() && (st = runBatches(beyond, false, status))) return st;
+    if (!oneWarp.empty() && (st = runBatches(oneWarp, false, status))) return st;
     // Timing of the call: [1] null model, [2] adjoint kernels, [0] both.
     ctx->lastNullMs = nullMs;
     ctx->lastDpMs = adjMs;

@@ -76,6 +76,15 @@ def test_pairs_beyond_the_unscaled_range():
     _check(*p, reads)
 
 
+def _budget_context(budget):
+    ctx = d.Context()
+    ctx.close()  # the same context anew, with the budget
+    ctx.opts.device_budget_bytes = budget
+    ctx.h = C.c_void_p()
+    assert ctx.lib.dmst_ctx_create(C.byref(ctx.opts), C.byref(ctx.h)) == F.DMST_OK
+    return ctx
+
+
 @pytest.mark.parametrize("M,L,n", [(100, 900, 6), (31, 300, 1), (32, 301, 3)])
 def test_automatic_store_follows_what_the_pipeline_holds(M, L, n):
     """The full forward store is taken when the budget holds it at once: 3 x 32
@@ -86,11 +95,40 @@ def test_automatic_store_follows_what_the_pipeline_holds(M, L, n):
     stripes = (M + 32) // 32
     need = 8 * n * ((stripes * (L + 31) * 96 + stripes + 31) // 32 * 32 + 4 * stripes * L)
     for budget, checkpointed in ((need, False), (need - 1, True)):
-        with d.Context() as ctx:
-            ctx.opts.device_budget_bytes = budget
-            ctx.close()  # the same context anew, with the budget
-            ctx.h = C.c_void_p()
-            assert ctx.lib.dmst_ctx_create(C.byref(ctx.opts), C.byref(ctx.h)) == F.DMST_OK
+        with _budget_context(budget) as ctx:
             pid = ctx.add_profile(*p)
             ctx.loglik_grad(ctx.add_dna(reads), pid)
             assert ctx.adjoint_checkpoint() == checkpointed
+
+
+def test_a_pair_beyond_the_budget_on_the_pipeline_alone():
+    """A read whose stores fit the budget on the one-warp kernel (two boundary
+    rows) and not on the pipeline (two per stripe and direction) runs on the
+    former and takes no more memory than the budget; shorter reads of the call
+    stay on the pipeline, and the results are those of a call without a budget."""
+    torch = pytest.importorskip("torch")
+    rng, prof, p = _profile(1000, 5)
+    reads = [synth.random_dna(rng, L, 0.5) for L in (20000, 700, 400)]
+    h = synth.sample_homolog(rng, prof, max_aa=60)
+    reads = [r[:100] + h + r[100 + len(h):] for r in reads]
+    stripes, L = 32, 20000
+    states = stripes * ((L + 31 + 63) // 64) * 32 * 11  # checkpoints: 11 values per lane
+    one_warp = 8 * (states + 2 * stripes * L + 40 + 2 * 64 * 96 + 4 * (L + 4) + 32)
+    pipelined = 8 * (states + 4 * stripes * L)  # at least
+    budget = (one_warp + pipelined) // 2
+    assert one_warp < budget < pipelined
+    got, held = [], []
+    for limit in (budget, 0):
+        with _budget_context(limit) as ctx:
+            ctx.adjoint_checkpoint(F.ADJ_CKPT_ON)
+            pid = ctx.add_profile(*p)
+            sids = ctx.add_dna(reads)
+            ctx.loglik_grad(sids[1:], pid)
+            ctx.score_pairs(sids, pid, F.MODE_FILTER)  # the null model's buffers for these reads
+            free = torch.cuda.mem_get_info()[0]
+            got.append(ctx.loglik_grad(sids, pid))
+            held.append(free - torch.cuda.mem_get_info()[0])
+    assert held[0] <= budget + (4 << 20) < held[1]
+    assert np.array_equal(got[0][0], got[1][0])
+    for x, y in zip(got[0][1:], got[1][1:]):
+        np.testing.assert_allclose(x, y, rtol=1e-11, atol=1e-13 * np.abs(y).max())
