@@ -26,6 +26,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <numeric>
@@ -1101,6 +1102,8 @@ static void commitSeqs(dmst_ctx *ctx, const std::vector<long long> &off, const s
     }
 }
 
+constexpr size_t kCodeBlock = (size_t)4 << 20;  // bytes of an upload of codes
+
 int dmst_seqs_add_decoded(dmst_ctx *ctx, const uint8_t *codes, const int64_t *offsets, int nseq, int *first_id) {
     if (!ctx || (!codes && nseq > 0)) return DMST_EINVAL;
     int st = checkOffsets(offsets, nseq);
@@ -1111,13 +1114,29 @@ int dmst_seqs_add_decoded(dmst_ctx *ctx, const uint8_t *codes, const int64_t *of
     std::vector<long long> off;
     std::vector<int> lens;
     if ((st = reserveSeqs(ctx, offsets, nseq, off, lens))) return st;
-    // one copy of the sequences as the device holds them (16-byte aligned starts)
+    // Blocks of sequences as the device holds them (16-byte aligned starts), one
+    // copy each; a sequence of a block or more (or all, when the host has no
+    // memory for a block) goes up from the caller's memory.
     if (nseq > 0) {
-        std::vector<uint8_t> up((size_t)(off[nseq - 1] + (lens[nseq - 1] + 15) / 16 * 16 - off[0]), 0);
-        for (int i = 0; i < nseq; ++i) std::memcpy(up.data() + (off[i] - off[0]), codes + offsets[i], lens[i]);
-        CK(cudaMemcpyAsync(ctx->dCodes.p + off[0], up.data(), up.size(), cudaMemcpyHostToDevice, ctx->stream),
-           "upload codes");
-        CK(cudaStreamSynchronize(ctx->stream), "upload codes");
+        auto endOf = [&](int i) { return off[i] + (lens[i] + 15) / 16 * 16; };
+        const size_t block = std::min(kCodeBlock, (size_t)(endOf(nseq - 1) - off[0]));
+        const std::unique_ptr<uint8_t[]> up(new (std::nothrow) uint8_t[block]);
+        for (int i = 0; i < nseq;) {
+            int e = i;
+            while (up && e < nseq && (size_t)(endOf(e) - off[i]) <= block) {
+                uint8_t *to = up.get() + (off[e] - off[i]);
+                std::memcpy(to, codes + offsets[e], lens[e]);
+                std::memset(to + lens[e], 0, (size_t)(endOf(e) - off[e]) - lens[e]);
+                ++e;
+            }
+            const bool direct = e == i;
+            if (direct) ++e;
+            CK(cudaMemcpyAsync(ctx->dCodes.p + off[i], direct ? codes + offsets[i] : up.get(),
+                               direct ? lens[i] : (size_t)(endOf(e - 1) - off[i]), cudaMemcpyHostToDevice, ctx->stream),
+               "upload codes");
+            CK(cudaStreamSynchronize(ctx->stream), "upload codes");  // the block is filled again
+            i = e;
+        }
     }
     commitSeqs(ctx, off, lens, first_id);
     return DMST_OK;
