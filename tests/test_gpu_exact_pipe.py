@@ -93,3 +93,41 @@ def test_filter_calls_have_no_exact_path(flag):
             ctx.score_pairs(sids[3:], pid, d.MODE_FILTER)  # other results in the buffers
             got.append([(r.filter_f, r.filter_ln, r.exact_path) for r in ctx.score_pairs(sids[:3], pid, mode)])
     assert got[0] == got[1] == got[2] and not any(g[2] for g in got[1])
+
+
+@pytest.mark.parametrize("M", [62, 63, 64, 65, 127, 128, 129])
+def test_reads_around_the_32_column_blocks(M):
+    """The kernel's window blocks are 32 columns; its first look ahead is two."""
+    p, reads = _case(M, [32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129], M + 1)
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        sids = ctx.add_dna(reads)
+        got = ctx.score_pairs(sids, pid, d.MODE_MID | d.MODE_FORCE_EXACT)
+        cols, _ = ctx.anchors(sids, pid)
+    for r, g, col in zip(reads, got, cols):
+        codes = d.decode_dna(r)
+        mid, flt, _ = port.score_pair(*p, codes)
+        assert (g.mid.m, g.mid.e) == mid and (g.filter.m, g.filter.e) == flt, len(r)
+        _same_anchors(col, port.anchors(*p, codes))
+
+
+def _same_anchors(got, want):
+    (am, ae, ar), (wm, we, wr) = got, want
+    np.testing.assert_array_equal(am, wm)
+    np.testing.assert_array_equal(ae[am != 0], np.asarray(we)[am != 0])
+    np.testing.assert_array_equal(ar[am != 0], np.asarray(wr)[am != 0])
+
+
+@pytest.mark.parametrize("M,n", [(300, 1), (300, 200), (900, 2)])
+def test_anchors_of_rescaled_rows_equal_oracle(M, n):
+    """One pair (both discovery sweeps side by side) and many (in turn), rows that
+    rescale in both sweeps: the anchors' products carry both rows' counts."""
+    p, reads = _case(M, [3 * M + 50, 2 * M, 700, 3 * M], M, homolog=M)
+    want = [port.anchors(*p, d.decode_dna(r)) for r in reads[:n]]
+    assert port.score_pair(*p, d.decode_dna(reads[0]))[2][0] > 0
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        sids = ctx.add_dna(reads)
+        cols, _ = ctx.anchors([sids[k % len(reads)] for k in range(n)], pid)
+    for k, got in enumerate(cols):
+        _same_anchors(got, want[k % len(reads)])
