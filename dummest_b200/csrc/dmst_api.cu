@@ -26,6 +26,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -1816,6 +1817,32 @@ static int submitCall(dmst_ctx *ctx, const dmst_pair *pairs, size_t n, int mode,
                 pairShape[i] = shapeTab[2 * (size_t)pairs[i].profile + lengthClass(L)];
             }
             ++groupPairs[pairShape[i]];
+        }
+        // Short reads against tall profiles, more pairs than the 12-warp CTAs'
+        // warps and no more than those of 16-warp ones, all about as long: one
+        // round on 16-warp CTAs (three rows per lane at most: four spill)
+        // instead of two.  2,000 pairs of M = 1000 x 30, 75 and 150 nt: 1.65,
+        // 1.80 and 2.08 ms, 2.55, 2.65 and 2.77 in two rounds; M = 2000 x 30 and
+        // 75: 3.14 and 3.37, 4.66 and 4.78.  Below 256 rows and from four rows
+        // per lane on, the gain is less than what the wider CTAs' steps cost in
+        // part of the sizes (M = 100 x 30: 0.50 for 0.49, M = 1000 x 600: 1.0).
+        if (byLength && mid && !search && !plain && n > (size_t)kCtaWarpsMid * ctx->smCount &&
+            n <= (size_t)kCtaWarps * ctx->smCount) {
+            int minM = INT_MAX, maxM = 0, minL = INT_MAX, maxL = 0;
+            for (size_t i = 0; i < n; ++i) {
+                const int M = ctx->profiles[pairs[i].profile].M, L = ctx->seqLen[pairs[i].seq];
+                minM = std::min(minM, M);
+                maxM = std::max(maxM, M);
+                minL = std::min(minL, L);
+                maxL = std::max(maxL, L);
+            }
+            if (minM >= 256 && untunedR(maxM, maxL) <= 3 && 2 * stagSteps(minM, minL, 3) > stagSteps(maxM, maxL, 3)) {
+                std::fill(std::begin(groupPairs), std::end(groupPairs), 0);
+                for (int &sh : pairShape) {
+                    sh = rIndex(std::min(kShapeR[sh / 3], 3)) * 3 + wIndex(kCtaWarps);
+                    ++groupPairs[sh];
+                }
+            }
         }
         if (!ctx->tune.forceR && ctx->opts.rows_per_lane == 0 && !plain) {
             int big = 0;

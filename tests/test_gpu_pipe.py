@@ -75,3 +75,17 @@ def test_batched_stripe_transitions_equal_oracle(R):
             want_mid, want_flt, _ = port.score_pair(*p, d.decode_dna(r))
             assert (m.mid.m, m.mid.e) == want_mid and (m.filter.m, m.filter.e) == want_flt, (M, len(r))
             assert f.filter_f == port.filter_pair(*p, d.decode_dna(r)), (M, len(r))
+
+
+@pytest.mark.parametrize("M,n", [(256, 1776), (256, 1777), (300, 2368), (300, 2369), (1000, 1900)])
+def test_wide_blocks_equal_oracle(M, n):
+    """Calls of more short reads than the 12-warp blocks' warps and as many as
+    the 16-warp blocks' (three rows per lane), and on both sides of them."""
+    p, reads = _case(M, [30 + 3 * k for k in range(20)], M)
+    with d.Context() as ctx:
+        pid = ctx.add_profile(*p)
+        sids = ctx.add_dna(reads)
+        got = ctx.score_pairs([sids[k % 20] for k in range(n)], pid, d.MODE_MID)
+    want = [port.score_pair(*p, d.decode_dna(r)) for r in reads]
+    for k, r in enumerate(got):
+        assert ((r.mid.m, r.mid.e), (r.filter.m, r.filter.e)) == (want[k % 20][0], want[k % 20][1])
