@@ -56,7 +56,7 @@ struct DevPair {
     int L;
     int M;
     int prof;
-    int R;              // profile rows per lane (1, 2 or 4)
+    int R;              // profile rows per lane (1 to 4; the plain schedule's stripes: 1, 2 or 4)
 };
 static_assert(sizeof(DevPair) == 32, "DevPair layout");
 

@@ -1,7 +1,8 @@
-// The row-contiguous stripe wavefront: the step functions of the exact
-// row-rescaled path (dp_exact_pipe.cuh, dp_exact.cuh) and of the plain
-// one-pair-per-launch schedule (dp_plain.cuh).  The batched kernel of the
-// fast path is dp_stagger.cuh.
+// The row-contiguous stripe wavefront: the step functions of the plain
+// one-pair-per-launch schedule (dp_plain.cuh), and what every schedule shares:
+// the pair's fields and sweep arguments, coefficients, W1 stores and copies.
+// The steps of the batched and the few-pair kernels are in dp_stagger.cuh,
+// those of the exact path in dp_exact_pipe.cuh.
 //
 // Layout.  The profile's rows are striped across the 32 lanes of a warp: a
 // stripe is S = 32*R consecutive rows, lane l owns rows l*R .. l*R+R-1 of the
@@ -69,19 +70,19 @@ struct PairCold {
 
 struct SweepArgs {
     PairCold *cold;         // in shared memory
-    const float *smE;       // emission table, [25][rowPad] (shared memory; the exact path reads it from global)
+    const float *smE;       // emission table, [25][rowPad] (shared memory, or global: tall profiles, the plain schedule)
     float *w1;              // this warp's W1 slot
     float *ring;            // this warp's stripe-boundary ring (4 floats per column)
     int L, rowPad, nS, P, D;
     // Stripes of this warp, in processing order: sFirst, sFirst + sStep, ...
-    // (nMine of them; the fast path: 0, 1, ..., nS-1).  The exact path runs a
-    // pair's stripes on several warps: the ring of stripe sp (processing
-    // order) is then ring + (sp % ringSlots) * ringStride.
+    // (nMine of them; the batched kernel: 0, 1, ..., nS-1; the few-pair kernel
+    // and the exact path: one at a time).  The plain schedule runs a pair's
+    // stripes on several warps: the ring of stripe sp (processing order) is then
+    // ring + (sp % ringSlots) * ringStride.
     int sFirst, sStep, nMine, ringSlots;
     long long ringStride;
-    // Exact replay for the traceback: the row-major (M+1) x L matrix that takes
-    // each cell's value before its row's rescale (backward: W1, forward: W0),
-    // or null.
+    // Exact replay for the traceback: the stripe's store, by step, of each cell's
+    // value before its row's rescale (backward: W1, forward: W0), or null.
     float *alignOut;
 
     __device__ __forceinline__ const uint8_t *codes() const {

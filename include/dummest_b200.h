@@ -458,8 +458,12 @@ int dmst_last_timing_ex(const dmst_ctx *ctx, double *out, int n);
  * 2 or 1) and 16, 8 or 12 warps per CTA.  dmst_autotune times the DP kernel of
  * every shape on the caller's sample of pairs (mode MID, each shape run twice,
  * the second timed) and keeps, per R, the fastest CTA shape and its rate in
- * computed cells per second.  Later calls with rows_per_lane == 0 then pick,
- * per profile, the R with the least expected time (computed rows / rate).
+ * computed cells per second.  Later batched mid calls with rows_per_lane == 0
+ * then pick, per profile and read-length class, the R with the least expected
+ * time (computed rows / rate), and its fastest CTA shape.  The rates are the mid
+ * kernel's: filter calls and the filter wave of a search take R by the step
+ * model of untuned calls and 8 warps per CTA, and calls of few pairs (at most
+ * six per SM) run on the stripe pipeline, tuned or not.
  * gcups6 (may be NULL) receives the rates in GCUPS of computed cells, for
  * R = 4, 2, 1 x 16, 8 warps; dmst_tuned_rates gives nine (R = 4, 2, 1 x 16, 8,
  * 12 warps) and dmst_tuned_rates_ex the first n <= 12 of all twelve
@@ -468,7 +472,8 @@ int dmst_last_timing_ex(const dmst_ctx *ctx, double *out, int n);
 int dmst_autotune(dmst_ctx *ctx, const dmst_pair *sample, size_t n, double *gcups6);
 int dmst_tuned_rates(const dmst_ctx *ctx, double *gcups9);
 int dmst_tuned_rates_ex(const dmst_ctx *ctx, double *gcups, int n);
-/* The shape a call would use for a profile of length M. */
+/* The shape that a batched mid call uses for a profile of length M and reads of
+ * 700 nt and more (before dmst_autotune: of 700 nt). */
 int dmst_tuned_shape(const dmst_ctx *ctx, int M, int *rows_per_lane, int *warps_per_cta);
 
 /* The stripe pipelines' wait budget: a warp that waits for the stripe before

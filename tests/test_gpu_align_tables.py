@@ -1,5 +1,5 @@
 """Traceback tables at the edges of their kernels: profiles around the exact
-kernel's 64-row stripes, reads around its 30-column blocks and around the
+kernel's 64-row stripes, reads of a few lengths and around the
 4096 columns that the optimal tables hold in shared memory.  A hit's
 alignments do not depend on its company, so a hit traced alone (its two
 discovery sweeps side by side, a block as wide as its read) equals the same hit

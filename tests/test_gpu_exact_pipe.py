@@ -1,5 +1,5 @@
 """The exact path's stripe pipeline against the plain-C oracle, bit for bit:
-profile lengths around its 64-row stripes, reads around its 30-column blocks,
+profile lengths around its 64-row stripes, reads around its 32-column blocks,
 one pair (a cluster of CTAs) to many, rows that rescale, anchors, and calls on
 both streams that share its scratch."""
 import numpy as np

@@ -1,11 +1,11 @@
 """The exact path's bounded waits end a call with DMST_ETIMEOUT, and the
 context stays usable.
 
-The stripe-pipelined exact kernel runs a pair's stripes on several warps; a
-warp waits (in shared memory, 64 ns sleeps) until the stripe before its own
-has written what it needs.  With the wait budget set to one sleep the first
-real wait gives up: the kernel marks the pair failed, every warp of the CTA
-leaves at its next block, and the call returns DMST_ETIMEOUT.  No wait is
+The stripe-pipelined exact kernel runs a pair's stripes of 64 rows on several
+warps; a warp waits (polling entries in global memory) until the stripe before
+its own has written what it needs.  With the wait budget set to one poll the
+first real wait gives up: the kernel marks the pair failed, every warp leaves at
+its next block, and the call returns DMST_ETIMEOUT.  No wait is
 unbounded, so nothing hangs.  With the default budget restored, the same call
 on the same context gives the results it gave before.
 """
